@@ -1,4 +1,6 @@
-"""Writes dtrig_table.inc, the constants of the FP64 sine/cosine in dtrig.cuh.
+"""Writes dtrig_table.inc, the constants of a table-driven FP64 sine/cosine (the
+form before dtrig.cuh's fixed-point one; no kernel includes it any more, only
+its host test reads it).
 
 * the table (sin(j*pi/256), cos(j*pi/256)), j = 0..511, each rounded to the
   nearest double from a 60-digit evaluation (exact zeros and ones at the
