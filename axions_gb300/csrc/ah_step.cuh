@@ -15,17 +15,15 @@
 namespace lat {
 
 template <class T, bool DIAG>
-__global__ void __launch_bounds__(BLOCK) ah_step_kernel(const Geom g, const Fields<T, 5> f, const StepCoefT<T> c,
-                                                        const DiagOut d)
+__global__ void __launch_bounds__(BLOCK) ah_step_kernel(const Geom g, const Flat r, const Fields<T, 5> f,
+                                                        const StepCoefT<T> c, const DiagOut d)
 {
     using TR = Trig<T>;
-    const int k = g.loz + (int)(blockIdx.x * BZ + threadIdx.x);
-    const int j = g.loy + (int)(blockIdx.y * BY + threadIdx.y);
-    const int i = g.lox + (int)blockIdx.z;
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
     double e_site = 0.0, g_site = 0.0;
 
-    if (k < g.hiz && j < g.hiy) {
-        const Nbr n = make_nbr(g, i, j, k);
+    if (q < r.n) {
+        const Nbr n = flat_nbr(g, r, q);
         const int s = n.s;
         const T* __restrict__ P0 = f.now[0];
         const T* __restrict__ P1 = f.now[1];
@@ -185,7 +183,7 @@ __global__ void __launch_bounds__(BLOCK) ah_step_kernel(const Geom g, const Fiel
         }
     }
 
-    if constexpr (DIAG) block_sum2_store(e_site, g_site, d.partials);
+    if constexpr (DIAG) flat_sum2_store(e_site, g_site, d.partials);
 }
 
 template <class T>
@@ -193,10 +191,10 @@ cudaError_t launch_ah_step_t(const Geom& g, const Fields<T, 5>& f, const StepCoe
                              cudaStream_t st)
 {
     const StepCoefT<T> c = coef_as<T>(c64);
-    const dim3 grid = site_grid(g);
-    const dim3 block(BZ, BY);
-    if (diag) ah_step_kernel<T, true><<<grid, block, 0, st>>>(g, f, c, d);
-    else ah_step_kernel<T, false><<<grid, block, 0, st>>>(g, f, c, d);
+    const Flat r = flat_region(g);
+    const int grid = flat_grid(r.n), block = flat_block(r.n);
+    if (diag) ah_step_kernel<T, true><<<grid, block, 0, st>>>(g, r, f, c, d);
+    else ah_step_kernel<T, false><<<grid, block, 0, st>>>(g, r, f, c, d);
     return cudaGetLastError();
 }
 

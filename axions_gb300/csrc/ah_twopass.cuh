@@ -81,15 +81,14 @@ __device__ __forceinline__ double tdiv(double a, double b, double inv_b)
 }
 
 template <bool STRICT, bool DIAG>
-__global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const double* __restrict__ TX,
+__global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Flat r, const double* __restrict__ TX,
                                                          const double* __restrict__ TY,
                                                          const double* __restrict__ TZ, const LinkSlots L)
 {
-    const int k = (int)(blockIdx.x * BZ + threadIdx.x);
-    const int j = (int)(blockIdx.y * BY + threadIdx.y);
-    const int i = (int)blockIdx.z;
-    if (k >= g.nz || j >= g.ny) return;
-    const Nbr n = make_nbr(g, i, j, k);
+    // g: the whole lattice as the region, so that q is the site index
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
+    if (q >= r.n) return;
+    const Nbr n = flat_nbr(g, r, q);
     const int s = n.s;
     const double tx = TX[s], ty = TY[s], tz = TZ[s];
     const double tyxp = TY[s + n.xp], tzxp = TZ[s + n.xp];
@@ -132,17 +131,15 @@ __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const dou
 }
 
 template <bool STRICT, bool DIAG, bool RECIP>
-__global__ void __launch_bounds__(BLOCK, 2) ah_update_kernel(const Geom g, const Fields<double, 5> f,
+__global__ void __launch_bounds__(BLOCK, 2) ah_update_kernel(const Geom g, const Flat r, const Fields<double, 5> f,
                                                           const LinkSlotsC L, const StepCoef c,
                                                           const DiagOut d)
 {
-    const int k = g.loz + (int)(blockIdx.x * BZ + threadIdx.x);
-    const int j = g.loy + (int)(blockIdx.y * BY + threadIdx.y);
-    const int i = g.lox + (int)blockIdx.z;
+    const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
     double e_site = 0.0, g_site = 0.0;
 
-    if (k < g.hiz && j < g.hiy) {
-        const Nbr n = make_nbr(g, i, j, k);
+    if (q < r.n) {
+        const Nbr n = flat_nbr(g, r, q);
         const int s = n.s;
         const int sxm = s + n.xm, sym_ = s + n.ym, szm = s + n.zm;
         const double* __restrict__ P0 = f.now[0];
@@ -320,7 +317,7 @@ __global__ void __launch_bounds__(BLOCK, 2) ah_update_kernel(const Geom g, const
             f.past[4][s] = mul_pow2(tz, 2.0) - qz + c.dt2 * ttz;
         }
     }
-    if constexpr (DIAG) block_sum2_store(e_site, g_site, d.partials);
+    if constexpr (DIAG) flat_sum2_store(e_site, g_site, d.partials);
 }
 
 template <bool STRICT>
@@ -335,18 +332,20 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
     all.hix = g.nx;
     all.hiy = g.ny;
     all.hiz = g.nz;
-    const dim3 block(BZ, BY);
-    if (diag) ah_links_kernel<STRICT, true><<<site_grid(all), block, 0, st>>>(g, f.now[2], f.now[3], f.now[4], Lw);
-    else ah_links_kernel<STRICT, false><<<site_grid(all), block, 0, st>>>(g, f.now[2], f.now[3], f.now[4], Lw);
+    const Flat ra = flat_region(all);
+    const int la = flat_grid(ra.n), lb = flat_block(ra.n);
+    if (diag) ah_links_kernel<STRICT, true><<<la, lb, 0, st>>>(all, ra, f.now[2], f.now[3], f.now[4], Lw);
+    else ah_links_kernel<STRICT, false><<<la, lb, 0, st>>>(all, ra, f.now[2], f.now[3], f.now[4], Lw);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    const dim3 grid = site_grid(g);
+    const Flat r = flat_region(g);
+    const int grid = flat_grid(r.n), block = flat_block(r.n);
     if (diag) {
-        if (recip) ah_update_kernel<STRICT, true, true><<<grid, block, 0, st>>>(g, f, Lr, c, d);
-        else ah_update_kernel<STRICT, true, false><<<grid, block, 0, st>>>(g, f, Lr, c, d);
+        if (recip) ah_update_kernel<STRICT, true, true><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
+        else ah_update_kernel<STRICT, true, false><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
     } else {
-        if (recip) ah_update_kernel<STRICT, false, true><<<grid, block, 0, st>>>(g, f, Lr, c, d);
-        else ah_update_kernel<STRICT, false, false><<<grid, block, 0, st>>>(g, f, Lr, c, d);
+        if (recip) ah_update_kernel<STRICT, false, true><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
+        else ah_update_kernel<STRICT, false, false><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
     }
     return cudaGetLastError();
 }

@@ -241,8 +241,7 @@ static int64_t footprint(const lat_params& p)
     const int64_t ncomp = p.model == LAT_MODEL_MOORE ? 7 : 5;
     int64_t b = ncomp * 2 * N * elem + N * elem;  // fields, divbuf
     if (p.model == LAT_MODEL_AH && elem == 8 && p.kernel_variant == 0) b += 8 * (int64_t)ah_link_slots() * N;
-    const dim3 gr = site_grid(make_geom(p));
-    b += 16 * (int64_t)gr.x * gr.y * gr.z;        // partials
+    b += 16 * partial_pairs(make_geom(p));        // partials
     b += (int64_t)sizeof(long long) + (int64_t)sizeof(unsigned long long);
     return b;
 }
@@ -295,8 +294,7 @@ int lat_create(const lat_params* p, lat_handle** out)
         h->links_bytes = sizeof(double) * (size_t)ah_link_slots() * (size_t)h->N;
         if ((rc = dev_alloc(h, (void**)&h->links, h->links_bytes))) return fail(rc);
     }
-    const dim3 gr = site_grid(h->geom);
-    h->nblocks = (int)(gr.x * gr.y * gr.z);
+    h->nblocks = (int)partial_pairs(h->geom);
     if ((rc = dev_alloc(h, (void**)&h->partials, sizeof(double) * 2 * (size_t)h->nblocks))) return fail(rc);
     if ((rc = dev_alloc(h, (void**)&h->det_total, sizeof(long long)))) return fail(rc);
     if ((rc = dev_alloc(h, (void**)&h->wind_sum, sizeof(unsigned long long)))) return fail(rc);
@@ -525,7 +523,9 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
             LAT_CKL(launch_divergence_f32(h->geom, (const float*)h->slot(th0, tPast), (const float*)h->slot(th0 + 1, tPast),
                                          (const float*)h->slot(th0 + 2, tPast), cf, (float*)h->divbuf, h->stream));
     }
-    int tiled_used = 0;  // CTAs of the x-marching FP32 step, if it ran
+    // partials the step writes: one per CTA of its kernel (the flat kernels of
+    // the Abelian-Higgs FP64 and one-pass steps unless another one runs)
+    int used = flat_grid(flat_region(h->geom).n);
     if (p.model == LAT_MODEL_AH) {
         if (h->elem == 8) {
             Fields<double, 5> f;
@@ -548,7 +548,7 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
                 f.past[c] = (float*)h->slot(c, tPast);
             }
             if (p.kernel_variant != 1)
-                LAT_CKL(launch_ah_tiled_f32(h->geom, f, cf, d, diag, h->chunk, h->stream, p.kernel_variant, &tiled_used));
+                LAT_CKL(launch_ah_tiled_f32(h->geom, f, cf, d, diag, h->chunk, h->stream, p.kernel_variant, &used));
             else LAT_CKL(launch_ah_step_f32(h->geom, f, cf, d, diag, h->stream));
         }
     } else {
@@ -559,22 +559,26 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
                 f.past[c] = (double*)h->slot(c, tPast);
             }
             LAT_CKL(launch_moore_step_f64(h->geom, f, cf, d, diag, h->stream));
+            used = tile_count(h->geom);
         } else {
             Fields<float, 7> f;
             for (int c = 0; c < 7; ++c) {
                 f.now[c] = (const float*)h->slot(c, tNow);
                 f.past[c] = (float*)h->slot(c, tPast);
             }
-            if (p.kernel_variant != 1)
-                LAT_CKL(launch_moore_tiled_f32(h->geom, f, cf, d, diag, h->chunk, h->stream, p.kernel_variant, &tiled_used));
-            else LAT_CKL(launch_moore_step_f32(h->geom, f, cf, d, diag, h->stream));
+            if (p.kernel_variant != 1) {
+                LAT_CKL(launch_moore_tiled_f32(h->geom, f, cf, d, diag, h->chunk, h->stream, p.kernel_variant, &used));
+            } else {
+                LAT_CKL(launch_moore_step_f32(h->geom, f, cf, d, diag, h->stream));
+                used = tile_count(h->geom);
+            }
         }
     }
     if (absorb) LAT_CKL(launch_absorb_update(h->geom, (int)h->elem, nowv, pastv, h->btt, p.dt * p.dt, h->stream));
     if (diag) {
-        // partials written by the step: one per CTA of the kernel that ran
-        const int used = tiled_used > 0 ? tiled_used : h->nblocks;
-        LAT_CKL(launch_finalize(h->partials, used, diag_dst, h->stream));
+        int nl = 0;
+        LAT_CK(launch_finalize(h->partials, used, diag_dst, h->stream, &nl));
+        h->launches += nl;
     }
     if (write) {
         h->n += 1;

@@ -32,6 +32,67 @@ inline dim3 site_grid(const Geom& g)
                 (unsigned)(g.hix - g.lox));
 }
 
+inline int tile_count(const Geom& g)
+{
+    const dim3 gr = site_grid(g);
+    return (int)(gr.x * gr.y * gr.z);
+}
+
+// Linear walk of the evolved region for the FP64 site kernels: thread q of the
+// launch takes the region's q-th site in linear order.  A 32-wide tile along z
+// leaves lanes idle where the extent is no multiple of 32 (24 % of them at
+// nz = 97, half at nz = 33), and idle lanes cost the FP64 pipe as much as
+// working ones.  Quotients by the extents are multiplications (q < 2^31).
+struct FlatDiv {
+    unsigned mul, shift;
+};
+struct Flat {
+    unsigned n;       // sites of the region
+    int hy, hz;       // its extents along y and z
+    FlatDiv dy, dz;
+};
+
+// floor(q / d) = (mulhi(q, mul) + q) >> shift for q < 2^31
+inline FlatDiv flat_div(unsigned d)
+{
+    unsigned s = 0;
+    while ((1ull << s) < d) ++s;
+    return FlatDiv{(unsigned)((((1ull << s) - d) << 32) / d + 1), s};
+}
+
+inline Flat flat_region(const Geom& g)
+{
+    Flat r;
+    r.hy = g.hiy - g.loy;
+    r.hz = g.hiz - g.loz;
+    r.n = (unsigned)(g.hix - g.lox) * (unsigned)r.hy * (unsigned)r.hz;
+    r.dy = flat_div((unsigned)r.hy);
+    r.dz = flat_div((unsigned)r.hz);
+    return r;
+}
+
+// Threads per block of the flat kernels: 256, and fewer where 256 would leave
+// fewer than four blocks for each of the 152 SMs (a warp keeps a quarter of an
+// SM's FP64 pipe busy by itself, so a small lattice is as fast as its warps are
+// spread: caller-owned 24^3 steps took 25.6 us with 256-thread blocks).
+inline int flat_block(unsigned n)
+{
+    int b = 256;
+    while (b > 32 && (n + b - 1) / b < 4 * 152) b /= 2;
+    return b;
+}
+inline int flat_grid(unsigned n)
+{
+    const unsigned b = (unsigned)flat_block(n);
+    return (int)((n + b - 1) / b);
+}
+// (energy, |G|) pairs a handle's diagnostic steps may write
+inline int64_t partial_pairs(const Geom& g)
+{
+    const int64_t tiles = tile_count(g), flat = flat_grid(flat_region(g).n);
+    return tiles > flat ? tiles : flat;
+}
+
 // ---------------------------------------------------------------------------
 // per-step coefficients.  Each is the exact double the reference evaluates
 // (same operands, same order), so an FP64 kernel reproduces its arithmetic.
@@ -148,8 +209,9 @@ cudaError_t launch_absorb_tt(const Geom&, int elem, void* const* now, void* cons
 cudaError_t launch_absorb_update(const Geom&, int elem, void* const* now, void* const* past, const void* tt,
                                  double dt2, cudaStream_t);
 
-// deterministic sum of per-block partials into out[0..1] (energy, |G|)
-cudaError_t launch_finalize(const double* partials, int nblocks, double* out, cudaStream_t);
+// deterministic sum of per-block partials into out[0..1] (energy, |G|); the
+// partials are overwritten.  *launches receives the kernels launched.
+cudaError_t launch_finalize(double* partials, int nblocks, double* out, cudaStream_t, int* launches);
 
 // conversions between the double host layout and FP32 device fields
 cudaError_t launch_d2f(const double* in, float* out, int64_t n, cudaStream_t);

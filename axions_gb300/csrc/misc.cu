@@ -10,27 +10,32 @@ namespace lat {
 
 namespace {
 
-// One block sums the (energy, |G|) pairs of all blocks: every thread walks a
-// fixed strided subset with Neumaier compensation, then a fixed tree combines
-// the threads.  The result does not depend on timing, only on the grid.
-__global__ void __launch_bounds__(1024) finalize_kernel(const double* __restrict__ partials, int nblocks,
-                                                        double* __restrict__ out)
+// Sums of (energy, |G|) pairs: every block takes `per` of the n pairs (`step`
+// pairs apart), every thread a fixed strided subset of them with Neumaier
+// compensation, then a fixed tree combines the threads.  The result does not
+// depend on timing, only on n.  A block's sum goes to out[2*b*out_step].
+constexpr int FIN_THREADS = 256;
+constexpr int FIN_PER = 4096;  // pairs per block
+
+__global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const double* partials, int n, int step, int per,
+                                                               double* out, int out_step)
 {
-    __shared__ double se[1024], sg[1024];
+    __shared__ double se[FIN_THREADS], sg[FIN_THREADS];
+    const int end = min(n, ((int)blockIdx.x + 1) * per);
     double e = 0, ce = 0, g = 0, cg = 0;
-    for (int b = threadIdx.x; b < nblocks; b += 1024) {
-        const double x = partials[2 * b], y = partials[2 * b + 1];
-        double t = e + x;
-        ce += (fabs(e) >= fabs(x)) ? (e - t) + x : (x - t) + e;
+    for (int b = (int)blockIdx.x * per + (int)threadIdx.x; b < end; b += FIN_THREADS) {
+        const double2 v = *reinterpret_cast<const double2*>(partials + 2 * (size_t)b * step);
+        double t = e + v.x;
+        ce += (fabs(e) >= fabs(v.x)) ? (e - t) + v.x : (v.x - t) + e;
         e = t;
-        t = g + y;
-        cg += (fabs(g) >= fabs(y)) ? (g - t) + y : (y - t) + g;
+        t = g + v.y;
+        cg += (fabs(g) >= fabs(v.y)) ? (g - t) + v.y : (v.y - t) + g;
         g = t;
     }
     se[threadIdx.x] = e + ce;
     sg[threadIdx.x] = g + cg;
-    __syncthreads();
-    for (int w = 512; w > 0; w >>= 1) {
+    __syncthreads();  // also: every pair of the block has been read before one is overwritten below
+    for (int w = FIN_THREADS / 2; w > 0; w >>= 1) {
         if ((int)threadIdx.x < w) {
             se[threadIdx.x] += se[threadIdx.x + w];
             sg[threadIdx.x] += sg[threadIdx.x + w];
@@ -38,8 +43,8 @@ __global__ void __launch_bounds__(1024) finalize_kernel(const double* __restrict
         __syncthreads();
     }
     if (threadIdx.x == 0) {
-        out[0] = se[0];
-        out[1] = sg[0];
+        out[2 * (size_t)blockIdx.x * out_step] = se[0];
+        out[2 * (size_t)blockIdx.x * out_step + 1] = sg[0];
     }
 }
 
@@ -79,9 +84,22 @@ inline unsigned grid_for(int64_t n)
 
 }  // namespace
 
-cudaError_t launch_finalize(const double* partials, int nblocks, double* out, cudaStream_t st)
+// One block up to FIN_PER pairs; above, blocks of FIN_PER pairs leave their sum
+// in their first pair, until one block's worth is left.  A single block walked
+// all of a large lattice's pairs before: 0.90 ms for the 221,184 of a 384^3
+// step, as much as 1/20 of the step itself; 42 us at 128^3.
+cudaError_t launch_finalize(double* partials, int nblocks, double* out, cudaStream_t st, int* launches)
 {
-    finalize_kernel<<<1, 1024, 0, st>>>(partials, nblocks, out);
+    int n = nblocks, step = 1;
+    *launches = 1;
+    while (n > FIN_PER) {
+        const int blocks = (n + FIN_PER - 1) / FIN_PER;
+        finalize_kernel<<<blocks, FIN_THREADS, 0, st>>>(partials, n, step, FIN_PER, partials, step * FIN_PER);
+        ++*launches;
+        n = blocks;
+        step *= FIN_PER;
+    }
+    finalize_kernel<<<1, FIN_THREADS, 0, st>>>(partials, n, step, FIN_PER, out, 1);
     return cudaGetLastError();
 }
 

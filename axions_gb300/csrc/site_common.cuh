@@ -83,6 +83,43 @@ __device__ __forceinline__ Nbr make_nbr(const Geom& g, int i, int j, int k)
     return n;
 }
 
+// Site q of a flat region (Flat of lattice_internal.cuh)
+__device__ __forceinline__ Nbr flat_nbr(const Geom& g, const Flat& r, unsigned q)
+{
+    const unsigned row = (__umulhi(q, r.dz.mul) + q) >> r.dz.shift;
+    const unsigned plane = (__umulhi(row, r.dy.mul) + row) >> r.dy.shift;
+    return make_nbr(g, g.lox + (int)plane, g.loy + (int)(row - plane * (unsigned)r.hy),
+                    g.loz + (int)(q - row * (unsigned)r.hz));
+}
+
+// Sum two doubles over a one-dimensional block (a power of two of threads, at
+// most BLOCK) and write them to partials[2*b], partials[2*b+1].  Fixed tree:
+// deterministic for a fixed grid.
+__device__ __forceinline__ void flat_sum2_store(double a, double b, double* partials)
+{
+    __shared__ double red[2][BLOCK / 32];
+    const int tid = threadIdx.x;
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+        a += __shfl_down_sync(0xffffffffu, a, o);
+        b += __shfl_down_sync(0xffffffffu, b, o);
+    }
+    if ((tid & 31) == 0) {
+        red[0][tid >> 5] = a;
+        red[1][tid >> 5] = b;
+    }
+    __syncthreads();
+    if (tid == 0) {
+        double sa = 0, sb = 0;
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+            sa += red[0][w];
+            sb += red[1][w];
+        }
+        partials[2 * blockIdx.x] = sa;
+        partials[2 * blockIdx.x + 1] = sb;
+    }
+}
+
 // Sum two doubles over the block (BLOCK threads) and write them to
 // partials[2*b], partials[2*b+1].  Fixed tree: deterministic for a fixed grid.
 __device__ __forceinline__ void block_sum2_store(double a, double b, double* partials)
