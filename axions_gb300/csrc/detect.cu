@@ -3,198 +3,268 @@
 // 1. Bilinear face crossings (mpi_evolution.cpp:536-789, evolution.cpp:749-1004):
 //    each site checks its three positive faces; each face's bilinear
 //    interpolation of (Re phi, Im phi) is inverted through a quadratic.  The
-//    reference appends roots to per-rank vectors; here a count pass, a scan of
-//    block totals and a write pass put every crossing at its position in the
-//    reference's order (sites in linear order; z-, y-, x-directed face; "+"
-//    root before "-" root) with no sort.  All arithmetic is double precision in
-//    the reference's order and this file is compiled with -fmad=false, so the
-//    output is bit-identical to the reference on identical fields.
+//    reference appends roots to per-rank vectors; here a pass that finds and
+//    counts them, a scan of block totals and a pass that places them put every
+//    crossing at its position in the reference's order (sites in linear order;
+//    z-, y-, x-directed face; "+" root before "-" root) with no sort.  A face's
+//    roots are found in double precision in the reference's order of operations
+//    and this file is compiled with -fmad=false, so the output is bit-identical
+//    to the reference on identical fields; faces that provably have none are
+//    left out of that by an FP32 test.
 // 2. Plaquette winding (new, defined in include/lattice_gpu.h).
+#include "detect_face.cuh"
 #include "lattice_internal.cuh"
 
 namespace lat {
 
 namespace {
 
-constexpr int DB = 256;  // sites (threads) per detection block
+constexpr int DB = 256;           // threads per detection block
+constexpr int DR = 4;             // sites per thread
+constexpr int DSITES = DB * DR;   // sites per detection block
+constexpr int DWARPS = DB / 32;
+constexpr int DCHUNKS = 3 * DR;   // most chunks of DB candidate faces in a block
 
-struct Roots {
-    int n;
-    double s1[2], s2[2];
+// Offsets to the forward neighbours of site s, and whether it is examined.
+struct Site {
+    int i, j, k, xp, yp, zp;
 };
 
-// One face: v00 at (u,w), v10 at (u+du,w), v01 at (u,w+dw), v11 at (u+du,w+dw).
-__device__ __forceinline__ Roots face_roots(const double v00[2], const double v10[2], const double v01[2],
-                                            const double v11[2], double u, double w, double du, double dw)
+__device__ __forceinline__ bool site_at(const DetectArgs& a, long long sl, Site& o)
 {
-    double coeff1[2], coeff2[2], coeff3[2], coeff4[2];
-#pragma unroll
-    for (int comp = 0; comp < 2; ++comp) {
-        coeff1[comp] = v11[comp] - v10[comp] - v01[comp] + v00[comp];
-        coeff2[comp] = (w + dw) * (v10[comp] - v00[comp]) + w * (v01[comp] - v11[comp]);
-        coeff3[comp] = (u + du) * (v01[comp] - v00[comp]) + u * (v10[comp] - v11[comp]);
-        coeff4[comp] = (u + du) * ((w + dw) * v00[comp] - w * v01[comp]) - u * ((w + dw) * v10[comp] - w * v11[comp]);
-    }
-    const double a = coeff1[1] * coeff3[0] - coeff1[0] * coeff3[1];
-    const double b = coeff1[1] * coeff4[0] + coeff2[1] * coeff3[0] - coeff1[0] * coeff4[1] - coeff2[0] * coeff3[1];
-    const double c = coeff2[1] * coeff4[0] - coeff2[0] * coeff4[1];
-    const double discrim = b * b - 4 * a * c;
-    Roots r;
-    r.n = 0;
-    if (a == 0) {
-        if (b != 0) {
-            const double sol2 = -c / b;
-            if (sol2 >= w && sol2 <= w + dw) {
-                const double sol1 = -(coeff3[0] * sol2 + coeff4[0]) / (coeff1[0] * sol2 + coeff2[0]);
-                if (sol1 >= u && sol1 <= u + du) { r.s1[r.n] = sol1; r.s2[r.n] = sol2; r.n++; }
-            }
-        }
-    } else if (discrim >= 0) {
-        const double sq = sqrt(discrim);
-        double sol2 = (-b + sq) / (2 * a);
-        if (sol2 >= w && sol2 <= w + dw) {
-            const double sol1 = -(coeff3[0] * sol2 + coeff4[0]) / (coeff1[0] * sol2 + coeff2[0]);
-            if (sol1 >= u && sol1 <= u + du) { r.s1[r.n] = sol1; r.s2[r.n] = sol2; r.n++; }
-        }
-        sol2 = (-b - sq) / (2 * a);
-        if (sol2 >= w && sol2 <= w + dw) {
-            const double sol1 = -(coeff3[0] * sol2 + coeff4[0]) / (coeff1[0] * sol2 + coeff2[0]);
-            if (sol1 >= u && sol1 <= u + du) { r.s1[r.n] = sol1; r.s2[r.n] = sol2; r.n++; }
-        }
-    }
-    return r;
-}
-
-struct SiteRoots {
-    Roots zf, yf, xf;
-    double x, y, z;
-    int total;
-};
-
-template <class T>
-__device__ __forceinline__ bool site_roots(const DetectArgs& a, const T* __restrict__ re, const T* __restrict__ im,
-                                           long long sl, SiteRoots& out)
-{
-    const long long N = (long long)a.nx * a.syz;
-    if (sl >= N) return false;
+    if (sl >= (long long)a.nx * a.syz) return false;
     const int s = (int)sl;
-    const int i = s / a.syz;
-    const int rem = s - i * a.syz;
-    const int j = rem / a.nz;
-    const int k = rem - j * a.nz;
-    if (i < a.lox || i >= a.hix || j < a.loy || j >= a.hiy || k < a.loz || k >= a.hiz) return false;
-    const int oxp = (i + 1 == a.nx) ? -(a.nx - 1) * a.syz : a.syz;
-    const int oyp = (j + 1 == a.ny) ? -(a.ny - 1) * a.nz : a.nz;
-    const int ozp = (k + 1 == a.nz) ? -(a.nz - 1) : 1;
-    double v0[2], vx[2], vy[2], vz[2], vxy[2], vxz[2], vyz[2];
-    v0[0] = (double)re[s];           v0[1] = (double)im[s];
-    vx[0] = (double)re[s + oxp];     vx[1] = (double)im[s + oxp];
-    vy[0] = (double)re[s + oyp];     vy[1] = (double)im[s + oyp];
-    vz[0] = (double)re[s + ozp];     vz[1] = (double)im[s + ozp];
-    vxy[0] = (double)re[s + oxp + oyp]; vxy[1] = (double)im[s + oxp + oyp];
-    vxz[0] = (double)re[s + oxp + ozp]; vxz[1] = (double)im[s + oxp + ozp];
-    vyz[0] = (double)re[s + oyp + ozp]; vyz[1] = (double)im[s + oyp + ozp];
-    // physical coordinates (mpi_evolution.cpp:547-549)
-    out.x = (double)(i - a.x0) * a.dx;
-    out.y = (double)(j - a.y0) * a.dy;
-    out.z = (double)(k - a.z0) * a.dz;
-    out.zf = face_roots(v0, vx, vy, vxy, out.x, out.y, a.dx, a.dy);   // z-directed face (x,y)
-    out.yf = face_roots(v0, vx, vz, vxz, out.x, out.z, a.dx, a.dz);   // y-directed face (x,z)
-    out.xf = face_roots(v0, vy, vz, vyz, out.y, out.z, a.dy, a.dz);   // x-directed face (y,z)
-    out.total = out.zf.n + out.yf.n + out.xf.n;
-    return true;
+    o.i = s / a.syz;
+    const int rem = s - o.i * a.syz;
+    o.j = rem / a.nz;
+    o.k = rem - o.j * a.nz;
+    o.xp = (o.i + 1 == a.nx) ? -(a.nx - 1) * a.syz : a.syz;
+    o.yp = (o.j + 1 == a.ny) ? -(a.ny - 1) * a.nz : a.nz;
+    o.zp = (o.k + 1 == a.nz) ? -(a.nz - 1) : 1;
+    return o.i >= a.lox && o.i < a.hix && o.j >= a.loy && o.j < a.hiy && o.k >= a.loz && o.k < a.hiz;
 }
 
-__device__ __forceinline__ int block_exclusive_scan(int v, int* total)
+// Roots found by the count pass, so that the write pass need not evaluate the
+// faces again: chunk c of block b put `count` triples at `base` of the stash.
+struct StashChunk {
+    unsigned base, count;
+};
+
+// a stash: 16 bytes (the counter), the blocks' chunk records, the triples
+inline StashChunk* stash_chunks(const DetectStash& sh) { return (StashChunk*)((char*)sh.buf + 16); }
+inline double* stash_xyz(const DetectStash& sh, int nb)
 {
-    __shared__ int warp_sums[DB / 32];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    int incl = v;
+    return (double*)((char*)sh.buf + 16 + sizeof(StashChunk) * DCHUNKS * (size_t)nb);
+}
+
+enum DetectMode { DETECT_COUNT, DETECT_STASH, DETECT_WRITE };
+
+// Sites [blockIdx.x*DSITES, +DSITES): candidate faces are listed in the
+// reference's order (sites in linear order; z-, y-, x-directed face), then
+// evaluated DB at a time.  COUNT: the block's number of crossings to totals;
+// STASH: the same, and the crossings to the stash (`used` counts them, beyond
+// `cap` they are not stored); WRITE: the crossings to xyz at totals (scanned).
+template <class T, int MODE>
+__global__ void __launch_bounds__(DB) detect_kernel(const DetectArgs a, const T* __restrict__ re,
+                                                    const T* __restrict__ im, const float eref, long long* totals,
+                                                    double* __restrict__ xyz, long long cap, unsigned* used,
+                                                    StashChunk* __restrict__ chunks)
+{
+    __shared__ unsigned short list[3 * DSITES];   // site within the block * 4 + face
+    __shared__ int wsum[DR * DWARPS];             // candidates of warp w, round r at [r*DWARPS + w]
+    __shared__ int csum[DWARPS];                  // crossings of a warp in the current chunk
+    __shared__ unsigned s_base;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const long long first = (long long)blockIdx.x * DSITES;
+
+    unsigned mask[DR];
 #pragma unroll
-    for (int o = 1; o < 32; o <<= 1) {
-        const int t = __shfl_up_sync(0xffffffffu, incl, o);
-        if (lane >= o) incl += t;
+    for (int r = 0; r < DR; ++r) {
+        Site o;
+        const long long sl = first + r * DB + tid;
+        mask[r] = 0;
+        if (site_at(a, sl, o)) {
+            const int s = (int)sl;
+            auto at = [&](int off) { return Corner{corner_float(re[s + off]), corner_float(im[s + off])}; };
+            const Corner v0 = at(0), vx = at(o.xp), vy = at(o.yp), vz = at(o.zp);
+            if (face_maybe(v0, vx, vy, at(o.xp + o.yp), eref)) mask[r] |= 1u;   // z-directed face (x,y)
+            if (face_maybe(v0, vx, vz, at(o.xp + o.zp), eref)) mask[r] |= 2u;   // y-directed face (x,z)
+            if (face_maybe(v0, vy, vz, at(o.yp + o.zp), eref)) mask[r] |= 4u;   // x-directed face (y,z)
+        }
+        int n = 0;
+#pragma unroll
+        for (int f = 0; f < 3; ++f) n += __popc(__ballot_sync(0xffffffffu, (mask[r] >> f) & 1u));
+        if (lane == 0) wsum[r * DWARPS + wid] = n;
     }
-    if (lane == 31) warp_sums[wid] = incl;
     __syncthreads();
+    static_assert(DR * DWARPS == 32, "one warp scans the warps' candidate counts");
     if (wid == 0) {
-        int ws = (lane < DB / 32) ? warp_sums[lane] : 0;
+        const int own = wsum[lane];
+        int incl = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const int t = __shfl_up_sync(0xffffffffu, ws, o);
-            if (lane >= o) ws += t;
+            const int t = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += t;
         }
-        if (lane < DB / 32) warp_sums[lane] = ws;  // inclusive over warps
+        wsum[lane] = incl - own;
+        if (lane == 31) s_base = (unsigned)incl;
     }
     __syncthreads();
-    const int warp_base = wid ? warp_sums[wid - 1] : 0;
-    if (total) *total = warp_sums[DB / 32 - 1];
-    return warp_base + incl - v;
-}
+    const int m = (int)s_base;
+#pragma unroll
+    for (int r = 0; r < DR; ++r) {
+        int pos = wsum[r * DWARPS + wid];
+        const unsigned below = (1u << lane) - 1u;
+#pragma unroll
+        for (int f = 0; f < 3; ++f) pos += __popc(__ballot_sync(0xffffffffu, (mask[r] >> f) & 1u) & below);
+#pragma unroll
+        for (int f = 0; f < 3; ++f)
+            if (mask[r] >> f & 1u) list[pos++] = (unsigned short)((r * DB + tid) * 4 + f);
+    }
+    __syncthreads();
 
-template <class T>
-__global__ void __launch_bounds__(DB) detect_count_kernel(const DetectArgs a, const T* __restrict__ re,
-                                                          const T* __restrict__ im, long long* block_totals)
-{
-    SiteRoots r;
-    const long long sl = (long long)blockIdx.x * DB + threadIdx.x;
-    const int cnt = site_roots<T>(a, re, im, sl, r) ? r.total : 0;
-    int total;
-    block_exclusive_scan(cnt, &total);
-    if (threadIdx.x == 0) block_totals[blockIdx.x] = total;
-}
-
-template <class T>
-__global__ void __launch_bounds__(DB) detect_write_kernel(const DetectArgs a, const T* __restrict__ re,
-                                                          const T* __restrict__ im, const long long* block_offsets,
-                                                          double* xyz, long long cap)
-{
-    SiteRoots r;
-    const long long sl = (long long)blockIdx.x * DB + threadIdx.x;
-    const bool ok = site_roots<T>(a, re, im, sl, r);
-    const int cnt = ok ? r.total : 0;
-    long long pos = block_offsets[blockIdx.x] + block_exclusive_scan(cnt, nullptr);
-    if (!ok) return;
-    auto emit = [&](double x, double y, double z) {
-        if (pos < cap) {
-            xyz[3 * pos + 0] = x;
-            xyz[3 * pos + 1] = y;
-            xyz[3 * pos + 2] = z;
+    long long run = MODE == DETECT_WRITE ? totals[blockIdx.x] : 0;   // crossings before the chunk
+    int mine = 0;
+    for (int c0 = 0; c0 < m; c0 += DB) {
+        Roots q;
+        q.n = 0;
+        int face = 0;
+        double x = 0, y = 0, z = 0;
+        if (c0 + tid < m) {
+            const int item = list[c0 + tid];
+            face = item & 3;
+            Site o;
+            const long long sl = first + (item >> 2);
+            site_at(a, sl, o);
+            const int s = (int)sl;
+            // physical coordinates (mpi_evolution.cpp:547-549)
+            x = (double)(o.i - a.x0) * a.dx;
+            y = (double)(o.j - a.y0) * a.dy;
+            z = (double)(o.k - a.z0) * a.dz;
+            const int d1 = face == 2 ? o.yp : o.xp, d2 = face == 0 ? o.yp : o.zp;
+            const double v00[2] = {(double)re[s], (double)im[s]};
+            const double v10[2] = {(double)re[s + d1], (double)im[s + d1]};
+            const double v01[2] = {(double)re[s + d2], (double)im[s + d2]};
+            const double v11[2] = {(double)re[s + d1 + d2], (double)im[s + d1 + d2]};
+            q = face_roots(v00, v10, v01, v11, face == 2 ? y : x, face == 0 ? y : z, face == 2 ? a.dy : a.dx,
+                           face == 0 ? a.dy : a.dz);
         }
-        ++pos;
-    };
-    for (int q = 0; q < r.zf.n; ++q) emit(r.zf.s1[q], r.zf.s2[q], r.z);
-    for (int q = 0; q < r.yf.n; ++q) emit(r.yf.s1[q], r.y, r.yf.s2[q]);
-    for (int q = 0; q < r.xf.n; ++q) emit(r.x, r.xf.s1[q], r.xf.s2[q]);
+        if constexpr (MODE == DETECT_COUNT) {
+            mine += q.n;
+        } else {
+            const unsigned one = __ballot_sync(0xffffffffu, q.n & 1), two = __ballot_sync(0xffffffffu, q.n & 2);
+            if (lane == 0) csum[wid] = __popc(one) + 2 * __popc(two);
+            __syncthreads();
+            int before = 0, all = 0;
+#pragma unroll
+            for (int w = 0; w < DWARPS; ++w) {
+                if (w < wid) before += csum[w];
+                all += csum[w];
+            }
+            const unsigned below = (1u << lane) - 1u;
+            before += __popc(one & below) + 2 * __popc(two & below);
+            long long pos;
+            if constexpr (MODE == DETECT_STASH) {
+                if (tid == 0) {
+                    s_base = all ? atomicAdd(used, (unsigned)all) : 0u;
+                    chunks[(size_t)blockIdx.x * DCHUNKS + c0 / DB] = StashChunk{s_base, (unsigned)all};
+                }
+                __syncthreads();
+                pos = (long long)s_base + before;
+            } else {
+                pos = run + before;
+            }
+            for (int t = 0; t < q.n; ++t, ++pos) {
+                if (pos >= cap) break;
+                xyz[3 * pos + 0] = face == 2 ? x : q.s1[t];
+                xyz[3 * pos + 1] = face == 0 ? q.s2[t] : (face == 1 ? y : q.s1[t]);
+                xyz[3 * pos + 2] = face == 0 ? z : q.s2[t];
+            }
+            run += all;
+            __syncthreads();  // csum and s_base are rewritten by the next chunk
+        }
+    }
+    if constexpr (MODE == DETECT_STASH) {
+        for (int c = (m + DB - 1) / DB + tid; c < DCHUNKS; c += DB)
+            chunks[(size_t)blockIdx.x * DCHUNKS + c] = StashChunk{0u, 0u};
+        if (tid == 0) totals[blockIdx.x] = run;
+    }
+    if constexpr (MODE == DETECT_COUNT) {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) mine += __shfl_down_sync(0xffffffffu, mine, o);
+        if (lane == 0) csum[wid] = mine;
+        __syncthreads();
+        if (tid == 0) {
+            int all = 0;
+            for (int w = 0; w < DWARPS; ++w) all += csum[w];
+            totals[blockIdx.x] = all;
+        }
+    }
+}
+
+// The stashed crossings of every block to their places (offsets: the scanned
+// totals); those at `cap` and beyond are left out.
+__global__ void __launch_bounds__(DB) detect_place_kernel(const double* __restrict__ stash,
+                                                          const StashChunk* __restrict__ chunks,
+                                                          const long long* __restrict__ offsets, double* __restrict__ xyz,
+                                                          long long cap)
+{
+    long long pos = offsets[blockIdx.x];
+    for (int c = 0; c < DCHUNKS; ++c) {
+        const StashChunk k = chunks[(size_t)blockIdx.x * DCHUNKS + c];
+        if (k.count == 0) continue;
+        const long long room = cap - pos;
+        const int n = 3 * (int)(room < (long long)k.count ? (room > 0 ? room : 0) : (long long)k.count);
+        for (int t = threadIdx.x; t < n; t += DB) xyz[3 * pos + t] = stash[3 * (size_t)k.base + t];
+        pos += k.count;
+    }
 }
 
 // Exclusive scan of block totals in place (one block); *total = grand total.
+// Tiles of 4096, four consecutive values a thread.
 __global__ void __launch_bounds__(1024) scan_totals_kernel(long long* v, int n, long long* total)
 {
-    __shared__ long long chunk_sum[1024];
-    const int t = threadIdx.x;
-    const int per = (n + 1023) / 1024;
-    const int b = t * per, e = min(n, b + per);
-    long long s = 0;
-    for (int q = b; q < e; ++q) s += v[q];
-    chunk_sum[t] = s;
-    __syncthreads();
-    if (t == 0) {
-        long long run = 0;
-        for (int q = 0; q < 1024; ++q) {
-            const long long c = chunk_sum[q];
-            chunk_sum[q] = run;
-            run += c;
+    __shared__ long long ws[32];
+    const int t = threadIdx.x, lane = t & 31, wid = t >> 5;
+    long long carry = 0;
+    for (int base = 0; base < n; base += 4096) {
+        long long own[4], sum = 0;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int q = base + 4 * t + r;
+            own[r] = q < n ? v[q] : 0;
+            sum += own[r];
         }
-        *total = run;
+        long long incl = sum;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const long long u = __shfl_up_sync(0xffffffffu, incl, o);
+            if (lane >= o) incl += u;
+        }
+        if (lane == 31) ws[wid] = incl;
+        __syncthreads();
+        if (wid == 0) {
+            const long long w = ws[lane];
+            long long wi = w;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const long long u = __shfl_up_sync(0xffffffffu, wi, o);
+                if (lane >= o) wi += u;
+            }
+            ws[lane] = wi;  // inclusive over warps
+        }
+        __syncthreads();
+        long long run = carry + (wid ? ws[wid - 1] : 0) + incl - sum;
+#pragma unroll
+        for (int r = 0; r < 4; ++r) {
+            const int q = base + 4 * t + r;
+            if (q < n) v[q] = run;
+            run += own[r];
+        }
+        carry += ws[31];
+        __syncthreads();  // ws is rewritten by the next tile
     }
-    __syncthreads();
-    long long run = chunk_sum[t];
-    for (int q = b; q < e; ++q) {
-        const long long c = v[q];
-        v[q] = run;
-        run += c;
-    }
+    if (t == 0) *total = carry;
 }
 
 // ---------------------------------------------------------------------------
@@ -274,35 +344,67 @@ inline unsigned nblocks_of(const DetectArgs& a) { return (unsigned)(((long long)
 
 }  // namespace
 
-int detect_block_sites() { return DB; }
+namespace {
 
-cudaError_t launch_detect_count_f64(const DetectArgs& a, const double* re, const double* im, long long* bt, int nb,
-                                    cudaStream_t st)
+// 16 eps N^3 with N = the largest distance from the origin in spacings (see face_maybe)
+inline float reference_error(const DetectArgs& a)
 {
-    detect_count_kernel<double><<<nb, DB, 0, st>>>(a, re, im, bt);
+    const double n = 1 + 0.5 * (a.nx > a.ny ? (a.nx > a.nz ? a.nx : a.nz) : (a.ny > a.nz ? a.ny : a.nz));
+    const double e = 16 * 1.1102230246251565e-16 * n * n * n;
+    return (float)(e < 1 ? e : 1);
+}
+
+template <class T>
+cudaError_t detect_launch(const DetectArgs& a, const T* re, const T* im, long long* bt, int nb, const DetectStash& sh,
+                          double* xyz, long long cap, cudaStream_t st)
+{
+    const float e = reference_error(a);
+    if (xyz) {
+        detect_kernel<T, DETECT_WRITE><<<nb, DB, 0, st>>>(a, re, im, e, bt, xyz, cap, nullptr, nullptr);
+    } else if (sh.cap > 0) {
+        const cudaError_t m = cudaMemsetAsync(sh.buf, 0, 16, st);
+        if (m != cudaSuccess) return m;
+        detect_kernel<T, DETECT_STASH><<<nb, DB, 0, st>>>(a, re, im, e, bt, stash_xyz(sh, nb), sh.cap,
+                                                          (unsigned*)sh.buf, stash_chunks(sh));
+    } else {
+        detect_kernel<T, DETECT_COUNT><<<nb, DB, 0, st>>>(a, re, im, e, bt, nullptr, 0, nullptr, nullptr);
+    }
     return cudaGetLastError();
 }
-cudaError_t launch_detect_count_f32(const DetectArgs& a, const float* re, const float* im, long long* bt, int nb,
-                                    cudaStream_t st)
+
+}  // namespace
+
+int detect_blocks(int64_t sites) { return (int)((sites + DSITES - 1) / DSITES); }
+
+size_t detect_stash_bytes(int nb, int64_t cap)
 {
-    detect_count_kernel<float><<<nb, DB, 0, st>>>(a, re, im, bt);
+    return 16 + sizeof(StashChunk) * DCHUNKS * (size_t)nb + 24 * (size_t)cap;
+}
+
+cudaError_t launch_detect_count(const DetectArgs& a, int elem, const void* re, const void* im, long long* bt, int nb,
+                                const DetectStash& sh, cudaStream_t st)
+{
+    return elem == 8 ? detect_launch(a, (const double*)re, (const double*)im, bt, nb, sh, nullptr, 0, st)
+                     : detect_launch(a, (const float*)re, (const float*)im, bt, nb, sh, nullptr, 0, st);
+}
+
+cudaError_t launch_detect_write(const DetectArgs& a, int elem, const void* re, const void* im, long long* bo, int nb,
+                                double* xyz, long long cap, cudaStream_t st)
+{
+    return elem == 8 ? detect_launch(a, (const double*)re, (const double*)im, bo, nb, DetectStash{}, xyz, cap, st)
+                     : detect_launch(a, (const float*)re, (const float*)im, bo, nb, DetectStash{}, xyz, cap, st);
+}
+
+cudaError_t launch_detect_place(const DetectStash& sh, const long long* bo, int nb, double* xyz, long long cap,
+                                cudaStream_t st)
+{
+    detect_place_kernel<<<nb, DB, 0, st>>>(stash_xyz(sh, nb), stash_chunks(sh), bo, xyz, cap);
     return cudaGetLastError();
 }
+
 cudaError_t launch_scan_totals(long long* bt, int nb, long long* total, cudaStream_t st)
 {
     scan_totals_kernel<<<1, 1024, 0, st>>>(bt, nb, total);
-    return cudaGetLastError();
-}
-cudaError_t launch_detect_write_f64(const DetectArgs& a, const double* re, const double* im, const long long* bo, int nb,
-                                    double* xyz, long long cap, cudaStream_t st)
-{
-    detect_write_kernel<double><<<nb, DB, 0, st>>>(a, re, im, bo, xyz, cap);
-    return cudaGetLastError();
-}
-cudaError_t launch_detect_write_f32(const DetectArgs& a, const float* re, const float* im, const long long* bo, int nb,
-                                    double* xyz, long long cap, cudaStream_t st)
-{
-    detect_write_kernel<float><<<nb, DB, 0, st>>>(a, re, im, bo, xyz, cap);
     return cudaGetLastError();
 }
 cudaError_t launch_winding_f64(const DetectArgs& a, int open_axes, const double* re, const double* im, int8_t* out,

@@ -1,6 +1,7 @@
 // C ABI of liblattice_gpu.so (include/lattice_gpu.h): handle management,
 // state transfer and the per-step orchestration that replaces the body of the
 // reference's time-step loop (mpi_evolution.cpp:354-985 and its relatives).
+#include <algorithm>
 #include <cmath>
 #include <cstdio>
 #include <cstring>
@@ -353,6 +354,7 @@ int lat_destroy(lat_handle* h)
     cudaFree(h->det_blocks);
     cudaFree(h->det_total);
     cudaFree(h->det_xyz);
+    cudaFree(h->det_stash);
     cudaFree(h->wind);
     cudaFree(h->wind_sum);
     chain_buffers_release(h->chain, nullptr);
@@ -743,14 +745,40 @@ static DetectArgs detect_args(const lat_handle* h)
     return a;
 }
 
-// count the crossings of `field` on the current level (block totals scanned in place)
-static int detect_count(lat_handle* h, int32_t field, int64_t* total_out)
+// Room for the crossings a count pass finds (launch_detect_write would find
+// them a second time): up to 2^21, 50 MB, which holds a noisy 128^3 level or
+// the strings of a 512^3 one; fewer where the caller wants fewer or the
+// lattice is small.  Without memory for it, or with more crossings than that,
+// they are found twice.
+static DetectStash detect_stash(lat_handle* h, int nb, int64_t want)
+{
+    const int64_t cap = std::min(std::min(want, 2 * h->N), (int64_t)1 << 21);
+    if (cap <= 0) return DetectStash{};
+    const size_t bytes = detect_stash_bytes(nb, cap);
+    if (bytes > h->det_stash_bytes) {
+        dev_free(h, &h->det_stash, h->det_stash_bytes);
+        h->det_stash_bytes = 0;
+        if (cudaMalloc(&h->det_stash, bytes) != cudaSuccess) {
+            cudaGetLastError();
+            h->det_stash = nullptr;
+            return DetectStash{};
+        }
+        h->det_stash_bytes = bytes;
+        h->bytes += (int64_t)bytes;
+    }
+    return DetectStash{h->det_stash, cap};
+}
+
+// count the crossings of `field` on the current level (block totals scanned in
+// place); `want` of them are to be written afterwards, *sh tells detect_write
+// where they are kept
+static int detect_count(lat_handle* h, int32_t field, int64_t want, int64_t* total_out, DetectStash* sh)
 {
     int rc0 = ensure_boundaries(h);
     if (rc0) return rc0;
     const DetectArgs a = detect_args(h);
     const int tNow = (int)((h->n + 1) % 2);
-    const int nb = (int)((h->N + detect_block_sites() - 1) / detect_block_sites());
+    const int nb = detect_blocks(h->N);
     if (nb > h->det_nb) {
         dev_free(h, (void**)&h->det_blocks, sizeof(long long) * (size_t)h->det_nb);
         h->det_nb = 0;
@@ -758,10 +786,10 @@ static int detect_count(lat_handle* h, int32_t field, int64_t* total_out)
         if (rc) return rc;
         h->det_nb = nb;
     }
+    *sh = detect_stash(h, nb, want);
     const void* re = h->slot(2 * field, tNow);
     const void* im = h->slot(2 * field + 1, tNow);
-    if (h->elem == 8) LAT_CKL(launch_detect_count_f64(a, (const double*)re, (const double*)im, h->det_blocks, nb, h->stream));
-    else LAT_CKL(launch_detect_count_f32(a, (const float*)re, (const float*)im, h->det_blocks, nb, h->stream));
+    LAT_CKL(launch_detect_count(a, (int)h->elem, re, im, h->det_blocks, nb, *sh, h->stream));
     LAT_CKL(launch_scan_totals(h->det_blocks, nb, h->det_total, h->stream));
     long long total = 0;
     LAT_CK(cudaMemcpyAsync(&total, h->det_total, sizeof(total), cudaMemcpyDeviceToHost, h->stream));
@@ -770,8 +798,8 @@ static int detect_count(lat_handle* h, int32_t field, int64_t* total_out)
     return LAT_OK;
 }
 
-// write the first nw crossings (after detect_count) into h->det_xyz
-static int detect_write(lat_handle* h, int32_t field, int64_t nw)
+// write the first nw of the `total` crossings (after detect_count) into h->det_xyz
+static int detect_write(lat_handle* h, int32_t field, int64_t total, int64_t nw, const DetectStash& sh)
 {
     if (nw <= 0) return LAT_OK;
     if (nw > h->det_cap) {
@@ -781,15 +809,14 @@ static int detect_write(lat_handle* h, int32_t field, int64_t nw)
         if (rc) return rc;
         h->det_cap = nw;
     }
-    const DetectArgs a = detect_args(h);
+    const int nb = detect_blocks(h->N);
+    if (total <= sh.cap) {
+        LAT_CKL(launch_detect_place(sh, h->det_blocks, nb, h->det_xyz, nw, h->stream));
+        return LAT_OK;
+    }
     const int tNow = (int)((h->n + 1) % 2);
-    const int nb = (int)((h->N + detect_block_sites() - 1) / detect_block_sites());
-    const void* re = h->slot(2 * field, tNow);
-    const void* im = h->slot(2 * field + 1, tNow);
-    if (h->elem == 8)
-        LAT_CKL(launch_detect_write_f64(a, (const double*)re, (const double*)im, h->det_blocks, nb, h->det_xyz, nw, h->stream));
-    else
-        LAT_CKL(launch_detect_write_f32(a, (const float*)re, (const float*)im, h->det_blocks, nb, h->det_xyz, nw, h->stream));
+    LAT_CKL(launch_detect_write(detect_args(h), (int)h->elem, h->slot(2 * field, tNow), h->slot(2 * field + 1, tNow),
+                                h->det_blocks, nb, h->det_xyz, nw, h->stream));
     return LAT_OK;
 }
 
@@ -801,12 +828,13 @@ int lat_detect_crossings(lat_handle* h, int32_t field, double* xyz, int64_t cap,
     LAT_REQUIRE(cap >= 0 && (xyz || cap == 0), "lat_detect_crossings: bad capacity");
     LAT_CK(cudaSetDevice(h->device));
     int64_t total = 0;
-    int rc = detect_count(h, field, &total);
+    DetectStash sh;
+    int rc = detect_count(h, field, cap, &total, &sh);
     if (rc) return rc;
     *count = total;
     const int64_t nw = total < cap ? total : cap;
     if (nw > 0) {
-        if ((rc = detect_write(h, field, nw))) return rc;
+        if ((rc = detect_write(h, field, total, nw, sh))) return rc;
         LAT_CK(cudaMemcpyAsync(xyz, h->det_xyz, sizeof(double) * 3 * (size_t)nw, cudaMemcpyDeviceToHost, h->stream));
         LAT_CK(cudaStreamSynchronize(h->stream));
     }
@@ -829,11 +857,12 @@ int lat_string_length(lat_handle* h, int32_t field, int32_t split, int32_t metho
     LAT_CK(cudaSetDevice(h->device));
     *L0 = *L1 = 0.0;
     int64_t total = 0;
-    int rc = detect_count(h, field, &total);
+    DetectStash sh;
+    int rc = detect_count(h, field, h->N, &total, &sh);
     if (rc) return rc;
     if (count) *count = total;
     if (total == 0) return LAT_OK;
-    if ((rc = detect_write(h, field, total))) return rc;
+    if ((rc = detect_write(h, field, total, total, sh))) return rc;
     if (method == LAT_CHAIN_AUTO) method = periodic ? LAT_CHAIN_HASH : LAT_CHAIN_EXHAUSTIVE;
     const ChainGeom g = make_chain_geom(h->p, total);
     double out[2];

@@ -35,6 +35,8 @@ struct lat_handle {
     int det_nb = 0;
     double* det_xyz = nullptr;
     int64_t det_cap = 0;
+    void* det_stash = nullptr;  // crossings kept from the count (DetectStash)
+    size_t det_stash_bytes = 0;
     int8_t* wind = nullptr;
     unsigned long long* wind_sum = nullptr;
     lat::ChainBuffers chain;   // string-length buffers

@@ -223,16 +223,22 @@ struct DetectArgs {
     double dx, dy, dz;
     int x0, y0, z0;
 };
-int detect_block_sites();
-cudaError_t launch_detect_count_f64(const DetectArgs&, const double* re, const double* im, long long* block_totals,
-                                    int nblocks, cudaStream_t);
-cudaError_t launch_detect_count_f32(const DetectArgs&, const float* re, const float* im, long long* block_totals,
-                                    int nblocks, cudaStream_t);
+// device buffer that keeps the crossings a count found, unordered, so that they
+// need not be found again to be written (cap triples; 0: none)
+struct DetectStash {
+    void* buf = nullptr;
+    int64_t cap = 0;
+};
+int detect_blocks(int64_t sites);                       // detection blocks of a lattice
+size_t detect_stash_bytes(int nblocks, int64_t cap);
+cudaError_t launch_detect_count(const DetectArgs&, int elem, const void* re, const void* im, long long* block_totals,
+                                int nblocks, const DetectStash&, cudaStream_t);
 cudaError_t launch_scan_totals(long long* block_totals, int nblocks, long long* total, cudaStream_t);
-cudaError_t launch_detect_write_f64(const DetectArgs&, const double* re, const double* im, const long long* block_offsets,
-                                    int nblocks, double* xyz, long long cap, cudaStream_t);
-cudaError_t launch_detect_write_f32(const DetectArgs&, const float* re, const float* im, const long long* block_offsets,
-                                    int nblocks, double* xyz, long long cap, cudaStream_t);
+// after the scan: the crossings found again, or (all of them stashed) placed
+cudaError_t launch_detect_write(const DetectArgs&, int elem, const void* re, const void* im, long long* block_offsets,
+                                int nblocks, double* xyz, long long cap, cudaStream_t);
+cudaError_t launch_detect_place(const DetectStash&, const long long* block_offsets, int nblocks, double* xyz,
+                                long long cap, cudaStream_t);
 cudaError_t launch_winding_f64(const DetectArgs&, int open_axes, const double* re, const double* im, int8_t* out,
                                unsigned long long* abs_sum, cudaStream_t);
 cudaError_t launch_winding_f32(const DetectArgs&, int open_axes, const float* re, const float* im, int8_t* out,
