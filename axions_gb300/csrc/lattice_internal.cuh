@@ -257,6 +257,8 @@ struct ChainGeom {
     int periodic[3];      // minimum image per axis (x, y from bc; z from bc_z)
     double cutoff;        // (dx*dx + dy*dy + dz*dz)^2, compared with squared distances
     double root_cutoff;   // sqrt(cutoff): the closing length the reference adds
+    float Lf[3];          // L, and the squared FP32 distance beyond which
+    float near2;          // two crossings are certainly out of reach
     int nnb;              // distinct neighbour-cell offsets
     signed char off[27][3];
 };

@@ -307,37 +307,73 @@ __global__ void bin_scatter_kernel(const ChainDev c)
     c.sp[q] = s;
 }
 
-// fn(j, d2) for every crossing j != i within the cutoff of crossing i
+// v truncated to 24 bits by integer instructions (off the FP64 pipe); what is
+// below the float range becomes 0, what is above Inf.
+__device__ __forceinline__ float trunc_f(double v)
+{
+    const unsigned hi = (unsigned)__double2hiint(v), lo = (unsigned)__double2loint(v), m = hi & 0x7fffffffu;
+    const unsigned f = ((m - (896u << 20)) << 3) | (lo >> 29);
+    return __uint_as_float((m < (897u << 20) ? 0u : (m >= (1151u << 20) ? 0x7f800000u : f)) | (hi & 0x80000000u));
+}
+
+// false only if s is beyond the cutoff of (x, y, z), in FP32: g.near2 allows for
+// the truncation of the coordinates
+__device__ __forceinline__ bool near_f(const ChainGeom& g, float x, float y, float z, const ChainPt& s)
+{
+    float a = fabsf(x - trunc_f(s.x)), b = fabsf(y - trunc_f(s.y)), c = fabsf(z - trunc_f(s.z));
+    a = fminf(a, fabsf(g.Lf[0] - a));
+    b = fminf(b, fabsf(g.Lf[1] - b));
+    c = fminf(c, fabsf(g.Lf[2] - c));
+    return !(a * a + b * b + c * c > g.near2);
+}
+
+// The crossings j != i within the cutoff of crossing i, by one warp: lane k
+// walks the k-th of the at most 27 neighbour cells, all lanes in step;
+// fn(hit, j, d2) is called by the whole warp.  (One thread per crossing walked
+// 27 cells one dependent load after another: 0.67 + 0.59 ms for the two sweeps
+// over 6.7x10^4 crossings.)
 template <class F>
-__device__ __forceinline__ void for_links(const ChainDev& c, int i, F&& fn)
+__device__ __forceinline__ void for_links(const ChainDev& c, int i, int lane, F&& fn)
 {
     const double* p = c.xyz + 3 * (size_t)i;
     const double x = p[0], y = p[1], z = p[2];
-    const int b = c.bin_of[i];
-    const int iz = b % c.g.nb[2], t = b / c.g.nb[2];
-    const int iy = t % c.g.nb[1], ix = t / c.g.nb[1];
-    for (int k = 0; k < c.g.nnb; ++k) {
-        const int jx = wrap_cell(ix + c.g.off[k][0], c.g.nb[0]);
-        const int jy = wrap_cell(iy + c.g.off[k][1], c.g.nb[1]);
-        const int jz = wrap_cell(iz + c.g.off[k][2], c.g.nb[2]);
+    const float xf = trunc_f(x), yf = trunc_f(y), zf = trunc_f(z);
+    long long q = 0, q1 = 0;
+    if (lane < c.g.nnb) {
+        const int b = c.bin_of[i];
+        const int iz = b % c.g.nb[2], t = b / c.g.nb[2];
+        const int iy = t % c.g.nb[1], ix = t / c.g.nb[1];
+        const int jx = wrap_cell(ix + c.g.off[lane][0], c.g.nb[0]);
+        const int jy = wrap_cell(iy + c.g.off[lane][1], c.g.nb[1]);
+        const int jz = wrap_cell(iz + c.g.off[lane][2], c.g.nb[2]);
         const int nb = (jx * c.g.nb[1] + jy) * c.g.nb[2] + jz;
-        const long long q1 = c.bin_start[nb + 1];
-        for (long long q = c.bin_start[nb]; q < q1; ++q) {
+        q = c.bin_start[nb];
+        q1 = c.bin_start[nb + 1];
+    }
+    for (; __any_sync(FULL, q < q1); ++q) {
+        bool hit = false;
+        int j = 0;
+        double d = 0;
+        if (q < q1) {
             const ChainPt s = c.sp[q];
-            if (s.idx == i) continue;
-            const double d = chain_d2(c.g, x, y, z, s.x, s.y, s.z);
-            if (d <= c.g.cutoff) fn(s.idx, d);
+            j = s.idx;
+            if (j != i && near_f(c.g, xf, yf, zf, s)) {
+                d = chain_d2(c.g, x, y, z, s.x, s.y, s.z);
+                hit = d <= c.g.cutoff;
+            }
         }
+        fn(hit, j, d);
     }
 }
 
+// one warp per crossing
 __global__ void adj_count_kernel(const ChainDev c)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= c.M) return;
     int n = 0;
-    for_links(c, i, [&](int, double) { ++n; });
-    c.deg[i] = n;
+    for_links(c, i, lane, [&](bool hit, int, double) { n += __popc(__ballot_sync(FULL, hit)); });
+    if (lane == 0) c.deg[i] = n;
 }
 
 // ---------------------------------------------------------------------------
@@ -373,23 +409,28 @@ __device__ void unite(int* parent, int a, int b, int* err)
     atomicExch(err, CHAIN_ERR_UNION);
 }
 
-// the links of i, in the order adj_count_kernel counted them; joins the sets
+// the links of i (one warp), in the order the warp meets them; joins the sets
 __global__ void adj_fill_kernel(const ChainDev c)
 {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    const int i = (int)(((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5), lane = threadIdx.x & 31;
     if (i >= c.M) return;
     long long pos = c.adj_start[i];
-    for_links(c, i, [&](int j, double d) {
-        AdjEdge e;
-        e.d2 = (unsigned long long)__double_as_longlong(d);
-        e.start = 0;
-        e.rev = -1;
-        e.j = j;
-        e.meta = 0;
-        c.adj[pos] = e;
-        c.edge_dead[pos] = 0;
-        ++pos;
-        if (j > i) unite(c.parent, i, j, &c.counters[2]);
+    for_links(c, i, lane, [&](bool hit, int j, double d) {
+        const unsigned hits = __ballot_sync(FULL, hit);
+        if (hit) {
+            const long long at = pos + __popc(hits & ((1u << lane) - 1u));
+            AdjEdge e;
+            e.d2 = (unsigned long long)__double_as_longlong(d);
+            e.start = 0;
+            e.rev = -1;
+            e.j = j;
+            e.meta = 0;
+            c.adj[at] = e;
+            c.edge_dead[at] = 0;
+            if (j > i) unite(c.parent, i, j, &c.counters[2]);
+        }
+        __syncwarp();
+        pos += __popc(hits);
     });
 }
 
@@ -557,38 +598,94 @@ __global__ void order_kernel(const ChainDev c)
     c.ord_cls[o] = cls;
 }
 
-// the sums in the reference's order, by one thread.  Every visit adds to both
-// sums, 0.0 to the one it does not count to (x + 0.0 == x for the non-negative
-// partial sums), so the two dependent chains interleave and the loads of a
-// batch are issued together.
-__global__ void __launch_bounds__(32) sum_kernel(const ChainDev c)
+// The sums in the reference's order, bit for bit, without its serial chain of
+// additions (6.8 ms for 6.7x10^4 crossings: a dependent FP64 addition takes
+// about 100 ns on GB300 and each crossing had two).  While a sum S >= 0 stays
+// in one binade, with u the spacing of its doubles there, S + v rounds to
+// S + u*r(v), r(v) = v/u rounded to the nearest integer, whatever S is, unless
+// v/u lies halfway between two integers (the tie looks at S).  So a tile of
+// values that has no tie and does not leave the binade adds up as integers,
+// in any order; any other tile is added value by value.  Warp 0 sums the
+// values of class 0, warp 1 those of class 1.
+struct ChainSum {
+    double s = 0.0;
+
+    // r(v) for the current binade; sets *odd where the rule does not apply
+    __device__ __forceinline__ unsigned long long units(double v, int es, bool* odd) const
+    {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(v);
+        if (b == 0) return 0;
+        const int ev = (int)(b >> 52);          // v > 0: no sign
+        const int d = es - ev;
+        if (ev == 0 || d < 0) {
+            *odd = true;
+            return 0;
+        }
+        if (d > 54) return 0;
+        const unsigned long long m = (b & 0xfffffffffffffull) | 0x10000000000000ull;
+        if (d == 0) return m;
+        const unsigned long long frac = m & ((1ull << d) - 1), half = 1ull << (d - 1);
+        if (frac == half) *odd = true;
+        return (m >> d) + (frac > half);
+    }
+
+    // adds N values a lane (value of sub-tile k in v[k], lanes in order)
+    template <int N>
+    __device__ __forceinline__ void add(const double (&v)[N], int lane)
+    {
+        const unsigned long long b = (unsigned long long)__double_as_longlong(s);
+        const int es = (int)(b >> 52);
+        bool odd = es == 0 || es == 0x7ff;
+        unsigned long long r = 0;
+#pragma unroll
+        for (int k = 0; k < N; ++k) r += units(v[k], es, &odd);
+#pragma unroll
+        for (int o = 16; o; o >>= 1) r += __shfl_xor_sync(FULL, r, o);
+        const unsigned long long m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) + r;
+        if (!__any_sync(FULL, odd) && m < 0x20000000000000ull) {
+            s = __longlong_as_double((long long)(((unsigned long long)es << 52) | (m & 0xfffffffffffffull)));
+            return;
+        }
+        if constexpr (N > 1) {
+#pragma unroll
+            for (int k = 0; k < N; ++k) {
+                const double one[1] = {v[k]};
+                add<1>(one, lane);
+            }
+        } else {
+            unsigned left = __ballot_sync(FULL, v[0] != 0.0);
+            while (left) {
+                s += __shfl_sync(FULL, v[0], __ffs(left) - 1);
+                left &= left - 1;
+            }
+        }
+    }
+};
+
+__global__ void __launch_bounds__(64) sum_kernel(const ChainDev c)
 {
-    if (threadIdx.x != 0) return;
-    constexpr int B = 16;
-    double L0 = 0.0, L1 = 0.0;
-    int base = 0;
-    for (; base + B <= c.M; base += B) {
-        double v[B];
-        unsigned char k[B];
+    constexpr int N = 16;
+    const int lane = threadIdx.x & 31, cls = threadIdx.x >> 5;
+    ChainSum sum;
+    double v[N];
+    unsigned char k[N];
+    auto load = [&](int base) {
 #pragma unroll
-        for (int u = 0; u < B; ++u) {
-            v[u] = c.ord_val[base + u];
-            k[u] = c.ord_cls[base + u];
+        for (int u = 0; u < N; ++u) {
+            const int q = min(base + 32 * u + lane, c.M - 1);
+            v[u] = c.ord_val[q];
+            k[u] = base + 32 * u + lane < c.M ? c.ord_cls[q] : 2;
         }
+    };
+    load(0);
+    for (int base = 0; base < c.M; base += 32 * N) {
+        double now[N];
 #pragma unroll
-        for (int u = 0; u < B; ++u) {
-            L0 += k[u] == 0 ? v[u] : 0.0;
-            L1 += k[u] == 1 ? v[u] : 0.0;
-        }
+        for (int u = 0; u < N; ++u) now[u] = k[u] == cls ? v[u] : 0.0;
+        if (base + 32 * N < c.M) load(base + 32 * N);
+        sum.add<N>(now, lane);
     }
-    for (; base < c.M; ++base) {
-        const double v = c.ord_val[base];
-        const unsigned char k = c.ord_cls[base];
-        L0 += k == 0 ? v : 0.0;
-        L1 += k == 1 ? v : 0.0;
-    }
-    c.out[0] = L0;
-    c.out[1] = L1;
+    if (lane == 0) c.out[cls] = sum.s;
 }
 
 // ---------------------------------------------------------------------------
@@ -876,8 +973,13 @@ ChainGeom make_chain_geom(const lat_params& p, int64_t M)
         if (q > (double)n[a]) q = (double)n[a];
         nb[a] = (long long)q;
     }
-    // at most about two cells per crossing: wider cells only add candidates
-    const long long cap = std::max<long long>(64, 2 * std::max<int64_t>(M, 1));
+    // Cells as small as the cutoff allows, as long as their tables (12 B a cell)
+    // stay small: 64 cells per crossing up to 2^22 cells (50 MB), else two per
+    // crossing.  Strings leave most cells empty, so two per crossing are cells
+    // several cutoffs wide, full of crossings out of reach (0.73 ms instead of
+    // a fraction of that for the link count of 6.7x10^4 crossings at 256^3).
+    const long long m1 = std::max<int64_t>(M, 1);
+    const long long cap = std::max<long long>(64, std::max<long long>(2 * m1, std::min<long long>(64 * m1, 1 << 22)));
     while (nb[0] * nb[1] * nb[2] > cap) {
         int a = 0;
         if (nb[1] > nb[a]) a = 1;
@@ -887,7 +989,13 @@ ChainGeom make_chain_geom(const lat_params& p, int64_t M)
     for (int a = 0; a < 3; ++a) {
         g.nb[a] = (int)nb[a];
         g.w[a] = g.L[a] / (double)nb[a];
+        g.Lf[a] = (float)g.L[a];
     }
+    // each coordinate difference is off by up to 2^-22 of the box (two
+    // truncations) and the box's own rounding, in three axes
+    const double reach = g.root_cutoff + 4 * 0x1p-22 * (g.L[0] + g.L[1] + g.L[2]);
+    const double near2 = reach * reach * (1 + 1e-5);
+    g.near2 = near2 < 1e38 ? (float)(near2 * (1 + 1e-6)) : INFINITY;
     // distinct neighbour offsets per axis: -1, 0, +1 wrap onto each other below 3 cells
     int offs[3][3], no[3];
     for (int a = 0; a < 3; ++a) {
@@ -986,7 +1094,8 @@ int chain_length_run(const ChainGeom& g, const double* d_xyz, int64_t M, int spl
         CH_CK(exclusive_scan(c.bin_cnt, c.nbins, c.bin_start, 1, c.scan_tot, c.scan_sum, st, &nl));
         CH_CK(cudaMemsetAsync(c.bin_cnt, 0, cnt_bytes, st));
         bin_scatter_kernel<<<blocks, tb, 0, st>>>(c);
-        adj_count_kernel<<<blocks, tb, 0, st>>>(c);
+        const unsigned wblocks = (unsigned)((32 * M + tb - 1) / tb);  // a warp per crossing
+        adj_count_kernel<<<wblocks, tb, 0, st>>>(c);
         CH_CK(exclusive_scan(c.deg, M, c.adj_start, 1, c.scan_tot, c.scan_sum, st, &nl));
         long long E = 0;
         CH_CK(cudaMemcpyAsync(&E, c.adj_start + M, sizeof(E), cudaMemcpyDeviceToHost, st));
@@ -995,14 +1104,14 @@ int chain_length_run(const ChainGeom& g, const double* d_xyz, int64_t M, int spl
         if ((rc = grow(&buf.edges, &buf.edge_bytes, ebytes, held))) return rc;
         c.adj = (AdjEdge*)buf.edges;
         c.edge_dead = (unsigned char*)buf.edges + ((sizeof(AdjEdge) * (size_t)E + 255) & ~(size_t)255);
-        adj_fill_kernel<<<blocks, tb, 0, st>>>(c);
+        adj_fill_kernel<<<wblocks, tb, 0, st>>>(c);
         adj_link_kernel<<<blocks, tb, 0, st>>>(c);
         flatten_kernel<<<blocks, tb, 0, st>>>(c);
         const int wgrid = (int)std::min<int64_t>(152 * 8, (M + WALK_WARPS - 1) / WALK_WARPS);
         walk_kernel<<<wgrid, 32 * WALK_WARPS, 0, st>>>(c);
         CH_CK(exclusive_scan(c.chain_len, M, c.chain_off, 0, c.scan_tot, c.scan_sum, st, &nl));
         order_kernel<<<blocks, tb, 0, st>>>(c);
-        sum_kernel<<<1, 32, 0, st>>>(c);
+        sum_kernel<<<1, 64, 0, st>>>(c);
         nl += 10;
     }
     CH_CK(cudaGetLastError());
