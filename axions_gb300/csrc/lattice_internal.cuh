@@ -180,7 +180,9 @@ cudaError_t launch_ah_twopass_fast(const Geom&, const Fields<double, 5>&, double
 // x-planes per CTA of the tiled FP32 step for a new handle (tuned value of the
 // shape if known in this process, else a heuristic); tune.cu
 int default_chunk(const lat_params& p);
-// x-planes per work item of a lattice stepped in a batch (its shape only)
+// tiles of a plane of the x-marching step
+int64_t march_tiles(const Geom& g);
+// x-planes per CTA of a served lattice's final diagnostics (its shape only)
 int batch_chunk(const Geom& g);
 // number of CTAs (and diagnostic partials) of the tiled FP32 step
 int tiled_blocks(const Geom&, int chunk);

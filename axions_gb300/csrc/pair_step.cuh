@@ -232,7 +232,8 @@ __device__ __forceinline__ void pair_stage(PairSmem<NS>& sm, int b, const Fields
 
 // One tile: z-pairs (bx*64.., by*4..) of the evolved region, x-planes
 // [bz*chunk, bz*chunk + chunk).  Called by every thread of the CTA.  With DIAG
-// the CTA's energy and |G| sums are written to part[0], part[1].  PIPE: the
+// the CTA's energy and |G| sums are written to part[0], part[1]; with psub > 0
+// the sums of every psub planes to part[0..1], part[pstride..], ...  PIPE: the
 // level n-1 of the own pair is loaded one plane ahead, and the plain step's
 // x-march is unrolled by two (the carried values then change registers
 // without copies); Abelian-Higgs in its own kernel.  The Moore tile, at the
@@ -241,7 +242,7 @@ __device__ __forceinline__ void pair_stage(PairSmem<NS>& sm, int b, const Fields
 template <int NS, bool DIAG, bool PIPE = false, bool Q12 = false>
 __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const Fields<float, 2 * NS + 3>& f,
                                           const PairCoef& c, const Charges<float>& ch, const DiagOut& d, int bx,
-                                          int by, int bz, int chunk, double* part)
+                                          int by, int bz, int chunk, double* part, int psub = 0, int pstride = 0)
 {
     using LI = LinkIdx<NS>;
     constexpr int TH = 2 * NS;  // first theta component
@@ -316,6 +317,31 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
     for (int b = 0; b < ST - 1; ++b) pair_stage<NS>(sm, b, f, g, wrap_idx(ib + b, g.nx), soff, sdst);
 
     double e_acc = 0.0, g_acc = 0.0;
+    // the CTA's sums so far to `part`
+    auto store_sums = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
+            g_acc += __shfl_down_sync(0xffffffffu, g_acc, o);
+        }
+        if (tz == 0) {
+            sm.red[0][ty] = e_acc;
+            sm.red[1][ty] = g_acc;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            double a = 0, b = 0;
+            for (int w = 0; w < PT_Y; ++w) {
+                a += sm.red[0][w];
+                b += sm.red[1][w];
+            }
+            part[0] = a;
+            part[1] = b;
+        }
+        __syncthreads();  // sm.red is reused
+        part += pstride;
+        e_acc = g_acc = 0.0;
+    };
     // level n-1 of the own pair for the next plane (PIPE)
     float2 qn[2 * NS + 3];
     if constexpr (PIPE) {
@@ -636,30 +662,13 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
         tzo = tzxp;
         carried = true;
         cur = nxt;
+        if constexpr (DIAG) {
+            if (psub > 0 && ((i + 1 - ib) % psub == 0 || i + 1 == ie)) store_sums();
+        }
     }
     __pipeline_wait_prior(0);  // nothing is in flight here; kept for an empty x-range
-
     if constexpr (DIAG) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
-            g_acc += __shfl_down_sync(0xffffffffu, g_acc, o);
-        }
-        if (tz == 0) {
-            sm.red[0][ty] = e_acc;
-            sm.red[1][ty] = g_acc;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double a = 0, b = 0;
-            for (int w = 0; w < PT_Y; ++w) {
-                a += sm.red[0][w];
-                b += sm.red[1][w];
-            }
-            part[0] = a;
-            part[1] = b;
-        }
-        __syncthreads();  // sm.red is reused by the CTA's next tile
+        if (psub == 0) store_sums();
     }
 }
 

@@ -183,13 +183,15 @@ inline bool tiled_vec_ok(const Geom& g, const Fields<T, NC>& f)
 
 // One tile: columns (bx*TZ.., by*TY..) of the evolved region, x-planes
 // [bz*chunk, bz*chunk + chunk).  Called by every thread of the CTA.  With DIAG
-// the CTA's energy and |G| sums are written to part[0], part[1].  `vec`
+// the CTA's energy and |G| sums are written to part[0], part[1]; with psub > 0
+// the sums of every psub planes to part[0..1], part[pstride..], ...  `vec`
 // selects the 16-byte staging (only where tiled_vec_ok holds); both stagings
 // fill the same shared-memory positions, so the results are bitwise equal.
 template <class T, int NS, bool DIAG>
 __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, const Fields<T, 2 * NS + 3>& f,
                                            const StepCoefT<T>& c, const Charges<T>& ch, const DiagOut& d, int bx,
-                                           int by, int bz, int chunk, double* part, bool vec)
+                                           int by, int bz, int chunk, double* part, bool vec, int psub = 0,
+                                           int pstride = 0)
 {
     using TR = Trig<T>;
     using LI = LinkIdx<NS>;
@@ -244,6 +246,31 @@ __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, 
     stage(1, wrap_idx(ib + 1, g.nx));
 
     double e_acc = 0.0, g_acc = 0.0;
+    // the CTA's sums so far to `part`
+    auto store_sums = [&]() {
+#pragma unroll
+        for (int o = 16; o > 0; o >>= 1) {
+            e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
+            g_acc += __shfl_down_sync(0xffffffffu, g_acc, o);
+        }
+        if (tz == 0) {
+            sm.red[0][ty] = e_acc;
+            sm.red[1][ty] = g_acc;
+        }
+        __syncthreads();
+        if (tid == 0) {
+            double a = 0, b = 0;
+            for (int w = 0; w < TT_Y; ++w) {
+                a += sm.red[0][w];
+                b += sm.red[1][w];
+            }
+            part[0] = a;
+            part[1] = b;
+        }
+        __syncthreads();  // sm.red is reused
+        part += pstride;
+        e_acc = g_acc = 0.0;
+    };
 
     // Two barriers per plane.  The first (after the wait) makes planes i and
     // i+1 visible and ends every read of plane i-1's stage and of the link
@@ -471,30 +498,13 @@ __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, 
 #pragma unroll
         for (int cc = 0; cc < 2 * NS; ++cc) vm[cc] = v[cc];
         cur = nxt;
+        if constexpr (DIAG) {
+            if (psub > 0 && ((i + 1 - ib) % psub == 0 || i + 1 == ie)) store_sums();
+        }
     }
     __pipeline_wait_prior(0);  // nothing is in flight here; kept for an empty x-range
-
     if constexpr (DIAG) {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
-            g_acc += __shfl_down_sync(0xffffffffu, g_acc, o);
-        }
-        if (tz == 0) {
-            sm.red[0][ty] = e_acc;
-            sm.red[1][ty] = g_acc;
-        }
-        __syncthreads();
-        if (tid == 0) {
-            double a = 0, b = 0;
-            for (int w = 0; w < TT_Y; ++w) {
-                a += sm.red[0][w];
-                b += sm.red[1][w];
-            }
-            part[0] = a;
-            part[1] = b;
-        }
-        __syncthreads();  // sm.red is reused by the CTA's next tile
+        if (psub == 0) store_sums();
     }
 }
 
