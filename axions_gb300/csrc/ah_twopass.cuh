@@ -12,9 +12,9 @@
 // STRICT = true keeps the reference's rounding operation by operation (the
 // translation unit is compiled with -fmad=false); the link data are the very
 // doubles the one-pass kernel computes, so the two paths agree bit for bit.
-// STRICT = false (LAT_F64_FAST) lets the compiler fuse multiply-adds, divides
-// by dt through a corrected reciprocal, and takes sin(P_yx) = -sin(P_xy)
-// (likewise zx, zy): the same arithmetic to within an ulp per operation.
+// STRICT = false (LAT_F64_FAST) lets the compiler fuse multiply-adds and takes
+// sin(P_yx) = -sin(P_xy) (likewise zx, zy): the same arithmetic to within an
+// ulp per operation.
 #pragma once
 
 #include "site_common.cuh"
@@ -55,30 +55,48 @@ inline LinkSlotsC link_slots_c(const double* L, long long N)
     return s;
 }
 
-// a / b where b = spacing^2 or spacing: exact reciprocal multiply when every
-// spacing is a power of two (then a*(1/b) == a/b for all a), else the IEEE
-// quotient by cdiv from the host reciprocal.
+// a / b where b = spacing^2 or spacing: the multiplication by the reciprocal,
+// exact when every spacing is a power of two (then a*(1/b) == a/b for all a),
+// else the IEEE quotient by cdiv from the host reciprocal.
 template <bool RECIP>
 __device__ __forceinline__ double sdiv(double a, double b, double inv_b)
 {
-    if constexpr (RECIP) return mul_pow2(a, inv_b);
+    if constexpr (RECIP) return __dmul_rn(a, inv_b);
     else return cdiv(a, b, inv_b);
 }
 
-// a / dt.  STRICT: the IEEE quotient by cdiv (two residual corrections from
-// the host reciprocal; a zero dividend returns a * (1/b), the same +-0).
-// Fast: q = a*r corrected by one residual step (Markstein), which returns the
-// correctly rounded quotient except in rare cases where it is one ulp off.
-template <bool STRICT>
-__device__ __forceinline__ double tdiv(double a, double b, double inv_b)
+// x != 0 by integer instructions (a comparison of doubles takes the FP64 pipe)
+__device__ __forceinline__ bool nonzero(double x) { return (__double_as_longlong(x) << 1) != 0; }
+
+// t - a / b.  With power-of-two spacings the quotient is exact, so one fused
+// operation rounds as the subtraction alone does.
+template <bool RECIP>
+__device__ __forceinline__ double sub_sdiv(double t, double a, double b, double inv_b)
 {
-    if constexpr (STRICT) return cdiv(a, b, inv_b);
-    else {
-        const double q = a * inv_b;
-        const double r = fma(-q, b, a);
-        return fma(r, inv_b, q);
+    if constexpr (RECIP) return __fma_rn(-a, inv_b, t);
+    else return t - cdiv(a, b, inv_b);
+}
+
+// x/dx2 + y/dy2 + z/dz2 - r, the quotients and sums rounded one by one (in that
+// order); with power-of-two spacings the scalings are exact and fold into the
+// additions, or, for equal spacings, into the last subtraction.
+template <bool RECIP>
+__device__ __forceinline__ double lap_minus(double x, double y, double z, double r, const StepCoef& c)
+{
+    if constexpr (RECIP) {
+        if (nonzero(c.iso)) return __fma_rn(__dadd_rn(__dadd_rn(x, y), z), c.inv_dx2, -r);
+        return __dadd_rn(__fma_rn(z, c.inv_dz2, __fma_rn(x, c.inv_dx2, __dmul_rn(y, c.inv_dy2))), -r);
+    } else {
+        return __dadd_rn(__dadd_rn(__dadd_rn(cdiv(x, c.dx2, c.inv_dx2), cdiv(y, c.dy2, c.inv_dy2)),
+                                   cdiv(z, c.dz2, c.inv_dz2)), -r);
     }
 }
+
+// 2*x - y: the doubling is exact, so the fused form rounds once as the
+// subtraction does
+__device__ __forceinline__ double twice_minus(double x, double y) { return __fma_rn(2.0, x, -y); }
+// t - 2*x
+__device__ __forceinline__ double minus_twice(double t, double x) { return __fma_rn(-2.0, x, t); }
 
 template <bool STRICT, bool DIAG>
 __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Flat r, const double* __restrict__ TX,
@@ -130,6 +148,179 @@ __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Fla
     }
 }
 
+// What the update of one site reads: the scalar and its neighbours, the past
+// level, the link phases, and the link data of the site and of its backward
+// neighbours (sP*_m: the plaquette sine there; sPyx, sPzx, sPzy in STRICT mode
+// sines of their own, else the negated sPxy, sPxz, sPyz).
+struct AhSite {
+    double p0, p1, p0xp, p1xp, p0xm, p1xm, p0yp, p1yp, p0ym, p1ym, p0zp, p1zp, p0zm, p1zm;
+    double q0, q1, tx, ty, tz, qx, qy, qz, txm, tym, tzm;
+    double cx, sx, cy, sy, cz, sz, cxm, sxm, cym, sym, czm, szm;
+    double sPxy, sPxz, sPyz, sPxy_m, sPxz_m, sPyz_m, sPyx, sPzx, sPzy, sPyx_m, sPzx_m, sPzy_m;
+    double cPxy, cPxz, cPyz, divPast;   // diagnostic steps
+};
+
+// The update of one site (mpi_evolution.cpp:412-501) and its diagnostics: new
+// values to `next` (phi, then theta), div(theta) to divNow.
+template <bool STRICT, bool DIAG, bool RECIP>
+__device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, const DiagOut& d, double (&next)[5],
+                                        double& divNow, double& e_site, double& g_site)
+{
+    const double p0 = v.p0, p1 = v.p1, p0xp = v.p0xp, p1xp = v.p1xp, p0xm = v.p0xm, p1xm = v.p1xm;
+    const double p0yp = v.p0yp, p1yp = v.p1yp, p0ym = v.p0ym, p1ym = v.p1ym;
+    const double p0zp = v.p0zp, p1zp = v.p1zp, p0zm = v.p0zm, p1zm = v.p1zm;
+    const double q0 = v.q0, q1 = v.q1, tx = v.tx, ty = v.ty, tz = v.tz, qx = v.qx, qy = v.qy, qz = v.qz;
+    const double cx = v.cx, sx = v.sx, cy = v.cy, sy = v.sy, cz = v.cz, sz = v.sz;
+    const double cxm = v.cxm, sxm_ = v.sxm, cym = v.cym, sym = v.sym, czm = v.czm, szm_ = v.szm;
+    const double sPxy = v.sPxy, sPxz = v.sPxz, sPyz = v.sPyz, sPxy_m = v.sPxy_m, sPxz_m = v.sPxz_m, sPyz_m = v.sPyz_m;
+    const double sPyx = v.sPyx, sPzx = v.sPzx, sPzy = v.sPzy;
+    const double sPyx_m = v.sPyx_m, sPzx_m = v.sPzx_m, sPzy_m = v.sPzy_m;
+    const double phiMagSqr = p0 * p0 + p1 * p1;
+    const double pot = c.halfLambda * (phiMagSqr - c.etaSq);
+
+    double tt0 = 0, tt1 = 0, curx, cury, curz;
+    if constexpr (STRICT) {
+        // covariant Laplacian (mpi_evolution.cpp:418-428), c = +1 then c = -1
+        tt0 = lap_minus<RECIP>(minus_twice(cx * p0xp + sx * p1xp, p0) + cxm * p0xm - sxm_ * p1xm,
+                               minus_twice(cy * p0yp + sy * p1yp, p0) + cym * p0ym - sym * p1ym,
+                               minus_twice(cz * p0zp + sz * p1zp, p0) + czm * p0zm - szm_ * p1zm, pot * p0, c);
+        tt1 = lap_minus<RECIP>(minus_twice(cx * p1xp - sx * p0xp, p1) + cxm * p1xm + sxm_ * p0xm,
+                               minus_twice(cy * p1yp - sy * p0yp, p1) + cym * p1ym + sym * p0ym,
+                               minus_twice(cz * p1zp - sz * p0zp, p1) + czm * p1zm + szm_ * p0zm, pot * p1, c);
+        if (nonzero(c.fric)) {
+            tt0 = tt0 - c.fric * cdiv(p0 - q0, c.dt, c.inv_dt);
+            tt1 = tt1 - c.fric * cdiv(p1 - q1, c.dt, c.inv_dt);
+        }
+        // gauge current (mpi_evolution.cpp:459-466)
+        curx = cx * (p1 * p0xp - p0 * p1xp) + sx * (p0 * p0xp + p1 * p1xp);
+        cury = cy * (p1 * p0yp - p0 * p1yp) + sy * (p0 * p0yp + p1 * p1yp);
+        curz = cz * (p1 * p0zp - p0 * p1zp) + sz * (p0 * p0zp + p1 * p1zp);
+    } else {
+        // The same quantities with fewer FP64 instructions.  The forward
+        // link-transported neighbour U_mu phi(x+mu), A = c phi0' + s phi1',
+        // B = c phi1' - s phi0', enters both the Laplacian and the current:
+        // j_mu = c (phi1 phi0' - phi0 phi1') + s (phi0 phi0' + phi1 phi1')
+        //      = phi1 A - phi0 B.
+        const double Ax = fma(sx, p1xp, cx * p0xp), Bx = fma(-sx, p0xp, cx * p1xp);
+        const double Ay = fma(sy, p1yp, cy * p0yp), By = fma(-sy, p0yp, cy * p1yp);
+        const double Az = fma(sz, p1zp, cz * p0zp), Bz = fma(-sz, p0zp, cz * p1zp);
+        const double x0 = fma(-sxm_, p1xm, fma(cxm, p0xm, Ax)), x1 = fma(sxm_, p0xm, fma(cxm, p1xm, Bx));
+        const double y0 = fma(-sym, p1ym, fma(cym, p0ym, Ay)), y1 = fma(sym, p0ym, fma(cym, p1ym, By));
+        const double z0 = fma(-szm_, p1zm, fma(czm, p0zm, Az)), z1 = fma(szm_, p0zm, fma(czm, p1zm, Bz));
+        curx = fma(p1, Ax, -p0 * Bx);
+        cury = fma(p1, Ay, -p0 * By);
+        curz = fma(p1, Az, -p0 * Bz);
+        if (nonzero(c.iso)) {
+            // Equal spacings: every term of an update carries its factor dt^2
+            // times a constant from the host and is added to the difference
+            // of the two levels, which is small and exact, before that is
+            // added to the level: 71 FP64 instructions a site (74 with the
+            // acceleration formed first) and one rounding of the level's size
+            // instead of two.
+            const double ps = c.kPot * (phiMagSqr - c.etaSq);
+            const double u0 = fma(-ps, p0, fma(-6.0, p0, x0 + y0 + z0)), u1 = fma(-ps, p1, fma(-6.0, p1, x1 + y1 + z1));
+            double d0 = p0 - q0, d1 = p1 - q1, dx = tx - qx, dy = ty - qy, dz = tz - qz;
+            if (nonzero(c.fric)) {
+                d0 = fma(-c.kFric, d0, d0);
+                d1 = fma(-c.kFric, d1, d1);
+            }
+            if (nonzero(c.damp)) {
+                dx = fma(-c.kDamp, dx, dx);
+                dy = fma(-c.kDamp, dy, dy);
+                dz = fma(-c.kDamp, dz, dz);
+            }
+            next[0] = p0 + fma(c.kLap, u0, d0);
+            next[1] = p1 + fma(c.kLap, u1, d1);
+            // current and lattice curl (mpi_evolution.cpp:459-487)
+            next[2] = tx + fma(c.kCur, curx, fma(-c.kLap, (sPxy - sPxy_m) + (sPxz - sPxz_m), dx));
+            next[3] = ty + fma(c.kCur, cury, fma(-c.kLap, (sPyx - sPyx_m) + (sPyz - sPyz_m), dy));
+            next[4] = tz + fma(c.kCur, curz, fma(-c.kLap, (sPzx - sPzx_m) + (sPzy - sPzy_m), dz));
+        } else {
+            tt0 = lap_minus<RECIP>(minus_twice(x0, p0), minus_twice(y0, p0), minus_twice(z0, p0), pot * p0, c);
+            tt1 = lap_minus<RECIP>(minus_twice(x1, p1), minus_twice(y1, p1), minus_twice(z1, p1), pot * p1, c);
+        }
+    }
+
+    if (STRICT || !nonzero(c.iso)) {
+        if constexpr (!STRICT) {
+            if (nonzero(c.fric)) {
+                tt0 = fma(-c.fric_dt, p0 - q0, tt0);
+                tt1 = fma(-c.fric_dt, p1 - q1, tt1);
+            }
+        }
+
+        // lattice curl (mpi_evolution.cpp:471-487)
+        double ttx = sub_sdiv<RECIP>(c.m2gg * curx, sPxy - sPxy_m, c.dy2, c.inv_dy2);
+        double tty = sub_sdiv<RECIP>(c.m2gg * cury, sPyx - sPyx_m, c.dx2, c.inv_dx2);
+        double ttz = sub_sdiv<RECIP>(c.m2gg * curz, sPzx - sPzx_m, c.dx2, c.inv_dx2);
+        ttx = sub_sdiv<RECIP>(ttx, sPxz - sPxz_m, c.dz2, c.inv_dz2);
+        tty = sub_sdiv<RECIP>(tty, sPyz - sPyz_m, c.dz2, c.inv_dz2);
+        ttz = sub_sdiv<RECIP>(ttz, sPzy - sPzy_m, c.dy2, c.inv_dy2);
+        if (nonzero(c.damp)) {
+            ttx = ttx - c.damp * cdiv(tx - qx, c.dt, c.inv_dt);
+            tty = tty - c.damp * cdiv(ty - qy, c.dt, c.inv_dt);
+            ttz = ttz - c.damp * cdiv(tz - qz, c.dt, c.inv_dt);
+        }
+        // mpi_evolution.cpp:432,499-501
+        next[0] = twice_minus(p0, q0) + c.dt2 * tt0;
+        next[1] = twice_minus(p1, q1) + c.dt2 * tt1;
+        next[2] = twice_minus(tx, qx) + c.dt2 * ttx;
+        next[3] = twice_minus(ty, qy) + c.dt2 * tty;
+        next[4] = twice_minus(tz, qz) + c.dt2 * ttz;
+    }
+
+    divNow = 0;
+    if (DIAG || d.store_div) {
+        const double txm = v.txm, tym = v.tym, tzm = v.tzm;
+        divNow = sdiv<RECIP>(tx - txm, c.dx2, c.inv_dx2) + sdiv<RECIP>(ty - tym, c.dy2, c.inv_dy2)
+               + sdiv<RECIP>(tz - tzm, c.dz2, c.inv_dz2);
+    }
+
+    if constexpr (DIAG) {
+        // energy density and Gauss deviation of the now level
+        // (evolution.cpp:322-334,377-427; mpi_evolution.cpp:509-532).  Each
+        // divisor other than dt occurs once per site, so cdiv's host
+        // reciprocal replaces the division's own (the same doubles).
+        const double cPxy = v.cPxy, cPxz = v.cPxz, cPyz = v.cPyz;
+        const double pt0 = cdiv(p0 - q0, c.dt, c.inv_dt);
+        const double pt1 = cdiv(p1 - q1, c.dt, c.inv_dt);
+        const double px0 = sdiv<RECIP>(p0 - cxm * p0xm + sxm_ * p1xm, c.dx, c.inv_dx);
+        const double px1 = sdiv<RECIP>(p1 - cxm * p1xm - sxm_ * p0xm, c.dx, c.inv_dx);
+        const double py0 = sdiv<RECIP>(p0 - cym * p0ym + sym * p1ym, c.dy, c.inv_dy);
+        const double py1 = sdiv<RECIP>(p1 - cym * p1ym - sym * p0ym, c.dy, c.inv_dy);
+        const double pz0 = sdiv<RECIP>(p0 - czm * p0zm + szm_ * p1zm, c.dz, c.inv_dz);
+        const double pz1 = sdiv<RECIP>(p1 - czm * p1zm - szm_ * p0zm, c.dz, c.inv_dz);
+        double tdc = 0, fc = 0, gauss = 0;
+        if (d.energy_form == LAT_ENERGY_MPI) {
+            const double a0 = cdiv(tx - qx, c.dt, c.inv_dt), a1 = cdiv(ty - qy, c.dt, c.inv_dt),
+                         a2 = cdiv(tz - qz, c.dt, c.inv_dt);
+            tdc = 0.5 * (a0 * a0 + a1 * a1 + a2 * a2);
+            fc = cdiv(1 - cPxy, c.gxy2, c.inv_gxy2) + cdiv(1 - cPxz, c.gxz2, c.inv_gxz2)
+               + cdiv(1 - cPyz, c.gyz2, c.inv_gyz2);
+        }
+        if (nonzero(c.g)) {
+            const double divPast = v.divPast;
+            const double divThetat = cdiv(divNow - divPast, c.dt, c.inv_dt);
+            gauss = cdiv(divThetat, c.g, c.inv_g) - c.twog * (p1 * pt0 - p0 * pt1);
+            if (d.energy_form != LAT_ENERGY_MPI) {
+                const double a0 = cdiv(tx - qx, c.gdtdx, c.inv_gdtdx), a1 = cdiv(ty - qy, c.gdtdy, c.inv_gdtdy),
+                             a2 = cdiv(tz - qz, c.gdtdz, c.inv_gdtdz);
+                tdc = 0.5 * (a0 * a0 + a1 * a1 + a2 * a2);
+                const double Fxy = cdiv(1 - cPxy, c.gxy2, c.inv_gxy2);
+                const double Fxz = cdiv(1 - cPxz, c.gxz2, c.inv_gxz2);
+                const double Fyz = cdiv(1 - cPyz, c.gyz2, c.inv_gyz2);
+                fc = Fxy + Fxz + Fyz;
+            }
+        }
+        const double pm = phiMagSqr - c.etaSq;
+        const double ed = pt0 * pt0 + pt1 * pt1 + px0 * px0 + px1 * px1 + py0 * py0 + py1 * py1 + pz0 * pz0
+                        + pz1 * pz1 + tdc + fc + c.quarterLambda * (pm * pm);
+        if (d.energy_form == LAT_ENERGY_MPI) e_site = ed * c.dx * c.dy * c.dz;
+        else e_site = c.dV * ed;
+        g_site = __longlong_as_double(__double_as_longlong(gauss) & 0x7fffffffffffffffll);
+    }
+}
+
 template <bool STRICT, bool DIAG, bool RECIP>
 __global__ void __launch_bounds__(BLOCK, 2) ah_update_kernel(const Geom g, const Flat r, const Fields<double, 5> f,
                                                           const LinkSlotsC L, const StepCoef c,
@@ -141,180 +332,43 @@ __global__ void __launch_bounds__(BLOCK, 2) ah_update_kernel(const Geom g, const
     if (q < r.n) {
         const Nbr n = flat_nbr(g, r, q);
         const int s = n.s;
-        const int sxm = s + n.xm, sym_ = s + n.ym, szm = s + n.zm;
+        const int sxm = s + n.xm, sym = s + n.ym, szm = s + n.zm;
         const double* __restrict__ P0 = f.now[0];
         const double* __restrict__ P1 = f.now[1];
-
-        const double p0 = P0[s], p1 = P1[s];
-        const double p0xp = P0[s + n.xp], p1xp = P1[s + n.xp], p0xm = P0[sxm], p1xm = P1[sxm];
-        const double p0yp = P0[s + n.yp], p1yp = P1[s + n.yp], p0ym = P0[sym_], p1ym = P1[sym_];
-        const double p0zp = P0[s + n.zp], p1zp = P1[s + n.zp], p0zm = P0[szm], p1zm = P1[szm];
-        const double q0 = f.past[0][s], q1 = f.past[1][s];
-        const double tx = f.now[2][s], ty = f.now[3][s], tz = f.now[4][s];
-        const double qx = f.past[2][s], qy = f.past[3][s], qz = f.past[4][s];
-
-        const double cx = L.p[L_CX][s], sx = L.p[L_SX][s];
-        const double cy = L.p[L_CY][s], sy = L.p[L_SY][s];
-        const double cz = L.p[L_CZ][s], sz = L.p[L_SZ][s];
-        const double cxm = L.p[L_CX][sxm], sxm_ = L.p[L_SX][sxm];
-        const double cym = L.p[L_CY][sym_], sym = L.p[L_SY][sym_];
-        const double czm = L.p[L_CZ][szm], szm_ = L.p[L_SZ][szm];
-        const double sPxy = L.p[L_PXY][s], sPxz = L.p[L_PXZ][s], sPyz = L.p[L_PYZ][s];
-        const double sPxy_m = L.p[L_PXY][sym_], sPxz_m = L.p[L_PXZ][szm], sPyz_m = L.p[L_PYZ][szm];
-        double sPyx, sPzx, sPzy, sPyx_m, sPzx_m, sPzy_m;
+        AhSite v;
+        v.p0 = P0[s], v.p1 = P1[s];
+        v.p0xp = P0[s + n.xp], v.p1xp = P1[s + n.xp], v.p0xm = P0[sxm], v.p1xm = P1[sxm];
+        v.p0yp = P0[s + n.yp], v.p1yp = P1[s + n.yp], v.p0ym = P0[sym], v.p1ym = P1[sym];
+        v.p0zp = P0[s + n.zp], v.p1zp = P1[s + n.zp], v.p0zm = P0[szm], v.p1zm = P1[szm];
+        v.q0 = f.past[0][s], v.q1 = f.past[1][s];
+        v.tx = f.now[2][s], v.ty = f.now[3][s], v.tz = f.now[4][s];
+        v.qx = f.past[2][s], v.qy = f.past[3][s], v.qz = f.past[4][s];
+        v.cx = L.p[L_CX][s], v.sx = L.p[L_SX][s];
+        v.cy = L.p[L_CY][s], v.sy = L.p[L_SY][s];
+        v.cz = L.p[L_CZ][s], v.sz = L.p[L_SZ][s];
+        v.cxm = L.p[L_CX][sxm], v.sxm = L.p[L_SX][sxm];
+        v.cym = L.p[L_CY][sym], v.sym = L.p[L_SY][sym];
+        v.czm = L.p[L_CZ][szm], v.szm = L.p[L_SZ][szm];
+        v.sPxy = L.p[L_PXY][s], v.sPxz = L.p[L_PXZ][s], v.sPyz = L.p[L_PYZ][s];
+        v.sPxy_m = L.p[L_PXY][sym], v.sPxz_m = L.p[L_PXZ][szm], v.sPyz_m = L.p[L_PYZ][szm];
         if constexpr (STRICT) {
-            sPyx = L.p[L_PYX][s];
-            sPzx = L.p[L_PZX][s];
-            sPzy = L.p[L_PZY][s];
-            sPyx_m = L.p[L_PYX][sxm];
-            sPzx_m = L.p[L_PZX][sxm];
-            sPzy_m = L.p[L_PZY][sym_];
+            v.sPyx = L.p[L_PYX][s], v.sPzx = L.p[L_PZX][s], v.sPzy = L.p[L_PZY][s];
+            v.sPyx_m = L.p[L_PYX][sxm], v.sPzx_m = L.p[L_PZX][sxm], v.sPzy_m = L.p[L_PZY][sym];
         } else {
-            sPyx = -sPxy;
-            sPzx = -sPxz;
-            sPzy = -sPyz;
-            sPyx_m = -L.p[L_PXY][sxm];
-            sPzx_m = -L.p[L_PXZ][sxm];
-            sPzy_m = -L.p[L_PYZ][sym_];
+            v.sPyx = -v.sPxy, v.sPzx = -v.sPxz, v.sPzy = -v.sPyz;
+            v.sPyx_m = -L.p[L_PXY][sxm], v.sPzx_m = -L.p[L_PXZ][sxm], v.sPzy_m = -L.p[L_PYZ][sym];
         }
-
-        const double twop0 = mul_pow2(p0, 2.0), twop1 = mul_pow2(p1, 2.0);  // 2 * p0, 2 * p1
-        const double phiMagSqr = p0 * p0 + p1 * p1;
-        const double pot = c.halfLambda * (phiMagSqr - c.etaSq);
-
-        double tt0, tt1, curx, cury, curz;
-        if constexpr (STRICT) {
-            // covariant Laplacian (mpi_evolution.cpp:418-428), c = +1 then c = -1
-            const double lap0 = sdiv<RECIP>(cx * p0xp + sx * p1xp - twop0 + cxm * p0xm - sxm_ * p1xm, c.dx2, c.inv_dx2)
-                              + sdiv<RECIP>(cy * p0yp + sy * p1yp - twop0 + cym * p0ym - sym * p1ym, c.dy2, c.inv_dy2)
-                              + sdiv<RECIP>(cz * p0zp + sz * p1zp - twop0 + czm * p0zm - szm_ * p1zm, c.dz2, c.inv_dz2);
-            const double lap1 = sdiv<RECIP>(cx * p1xp - sx * p0xp - twop1 + cxm * p1xm + sxm_ * p0xm, c.dx2, c.inv_dx2)
-                              + sdiv<RECIP>(cy * p1yp - sy * p0yp - twop1 + cym * p1ym + sym * p0ym, c.dy2, c.inv_dy2)
-                              + sdiv<RECIP>(cz * p1zp - sz * p0zp - twop1 + czm * p1zm + szm_ * p0zm, c.dz2, c.inv_dz2);
-            tt0 = lap0 - pot * p0;
-            tt1 = lap1 - pot * p1;
-            if (c.fric != 0) {
-                tt0 = tt0 - c.fric * tdiv<STRICT>(p0 - q0, c.dt, c.inv_dt);
-                tt1 = tt1 - c.fric * tdiv<STRICT>(p1 - q1, c.dt, c.inv_dt);
-            }
-            // gauge current (mpi_evolution.cpp:459-466)
-            curx = cx * (p1 * p0xp - p0 * p1xp) + sx * (p0 * p0xp + p1 * p1xp);
-            cury = cy * (p1 * p0yp - p0 * p1yp) + sy * (p0 * p0yp + p1 * p1yp);
-            curz = cz * (p1 * p0zp - p0 * p1zp) + sz * (p0 * p0zp + p1 * p1zp);
-        } else {
-            // The same quantities with fewer FP64 instructions.  The forward
-            // link-transported neighbour U_mu phi(x+mu), A = c phi0' + s phi1',
-            // B = c phi1' - s phi0', enters both the Laplacian and the current:
-            // j_mu = c (phi1 phi0' - phi0 phi1') + s (phi0 phi0' + phi1 phi1')
-            //      = phi1 A - phi0 B.
-            // With equal spacings the three directions are summed before one
-            // scaling; friction uses fric/dt from the host.
-            const double Ax = fma(sx, p1xp, cx * p0xp), Bx = fma(-sx, p0xp, cx * p1xp);
-            const double Ay = fma(sy, p1yp, cy * p0yp), By = fma(-sy, p0yp, cy * p1yp);
-            const double Az = fma(sz, p1zp, cz * p0zp), Bz = fma(-sz, p0zp, cz * p1zp);
-            double lap0, lap1;
-            if (c.iso != 0) {
-                const double s0 = fma(-sxm_, p1xm, fma(cxm, p0xm, Ax)) + fma(-sym, p1ym, fma(cym, p0ym, Ay))
-                                + fma(-szm_, p1zm, fma(czm, p0zm, Az));
-                const double s1 = fma(sxm_, p0xm, fma(cxm, p1xm, Bx)) + fma(sym, p0ym, fma(cym, p1ym, By))
-                                + fma(szm_, p0zm, fma(czm, p1zm, Bz));
-                lap0 = sdiv<RECIP>(fma(-6.0, p0, s0), c.dx2, c.inv_dx2);
-                lap1 = sdiv<RECIP>(fma(-6.0, p1, s1), c.dx2, c.inv_dx2);
-            } else {
-                lap0 = sdiv<RECIP>(fma(-sxm_, p1xm, fma(cxm, p0xm, Ax)) - twop0, c.dx2, c.inv_dx2)
-                     + sdiv<RECIP>(fma(-sym, p1ym, fma(cym, p0ym, Ay)) - twop0, c.dy2, c.inv_dy2)
-                     + sdiv<RECIP>(fma(-szm_, p1zm, fma(czm, p0zm, Az)) - twop0, c.dz2, c.inv_dz2);
-                lap1 = sdiv<RECIP>(fma(sxm_, p0xm, fma(cxm, p1xm, Bx)) - twop1, c.dx2, c.inv_dx2)
-                     + sdiv<RECIP>(fma(sym, p0ym, fma(cym, p1ym, By)) - twop1, c.dy2, c.inv_dy2)
-                     + sdiv<RECIP>(fma(szm_, p0zm, fma(czm, p1zm, Bz)) - twop1, c.dz2, c.inv_dz2);
-            }
-            tt0 = fma(-pot, p0, lap0);
-            tt1 = fma(-pot, p1, lap1);
-            if (c.fric != 0) {
-                tt0 = fma(-c.fric_dt, p0 - q0, tt0);
-                tt1 = fma(-c.fric_dt, p1 - q1, tt1);
-            }
-            curx = fma(p1, Ax, -p0 * Bx);
-            cury = fma(p1, Ay, -p0 * By);
-            curz = fma(p1, Az, -p0 * Bz);
-        }
-
-        // lattice curl (mpi_evolution.cpp:471-487)
-        const double Fxy_y = sdiv<RECIP>(sPxy - sPxy_m, c.dy2, c.inv_dy2);
-        const double Fxz_z = sdiv<RECIP>(sPxz - sPxz_m, c.dz2, c.inv_dz2);
-        const double Fyx_x = sdiv<RECIP>(sPyx - sPyx_m, c.dx2, c.inv_dx2);
-        const double Fyz_z = sdiv<RECIP>(sPyz - sPyz_m, c.dz2, c.inv_dz2);
-        const double Fzx_x = sdiv<RECIP>(sPzx - sPzx_m, c.dx2, c.inv_dx2);
-        const double Fzy_y = sdiv<RECIP>(sPzy - sPzy_m, c.dy2, c.inv_dy2);
-
-        double ttx = c.m2gg * curx - Fxy_y - Fxz_z;
-        double tty = c.m2gg * cury - Fyx_x - Fyz_z;
-        double ttz = c.m2gg * curz - Fzx_x - Fzy_y;
-        if (c.damp != 0) {
-            ttx = ttx - c.damp * tdiv<STRICT>(tx - qx, c.dt, c.inv_dt);
-            tty = tty - c.damp * tdiv<STRICT>(ty - qy, c.dt, c.inv_dt);
-            ttz = ttz - c.damp * tdiv<STRICT>(tz - qz, c.dt, c.inv_dt);
-        }
-
-        double divNow = 0;
-        if (DIAG || d.store_div) {
-            const double txm = f.now[2][sxm], tym = f.now[3][sym_], tzm = f.now[4][szm];
-            divNow = sdiv<RECIP>(tx - txm, c.dx2, c.inv_dx2) + sdiv<RECIP>(ty - tym, c.dy2, c.inv_dy2)
-                   + sdiv<RECIP>(tz - tzm, c.dz2, c.inv_dz2);
-        }
-
+        if (DIAG || d.store_div) v.txm = f.now[2][sxm], v.tym = f.now[3][sym], v.tzm = f.now[4][szm];
         if constexpr (DIAG) {
-            // energy density and Gauss deviation of the now level
-            // (evolution.cpp:322-334,377-427; mpi_evolution.cpp:509-532).  Each
-            // divisor other than dt occurs once per site, so cdiv's host
-            // reciprocal replaces the division's own (the same doubles).
-            const double cPxy = L.p[L_CPXY][s], cPxz = L.p[L_CPXZ][s], cPyz = L.p[L_CPYZ][s];
-            const double pt0 = tdiv<STRICT>(p0 - q0, c.dt, c.inv_dt);
-            const double pt1 = tdiv<STRICT>(p1 - q1, c.dt, c.inv_dt);
-            const double px0 = sdiv<RECIP>(p0 - cxm * p0xm + sxm_ * p1xm, c.dx, c.inv_dx);
-            const double px1 = sdiv<RECIP>(p1 - cxm * p1xm - sxm_ * p0xm, c.dx, c.inv_dx);
-            const double py0 = sdiv<RECIP>(p0 - cym * p0ym + sym * p1ym, c.dy, c.inv_dy);
-            const double py1 = sdiv<RECIP>(p1 - cym * p1ym - sym * p0ym, c.dy, c.inv_dy);
-            const double pz0 = sdiv<RECIP>(p0 - czm * p0zm + szm_ * p1zm, c.dz, c.inv_dz);
-            const double pz1 = sdiv<RECIP>(p1 - czm * p1zm - szm_ * p0zm, c.dz, c.inv_dz);
-            double tdc = 0, fc = 0, gauss = 0;
-            if (d.energy_form == LAT_ENERGY_MPI) {
-                const double a0 = tdiv<true>(tx - qx, c.dt, c.inv_dt), a1 = tdiv<true>(ty - qy, c.dt, c.inv_dt),
-                             a2 = tdiv<true>(tz - qz, c.dt, c.inv_dt);
-                tdc = 0.5 * (a0 * a0 + a1 * a1 + a2 * a2);
-                fc = cdiv(1 - cPxy, c.gxy2, c.inv_gxy2) + cdiv(1 - cPxz, c.gxz2, c.inv_gxz2)
-                   + cdiv(1 - cPyz, c.gyz2, c.inv_gyz2);
-            }
-            if (c.g != 0) {
-                const double divPast = reinterpret_cast<const double*>(d.divbuf)[s];
-                const double divThetat = tdiv<true>(divNow - divPast, c.dt, c.inv_dt);
-                gauss = cdiv(divThetat, c.g, c.inv_g) - c.twog * (p1 * pt0 - p0 * pt1);
-                if (d.energy_form != LAT_ENERGY_MPI) {
-                    const double a0 = cdiv(tx - qx, c.gdtdx, c.inv_gdtdx), a1 = cdiv(ty - qy, c.gdtdy, c.inv_gdtdy),
-                                 a2 = cdiv(tz - qz, c.gdtdz, c.inv_gdtdz);
-                    tdc = 0.5 * (a0 * a0 + a1 * a1 + a2 * a2);
-                    const double Fxy = cdiv(1 - cPxy, c.gxy2, c.inv_gxy2);
-                    const double Fxz = cdiv(1 - cPxz, c.gxz2, c.inv_gxz2);
-                    const double Fyz = cdiv(1 - cPyz, c.gyz2, c.inv_gyz2);
-                    fc = Fxy + Fxz + Fyz;
-                }
-            }
-            const double pm = phiMagSqr - c.etaSq;
-            const double ed = pt0 * pt0 + pt1 * pt1 + px0 * px0 + px1 * px1 + py0 * py0 + py1 * py1 + pz0 * pz0
-                            + pz1 * pz1 + tdc + fc + c.quarterLambda * (pm * pm);
-            if (d.energy_form == LAT_ENERGY_MPI) e_site = ed * c.dx * c.dy * c.dz;
-            else e_site = c.dV * ed;
-            g_site = fabs(gauss);
+            v.cPxy = L.p[L_CPXY][s], v.cPxz = L.p[L_CPXZ][s], v.cPyz = L.p[L_CPYZ][s];
+            if (nonzero(c.g)) v.divPast = reinterpret_cast<const double*>(d.divbuf)[s];
         }
-
+        double next[5], divNow;
+        ah_site<STRICT, DIAG, RECIP>(v, c, d, next, divNow, e_site, g_site);
         if (d.store_div) reinterpret_cast<double*>(d.divbuf)[s] = divNow;
-
-        if (d.write) {  // in-place update of the past slot (mpi_evolution.cpp:432,499-501)
-            f.past[0][s] = twop0 - q0 + c.dt2 * tt0;
-            f.past[1][s] = twop1 - q1 + c.dt2 * tt1;
-            f.past[2][s] = mul_pow2(tx, 2.0) - qx + c.dt2 * ttx;
-            f.past[3][s] = mul_pow2(ty, 2.0) - qy + c.dt2 * tty;
-            f.past[4][s] = mul_pow2(tz, 2.0) - qz + c.dt2 * ttz;
+        if (d.write) {  // in-place update of the past slot
+#pragma unroll
+            for (int m = 0; m < 5; ++m) f.past[m][s] = next[m];
         }
     }
     if constexpr (DIAG) flat_sum2_store(e_site, g_site, d.partials);

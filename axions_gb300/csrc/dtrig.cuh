@@ -9,8 +9,7 @@
 //
 //   x = k*pi/2 + r, |r| <= pi/4(1 + 2^-6): k from a float copy of x (FP32),
 //       r by a two-part Cody-Waite step (Cody & Waite 1980): k*P1 is exact
-//       (16 + 36 bits), the second FMA rounds once.  Where r cancels below
-//       2^-20 a third part is taken off as well;
+//       (16 + 36 bits), the second FMA rounds once;
 //   r = m*2^e with m in [1/2, 1) as a 64-bit fraction, z = r^2 likewise;
 //   sin r = r*S(z), cos r = C(z): the Taylor polynomials of degree 9 in z
 //       (truncation below 2^-66) by Horner's rule, the first steps on 32-bit
@@ -30,8 +29,8 @@
 // results do not depend on the translation unit's -fmad setting: the strict
 // and fast FP64 kernels and the one-pass kernel get the very same doubles.
 //
-// |x| >= 2^16 (where k no longer fits the exact product) and NaN/Inf go to
-// CUDA's sin/cos; |x| < 2^-27 returns sin x = x, cos x = 1.
+// |x| >= 2^16 (where k no longer fits the exact product), NaN/Inf and arguments
+// within 2^-20 of a multiple of pi/2 other than 0 go to CUDA's sin/cos; |x| < 2^-27 returns sin x = x, cos x = 1.
 #pragma once
 
 #include <cuda_runtime.h>
@@ -47,10 +46,9 @@ namespace dtrig {
 constexpr int kHiLarge = 0x40f00000;  // high word of 2^16
 constexpr int kHiTiny = 0x3e400000;   // high word of 2^-27
 
-// pi/2 = P1 + P2 + P3: 36 bits, then the nearest doubles of the rests
+// pi/2 = P1 + P2 within 2^-93: 36 bits, then the nearest double of the rest
 constexpr double kP1 = 0x1.921fb54440000p+0;
 constexpr double kP2 = 0x1.68c234c4c6629p-39;
-constexpr double kP3 = -0x1.1fc8f8cbb5bf7p-93;
 
 // Taylor coefficients 1/(2n+1)! and 1/(2n)!: n = 0..5 as fractions of 2^64
 // (1 as 2^64 - 1), n = 6..9 as fractions of 2^60
@@ -84,7 +82,10 @@ __device__ __forceinline__ uint64_t mul_hi(uint64_t a, uint64_t b)
 
 // r = x - k*pi/2 and k (its low bits) for 2^-27 <= |x| < 2^16.  The float
 // copy of x is x truncated to 24 bits, moved there by integer instructions.
-__device__ __forceinline__ double reduce(double x, uint32_t& quadrant)
+// `cancelled`: x is within 2^-20 of a multiple of pi/2 other than 0, where the
+// second part of pi/2 no longer gives r to 53 bits.  (A third FMA there is
+// compiled without a branch, so every call paid for it.)
+__device__ __forceinline__ double reduce(double x, uint32_t& quadrant, bool& cancelled)
 {
     const uint32_t hi = (uint32_t)__double2hiint(x), lo = (uint32_t)__double2loint(x);
     const uint32_t sign = hi & 0x80000000u;
@@ -96,9 +97,8 @@ __device__ __forceinline__ double reduce(double x, uint32_t& quadrant)
     // k as a double (at most 17 bits: the low word is zero)
     const uint32_t kh = (ka == 0 ? 0u : (ka >> 3) + (896u << 20)) | (kf & 0x80000000u);
     const double k = __longlong_as_double((long long)((uint64_t)kh << 32));
-    double r = __fma_rn(-k, kP1, x);
-    r = __fma_rn(-k, kP2, r);
-    if (ka != 0 && ((uint32_t)__double2hiint(r) & 0x7fffffffu) < 0x3eb00000u) r = __fma_rn(-k, kP3, r);
+    const double r = __fma_rn(-k, kP2, __fma_rn(-k, kP1, x));
+    cancelled = ka != 0 && ((uint32_t)__double2hiint(r) & 0x7fffffffu) < 0x3eb00000u;
     return r;
 }
 
@@ -164,9 +164,10 @@ __device__ __forceinline__ double dsin(double x)
 {
     using namespace dtrig;
     const int hi = __double2hiint(x) & 0x7fffffff;
-    if (hi >= kHiLarge) return ::sin(x);
     uint32_t q;
-    const Arg a = arg_of(reduce(x, q));
+    bool cancelled;
+    const Arg a = arg_of(reduce(x, q, cancelled));
+    if (hi >= kHiLarge || (cancelled && hi >= kHiTiny)) return ::sin(x);
     // quadrants 0..3: sin r, cos r, -sin r, -cos r
     const bool odd = q & 1;
     const uint64_t p = poly(a.z, odd);
@@ -179,12 +180,13 @@ __device__ __forceinline__ void dsincos(double x, double* sp, double* cp)
 {
     using namespace dtrig;
     const int hi = __double2hiint(x) & 0x7fffffff;
-    if (hi >= kHiLarge) {
+    uint32_t q;
+    bool cancelled;
+    const Arg a = arg_of(reduce(x, q, cancelled));
+    if (hi >= kHiLarge || (cancelled && hi >= kHiTiny)) {
         ::sincos(x, sp, cp);
         return;
     }
-    uint32_t q;
-    const Arg a = arg_of(reduce(x, q));
     const uint64_t sb = sin_bits(a, poly(a.z, false)), cb = cos_bits(poly(a.z, true));
     const bool odd = q & 1;
     const uint32_t ss = odd ? 0u : a.sign, cs = odd ? a.sign : 0u;

@@ -23,29 +23,41 @@ __device__ __forceinline__ double mul_pow2(double x, double p)
     return __longlong_as_double(bx + ((long long)e << 52));
 }
 
-// a / b for a divisor b whose reciprocal y = RN(1/b) was computed on the host:
-// q = a*y, then two residual corrections q += (a - b*q)*y with exact FMA
-// residuals.  The first makes q a faithful quotient; from a faithful q and
-// |y - 1/b| < 2^-53 |1/b|, the second returns the correctly rounded a / b
-// (Markstein's theorem; P. Markstein, IBM J. Res. Dev. 34(1), 1990, and the
-// Handbook of Floating-Point Arithmetic, ch. 4).  So the double is the IEEE
-// quotient, at five FP64 instructions instead of a full division's reciprocal
-// refinement.  A zero a returns a*y (the IEEE quotient +-0); otherwise |a|
-// or |b| outside [2^-400, 2^401) (subnormals, Inf/NaN, and wherever quotient
-// or residual could leave the normal range) take the IEEE division.
-__device__ __forceinline__ bool is_zero(double a) { return (__double_as_longlong(a) << 1) == 0; }
-
+// The IEEE quotient a / b for a divisor b whose reciprocal y = RN(1/b) was
+// computed on the host, by integer instructions: GB300 issues 2 FP64
+// instructions per SM and cycle, and its integer pipes have time while an FP64
+// step runs.  With the 53-bit mantissas A, B, Y of a, b, y, the high word of
+// A*Y is A/B scaled, off by less than two units of the quotient's 53 bits
+// (y's rounding); the remainder A*2^s - q*B, exact modulo 2^64, then tells
+// which neighbour is nearest.  A quotient of two 53-bit numbers never lies
+// halfway between two doubles.  (Before: the Markstein quotient on the FP64
+// pipe, five instructions, 80 SM cycles a warp against about 25.)  |a| or |b|
+// outside [2^-400, 2^401) (subnormals, Inf/NaN, and wherever the quotient
+// could leave the normal range) take the IEEE division; a zero a returns +-0.
 __device__ __forceinline__ double cdiv(double a, double b, double y)
 {
+    typedef unsigned long long u64;
     constexpr unsigned lo = 1023 - 400, span = 800;  // biased exponents lo .. lo + span
-    const unsigned ea = ((unsigned)__double2hiint(a) >> 20) & 0x7ffu;
-    const unsigned eb = ((unsigned)__double2hiint(b) >> 20) & 0x7ffu;
-    if (eb - lo > span) return a / b;
-    if (is_zero(a)) return __dmul_rn(a, y);
-    if (ea - lo > span) return a / b;
-    double q = __dmul_rn(a, y);
-    q = __fma_rn(__fma_rn(-q, b, a), y, q);
-    return __fma_rn(__fma_rn(-q, b, a), y, q);
+    const u64 ba = (u64)__double_as_longlong(a), bb = (u64)__double_as_longlong(b), by = (u64)__double_as_longlong(y);
+    const unsigned ea = (unsigned)(ba >> 52) & 0x7ffu, eb = (unsigned)(bb >> 52) & 0x7ffu;
+    const u64 sign = (ba ^ bb) & 0x8000000000000000ull;
+    if (ea - lo > span || eb - lo > span) {
+        if ((ba << 1) == 0 && eb - lo <= span) return __longlong_as_double((long long)sign);
+        return a / b;
+    }
+    const u64 mask = 0xfffffffffffffull, one = 0x10000000000000ull;
+    const u64 A = (ba & mask) | one, B = (bb & mask) | one, Y = (by & mask) | one;
+    // A*Y*2^-42 = (A/B)*2^63, or 2^62 where B = 2^52 (then Y = 2^52 too)
+    const u64 An = A << 11, Yn = Y << 11;
+    const unsigned ah = (unsigned)(An >> 32), al = (unsigned)An, yh = (unsigned)(Yn >> 32), yl = (unsigned)Yn;
+    const u64 H = (u64)ah * yh + (((u64)ah * yl) >> 32) + (((u64)al * yh) >> 32);
+    const int below = A < B ? 1 : 0;                      // the quotient is A*2^(52 + below) / B
+    const int shift = 11 - below - (B == one ? 1 : 0);
+    u64 q = (H >> shift) + ((H >> (shift - 1)) & 1);
+    const long long rem = (long long)((A << (52 + below)) - q * B);   // exact: |rem| < 2.6 B < 2^55
+    const long long r2 = 2 * rem, m = (long long)B;
+    q += (u64)((r2 > m ? 1 : 0) + (r2 > 3 * m ? 1 : 0) - (r2 < -m ? 1 : 0) - (r2 < -3 * m ? 1 : 0));
+    return __longlong_as_double((long long)(sign | (((u64)(ea - eb + 1022u - (unsigned)below) << 52) + q)));
 }
 
 }  // namespace lat

@@ -98,6 +98,11 @@ StepCoef make_coef(const lat_params& p, int64_t n)
     c.inv_gyz2 = c.gyz2 != 0 ? 1.0 / c.gyz2 : 0.0;
     c.iso = (p.dx == p.dy && p.dx == p.dz) ? 1.0 : 0.0;
     c.fric_dt = c.fric / p.dt;
+    c.kLap = c.dt2 / c.dx2;
+    c.kPot = c.halfLambda * c.dx2;
+    c.kFric = c.fric * p.dt;
+    c.kCur = c.m2gg * c.dt2;
+    c.kDamp = c.damp * p.dt;
     return c;
 }
 

@@ -118,7 +118,9 @@ inline int64_t partial_pairs(const Geom& g)
     X(inv_dx2) X(inv_dy2) X(inv_dz2) X(inv_dt) X(inv_dx) X(inv_dy) X(inv_dz) X(inv_g) \
     X(inv_gdtdx) X(inv_gdtdy) X(inv_gdtdz) X(inv_gxy2) X(inv_gxz2) X(inv_gyz2) \
     X(iso)                               /* 1 when dx == dy == dz, else 0 */      \
-    X(fric_dt)                           /* fric / dt (fused FP64 step)    */
+    X(fric_dt)                           /* fric / dt (fused FP64 step)    */ \
+    X(kLap) X(kPot) X(kFric) X(kCur) X(kDamp) /* fused FP64 step, equal spacings:  \
+        dt2/dx2, 0.5*lambda*dx2, fric*dt, m2gg*dt2, damp*dt */
 
 template <class R>
 struct StepCoefT {
