@@ -41,6 +41,7 @@ UNITS = {
     "string_ic.cu": ["-fmad=false"],
     "noalloc.cu": ["-fmad=false"],
     "ah_f64_fast.cu": [],
+    "moore_f64_fast.cu": [],
     "ah_f32.cu": [],
     "moore_f32.cu": [],
     "misc.cu": [],

@@ -565,8 +565,15 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
                 f.now[c] = (const double*)h->slot(c, tNow);
                 f.past[c] = (double*)h->slot(c, tPast);
             }
-            LAT_CKL(launch_moore_step_f64(h->geom, f, cf, d, diag, h->stream));
-            used = tile_count(h->geom);
+            if (p.kernel_variant == 1) {
+                LAT_CKL(launch_moore_step_f64(h->geom, f, cf, d, diag, h->stream));
+                used = tile_count(h->geom);
+            } else {
+                LAT_CKL(p.precision == LAT_F64_FAST
+                            ? launch_moore_march_fast(h->geom, f, cf, d, diag, h->recip, h->stream)
+                            : launch_moore_march_strict(h->geom, f, cf, d, diag, h->recip, h->stream));
+                used = (int)moore_march_partials(h->geom);
+            }
         } else {
             Fields<float, 7> f;
             for (int c = 0; c < 7; ++c) {

@@ -87,10 +87,11 @@ inline int flat_grid(unsigned n)
     return (int)((n + b - 1) / b);
 }
 // (energy, |G|) pairs a handle's diagnostic steps may write
+int64_t moore_march_partials(const Geom& g);
 inline int64_t partial_pairs(const Geom& g)
 {
-    const int64_t tiles = tile_count(g), flat = flat_grid(flat_region(g).n);
-    return tiles > flat ? tiles : flat;
+    const int64_t tiles = tile_count(g), flat = flat_grid(flat_region(g).n), march = moore_march_partials(g);
+    return tiles > flat ? (tiles > march ? tiles : march) : (flat > march ? flat : march);
 }
 
 // ---------------------------------------------------------------------------
@@ -179,6 +180,12 @@ cudaError_t launch_ah_twopass_strict(const Geom&, const Fields<double, 5>&, doub
                                      bool diag, bool recip, cudaStream_t);
 cudaError_t launch_ah_twopass_fast(const Geom&, const Fields<double, 5>&, double* L, const StepCoef&, const DiagOut&,
                                    bool diag, bool recip, cudaStream_t);
+// x-marching Moore FP64 step (moore_march.cuh); moore_march_partials: its CTAs,
+// one diagnostic partial each
+cudaError_t launch_moore_march_strict(const Geom&, const Fields<double, 7>&, const StepCoef&, const DiagOut&, bool diag,
+                                      bool recip, cudaStream_t);
+cudaError_t launch_moore_march_fast(const Geom&, const Fields<double, 7>&, const StepCoef&, const DiagOut&, bool diag,
+                                    bool recip, cudaStream_t);
 // x-planes per CTA of the tiled FP32 step for a new handle (tuned value of the
 // shape if known in this process, else a heuristic); tune.cu
 int default_chunk(const lat_params& p);
