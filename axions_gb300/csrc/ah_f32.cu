@@ -1,5 +1,5 @@
-// Abelian-Higgs step kernels, float instantiation: the tiled FP32 step
-// (tiled_step.cuh) and the one-pass kernel kept for cross-checks.
+// Abelian-Higgs step kernels, float instantiation: the FP32 pair step
+// (pair_step.cuh, the tiled step of tiled_step.cuh for checks) and the one-pass kernel kept for cross-checks.
 #include "ah_step.cuh"
 #include "pair_step.cuh"
 #include "tiled_step.cuh"
@@ -12,21 +12,13 @@ cudaError_t launch_ah_step_f32(const Geom& g, const Fields<float, 5>& f, const S
     return launch_ah_step_t<float>(g, f, c, d, diag, st);
 }
 
-// variant 0: the pair step where the layout allows it, else the tiled step
-// (16-byte staging where allowed); 2: the tiled step staging one element per
-// copy; 3: the tiled step with 16-byte staging.  *blocks = the CTAs (and
+// variant 0: the pair step; 2: the tiled step staging one element per
+// copy; 3: the tiled step with 16-byte staging where allowed.  *blocks = the CTAs (and
 // diagnostic partials) of the kernel that ran.
 cudaError_t launch_ah_tiled_f32(const Geom& g, const Fields<float, 5>& f, const StepCoef& c, const DiagOut& d,
                                   bool diag, int chunk, cudaStream_t st, int variant, int* blocks)
 {
-    if (variant == 0) {
-        const cudaError_t e = launch_pair_t<1>(g, f, c, d, diag, chunk, st);
-        if (e != cudaErrorNotSupported) {
-            const dim3 t = pair_grid(g, chunk);
-            *blocks = (int)(t.x * t.y * t.z);
-            return e;
-        }
-    }
+    if (variant == 0) return launch_pair_t<1>(g, f, c, d, diag, chunk, st, blocks);
     const dim3 t = tiled_grid(g, chunk);
     *blocks = (int)(t.x * t.y * t.z);
     return launch_tiled_t<float, 1>(g, f, c, d, diag, chunk, st, variant != 2);
@@ -42,10 +34,11 @@ cudaError_t launch_divergence_f32(const Geom& g, const float* tx, const float* t
 
 namespace lat {
 
-int tiled_blocks(const Geom& g, int chunk)
+int64_t march_tiles(const Geom& g, bool moore)
 {
-    const dim3 t = tiled_grid(g, chunk);
-    return (int)(t.x * t.y * t.z);
+    const dim3 t = pair_shape_grid(g, moore ? 32 : pair_tz2(g), 1), w = tiled_grid(g, 1);
+    const bool pair = !moore || (g.loz == 0 && g.hiz == g.nz && g.nz % 4 == 0 && 10 * g.nz >= 9 * 64 * (int)t.x);
+    return pair ? (int64_t)t.x * t.y : (int64_t)w.x * w.y;
 }
 
 }  // namespace lat

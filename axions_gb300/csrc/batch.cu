@@ -2,14 +2,13 @@
 //
 // The reference runs one lattice per program invocation; an ensemble of small
 // lattices (different seeds, couplings and sizes) is a loop of separate runs.
-// Here every lattice of a batch advances in the same kernel launch: a
-// persistent grid (one or two CTAs per SM) walks a table of work items, one
-// item per (lattice, y/z tile, x-chunk) of the FP32 step: the pair tile
-// (pair_step.cuh, two z-sites per thread) where the lattice's layout allows
-// it, else the tiled step's tile (tiled_step.cuh).  A call advancing K steps is one CUDA graph: a copy of the
-// K per-step job tables from pinned host memory, then for each step the step
-// kernel and a per-lattice diagnostic reduction.  The graph is reused as long
-// as K is; lattices join and leave between calls by rewriting the tables.
+// Here the lattices of a batch advance together: a persistent grid per kernel
+// walks a table of work items, one item per (lattice, y/z tile, x-chunk) of the
+// FP32 pair step (pair_step.cuh) or, for Moore lattices it does not take, the
+// tiled step (tiled_step.cuh).  A call advancing K steps is one CUDA graph: a
+// copy of the K per-step job tables from pinned host memory, then for each
+// kernel its K steps.  The graph is reused as long as K is; lattices join and
+// leave between calls by rewriting the tables.
 //
 // Each lattice's arithmetic uses only its own fields and coefficients and the
 // same tile decomposition as the single-lattice path, and its diagnostics are
@@ -19,6 +18,7 @@
 #include <cstring>
 #include <map>
 #include <string>
+#include <type_traits>
 #include <vector>
 
 #include "lattice_handle.hpp"
@@ -38,15 +38,15 @@ struct BatchJob {
     Geom g;
     Fields<float, 7> f;     // AH uses the first 5 components
     union {
-        StepCoefT<float> c;  // tiled tile
-        PairCoef pc;         // pair tile
+        StepCoefT<float> c;  // tiled step
+        PairCoef pc;         // pair step
     };
     Charges<float> ch;
     DiagOut d;
     int diag;               // record diagnostics at this step
     int chunk;
     int psub;               // planes per diagnostic partial (0: one per item)
-    int vec;                // 16-byte staging (tiled_vec_ok)
+    int vec;                // tiled step: 16-byte staging
     int tiles_z, tiles_y;
     int items;              // tiles_z * tiles_y * x-chunks
     int partials;           // diagnostic partials of the step
@@ -71,7 +71,14 @@ int batch_chunk(const Geom& g)
 
 namespace {
 
-template <int NS, bool PAIR, bool DIAG, bool Q12>
+// the tiled step's tile in place of a PairShape
+struct Tiled {};
+template <class SH>
+constexpr bool is_tiled = std::is_same<SH, Tiled>::value;
+template <int NS, class SH>
+using TileSmem = std::conditional_t<is_tiled<SH>, TiledSmem<float, NS>, PairSmem<NS>>;
+
+template <int NS, class SH, bool DIAG, bool Q12>
 __device__ __forceinline__ void run_item(unsigned char* smem_raw, const BatchJob& J, const Fields<float, 5>& f5,
                                          int bx, int by, int bz)
 {
@@ -79,17 +86,13 @@ __device__ __forceinline__ void run_item(unsigned char* smem_raw, const BatchJob
     const int per = J.psub > 0 ? J.chunk / J.psub : 1;
     const int stride = 2 * J.tiles_y * J.tiles_z;
     double* part = DIAG ? J.d.partials + 2 * ((bz * per * J.tiles_y + by) * J.tiles_z + bx) : nullptr;
-    if constexpr (PAIR) {
-        PairSmem<NS>& ps = *reinterpret_cast<PairSmem<NS>*>(smem_raw);
-        if constexpr (NS == 1) pair_tile<1, DIAG>(ps, J.g, f5, J.pc, J.ch, J.d, bx, by, bz, J.chunk, part, J.psub, stride);
-        else pair_tile<2, DIAG, false, Q12>(ps, J.g, J.f, J.pc, J.ch, J.d, bx, by, bz, J.chunk, part, J.psub, stride);
-        return;
-    }
-    TiledSmem<float, NS>& sm = *reinterpret_cast<TiledSmem<float, NS>*>(smem_raw);
-    if constexpr (NS == 1)
-        tiled_tile<float, 1, DIAG>(sm, J.g, f5, J.c, J.ch, J.d, bx, by, bz, J.chunk, part, J.vec != 0, J.psub, stride);
-    else
+    TileSmem<NS, SH>& sm = *reinterpret_cast<TileSmem<NS, SH>*>(smem_raw);
+    if constexpr (is_tiled<SH>)
         tiled_tile<float, 2, DIAG>(sm, J.g, J.f, J.c, J.ch, J.d, bx, by, bz, J.chunk, part, J.vec != 0, J.psub, stride);
+    else if constexpr (NS == 1)
+        pair_tile<1, DIAG, false, false>(sm, SH{}, J.g, f5, J.pc, J.ch, J.d, bx, by, bz, J.chunk, part, J.psub, stride);
+    else
+        pair_tile<2, DIAG, false, Q12>(sm, SH{}, J.g, J.f, J.pc, J.ch, J.d, bx, by, bz, J.chunk, part, J.psub, stride);
 }
 
 // Sum of a job's n diagnostic partials by the CTA that finished its last item:
@@ -124,21 +127,19 @@ __device__ __forceinline__ void sum_partials(const double* partials, int n, doub
     }
 }
 
-// Persistent step kernel for the lattices with NS scalars that use the pair
-// tile (PAIR) or the tiled tile: CTAs stride over the work items of all of
-// them.  One kernel per model and tile keeps each kernel's register use to
-// that tile's: four 4-warp CTAs per SM for the pair tile, as the pair step,
-// four (Abelian-Higgs) or three (Moore) 8-warp CTAs for the tiled tile.  Q12:
-// the Moore pair lattices with charges 1 and 2, whose link factors the tile
-// forms in closed form (pair_step.cuh).  At a diagnostic step the CTA that
-// finishes a job's last item also sums the job's partials (a separate launch
-// after every step took 3 us of a 64^3 ensemble's step).
-template <int NS, bool PAIR, bool Q12 = false>
-__global__ void __launch_bounds__(PAIR ? PT_THREADS : TT_THREADS, PAIR ? 4 : (NS == 1 ? 4 : 3))
+// Persistent step kernel for the lattices with NS scalars whose tile is SH: CTAs
+// stride over the work items of all of them, four 4-warp CTAs per SM (tiled
+// step: three 8-warp CTAs).  Q12: the Moore lattices with charges 1 and 2,
+// whose link factors the tile forms in closed form (pair_step.cuh).  At a
+// diagnostic step the CTA that finishes a job's last item also sums the job's
+// partials (a separate launch after every step took 3 us of a 64^3 ensemble's
+// step).
+template <int NS, class SH, bool Q12>
+__global__ void __launch_bounds__(is_tiled<SH> ? TT_THREADS : PT_THREADS, is_tiled<SH> ? 3 : 4)
 batch_step_kernel(const BatchHead* __restrict__ tab, BatchJob* __restrict__ jobs)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
-    constexpr int THREADS = PAIR ? PT_THREADS : TT_THREADS;
+    constexpr int THREADS = is_tiled<SH> ? TT_THREADS : PT_THREADS;
     __shared__ BatchJob sj;
     __shared__ Fields<float, 5> sf5;  // Abelian-Higgs view of sj.f
     __shared__ int s_job, s_last;
@@ -177,7 +178,7 @@ batch_step_kernel(const BatchHead* __restrict__ tab, BatchJob* __restrict__ jobs
         const int by = r % sj.tiles_y;
         const int bz = r / sj.tiles_y;
         if (sj.diag) {
-            run_item<NS, PAIR, true, Q12>(smem_raw, sj, sf5, bx, by, bz);
+            run_item<NS, SH, true, Q12>(smem_raw, sj, sf5, bx, by, bz);
             if (tid == 0) {   // the thread that wrote the item's partials
                 __threadfence();
                 s_last = atomicAdd(&jobs[s_job].done, 1) == sj.items - 1;
@@ -188,21 +189,29 @@ batch_step_kernel(const BatchHead* __restrict__ tab, BatchJob* __restrict__ jobs
                 sum_partials<THREADS>(sj.d.partials, sj.partials, sj.diag_out, reinterpret_cast<double*>(smem_raw), tid);
             }
         } else {
-            run_item<NS, PAIR, false, Q12>(smem_raw, sj, sf5, bx, by, bz);
+            run_item<NS, SH, false, Q12>(smem_raw, sj, sf5, bx, by, bz);
         }
         __syncthreads();  // sj and the tile's shared memory are reused by the next item
     }
 }
 
-template <int NS, bool PAIR>
-size_t batch_smem_ns()
+// Job tables (step kernels): 0..3 Abelian-Higgs on 64x4 and 32x8 tiles with
+// 16-byte staging, then with element staging; 4, 5 Moore on 64x4 tiles, with
+// any charges and with 1 and 2; 6 Moore on the tiled step.
+constexpr int kTables = 7;
+enum { kMoorePair = 4, kMoorePair12 = 5, kMooreTiled = 6 };
+using BatchKernel = void (*)(const BatchHead*, BatchJob*);
+const BatchKernel kKernel[kTables] = {
+    batch_step_kernel<1, PairShape<32, true>, false>, batch_step_kernel<1, PairShape<16, true>, false>,
+    batch_step_kernel<1, PairShape<32, false>, false>, batch_step_kernel<1, PairShape<16, false>, false>,
+    batch_step_kernel<2, PairShape<32, true>, false>, batch_step_kernel<2, PairShape<32, true>, true>,
+    batch_step_kernel<2, Tiled, false>};
+size_t table_smem(int table)
 {
-    return PAIR ? sizeof(PairSmem<NS>) : sizeof(TiledSmem<float, NS>);
+    return table == kMooreTiled ? sizeof(TiledSmem<float, 2>) : (table < kMoorePair ? sizeof(PairSmem<1>) : sizeof(PairSmem<2>));
 }
-
-// job tables per step: [tiled AH, tiled Moore, pair AH, pair Moore, pair Moore
-// with charges 1 and 2]
-constexpr int kTables = 5;
+dim3 table_block(int table) { return table == kMooreTiled ? dim3(TT_Z, TT_Y) : dim3(PT_TZ, PT_Y); }
+constexpr size_t kMaxGraphs = 32;  // graphs kept per batch, by the set of tables they launch
 
 }  // namespace
 
@@ -221,14 +230,14 @@ struct lat_batch {
     int device = 0;
     int max_jobs = 0;
     cudaStream_t stream = nullptr;
-    int grid[kTables] = {};          // persistent CTAs of each step kernel (table order)
+    int grid[kTables] = {};          // persistent CTAs of each step kernel
     int K = 0;                       // steps the buffers below hold and the graphs make
     int chunk = 0;                   // x-planes per work item; 0: lat_batch_advance's rule
     char* tab_host = nullptr;        // pinned, and its device copy: BatchHead[K][kTables], then BatchJob[K][max_jobs]
     char* tab_dev = nullptr;
     double* diag_dev = nullptr;      // [K][max_jobs][2]
     double* diag_host = nullptr;     // pinned copy
-    cudaGraphExec_t exec[1 << kTables] = {};   // graphs of K steps, by the set of tables they launch
+    std::map<unsigned, cudaGraphExec_t> exec;  // graphs of K steps, by the set of tables they launch
     cudaStream_t side[kTables] = {};           // one stream per table while a graph is captured
     cudaEvent_t fork = nullptr, join[kTables] = {};
     int64_t launches = 0;
@@ -250,10 +259,8 @@ struct lat_batch {
 
 static void release_graph(lat_batch* b)
 {
-    for (auto& e : b->exec) {
-        if (e) cudaGraphExecDestroy(e);
-        e = nullptr;
-    }
+    for (auto& e : b->exec) cudaGraphExecDestroy(e.second);
+    b->exec.clear();
     cudaFreeHost(b->tab_host);
     cudaFree(b->tab_dev);
     cudaFree(b->diag_dev);
@@ -270,7 +277,7 @@ static void release_graph(lat_batch* b)
 // the tables' chains of K step kernels are independent and form parallel
 // branches: 18 Abelian-Higgs and 6 Moore 64^3 lattices, which fill neither
 // kernel's CTA slots alone, stepped one after the other before.  Graphs are
-// kept per mask (at most 31), as jobs of a model come and go between calls.
+// kept per mask, as jobs of a model come and go between calls.
 static int ensure_graph(lat_batch* b, int K, unsigned mask)
 {
     if (b->K != K) {
@@ -286,7 +293,11 @@ static int ensure_graph(lat_batch* b, int K, unsigned mask)
             BATCH_CK(e);
         }
     }
-    if (b->exec[mask]) return LAT_OK;
+    if (b->exec.count(mask)) return LAT_OK;
+    if (b->exec.size() >= kMaxGraphs) {
+        for (auto& e : b->exec) cudaGraphExecDestroy(e.second);
+        b->exec.clear();
+    }
     BATCH_CK(cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
     cudaMemcpyAsync(b->tab_dev, b->tab_host, b->table_bytes(), cudaMemcpyHostToDevice, b->stream);
     cudaEventRecord(b->fork, b->stream);
@@ -294,16 +305,8 @@ static int ensure_graph(lat_batch* b, int K, unsigned mask)
         if (!(mask & (1u << q))) continue;
         cudaStream_t st = b->side[q];
         cudaStreamWaitEvent(st, b->fork, 0);
-        const dim3 tt(TT_Z, TT_Y), pt(PT_TZ, PT_Y);
-        for (int s = 0; s < K; ++s) {
-            const BatchHead* t = b->head(b->tab_dev, s, q);
-            BatchJob* j = b->jobs_of(b->tab_dev, s);
-            if (q == 0) batch_step_kernel<1, false><<<b->grid[0], tt, batch_smem_ns<1, false>(), st>>>(t, j);
-            else if (q == 1) batch_step_kernel<2, false><<<b->grid[1], tt, batch_smem_ns<2, false>(), st>>>(t, j);
-            else if (q == 2) batch_step_kernel<1, true><<<b->grid[2], pt, batch_smem_ns<1, true>(), st>>>(t, j);
-            else if (q == 3) batch_step_kernel<2, true><<<b->grid[3], pt, batch_smem_ns<2, true>(), st>>>(t, j);
-            else batch_step_kernel<2, true, true><<<b->grid[4], pt, batch_smem_ns<2, true>(), st>>>(t, j);
-        }
+        for (int s = 0; s < K; ++s)
+            kKernel[q]<<<b->grid[q], table_block(q), table_smem(q), st>>>(b->head(b->tab_dev, s, q), b->jobs_of(b->tab_dev, s));
         cudaEventRecord(b->join[q], st);
         cudaStreamWaitEvent(b->stream, b->join[q], 0);
     }
@@ -311,28 +314,26 @@ static int ensure_graph(lat_batch* b, int K, unsigned mask)
                     b->stream);
     cudaGraph_t graph = nullptr;
     BATCH_CK(cudaStreamEndCapture(b->stream, &graph));
-    const cudaError_t e = cudaGraphInstantiate(&b->exec[mask], graph, 0);
+    cudaGraphExec_t exec = nullptr;
+    const cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
     cudaGraphDestroy(graph);
-    if (e != cudaSuccess) b->exec[mask] = nullptr;
     BATCH_CK(e);
+    b->exec[mask] = exec;
     return LAT_OK;
 }
 
-// The table (step kernel) of a lattice: the pair tile where its own layout
-// allows it, else the tiled tile; its model; for a Moore pair lattice whether
-// its charges are 1 and 2.  The choice depends on the lattice alone, never on
-// its company.
+// The table (step kernel) of a lattice, by its model and tile, for a Moore
+// lattice also whether its charges are 1 and 2: it depends on the lattice alone,
+// never on its company.
 static int table_of(const lat_handle* h, const Fields<float, 7>& fj)
 {
-    Fields<float, 5> f5;
-    for (int c = 0; c < 5; ++c) {
-        f5.now[c] = fj.now[c];
-        f5.past[c] = fj.past[c];
+    if (h->p.model == LAT_MODEL_MOORE) {
+        if (!pair_moore_ok(h->geom, fj)) return kMooreTiled;
+        return small_int_power(h->p.q1) == 1 && small_int_power(h->p.q2) == 2 ? kMoorePair12 : kMoorePair;
     }
-    const bool moore = h->p.model == LAT_MODEL_MOORE;
-    const bool pair = moore ? pair_ok(h->geom, fj) : pair_ok(h->geom, f5);
-    const bool q12 = moore && pair && small_int_power(h->p.q1) == 1 && small_int_power(h->p.q2) == 2;
-    return q12 ? 4 : (pair ? 2 : 0) + (moore ? 1 : 0);
+    Fields<float, 5> f5;
+    for (int c = 0; c < 5; ++c) f5.now[c] = fj.now[c];
+    return (tiled_vec_ok(h->geom, f5) ? 0 : 2) + (pair_tz2(h->geom) == 32 ? 0 : 1);
 }
 
 static Fields<float, 7> level_fields(const lat_handle* h, int64_t n)
@@ -365,17 +366,13 @@ int lat_batch_create(int32_t max_jobs, lat_batch** out)
     }
     int sms = 0;
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, b->device);
-    auto grid_of = [&](auto kernel, int threads, size_t smem) {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    for (int q = 0; q < kTables; ++q) {
+        const size_t smem = table_smem(q);
+        cudaFuncSetAttribute(kKernel[q], cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, threads, smem);
-        return std::max(1, sms * std::max(1, per_sm));
-    };
-    b->grid[0] = grid_of(batch_step_kernel<1, false>, TT_THREADS, batch_smem_ns<1, false>());
-    b->grid[1] = grid_of(batch_step_kernel<2, false>, TT_THREADS, batch_smem_ns<2, false>());
-    b->grid[2] = grid_of(batch_step_kernel<1, true>, PT_THREADS, batch_smem_ns<1, true>());
-    b->grid[3] = grid_of(batch_step_kernel<2, true>, PT_THREADS, batch_smem_ns<2, true>());
-    b->grid[4] = grid_of(batch_step_kernel<2, true, true>, PT_THREADS, batch_smem_ns<2, true>());
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kKernel[q], (int)(table_block(q).x * table_block(q).y), smem);
+        b->grid[q] = std::max(1, sms * std::max(1, per_sm));
+    }
     bool ok = cudaEventCreateWithFlags(&b->fork, cudaEventDisableTiming) == cudaSuccess;
     for (int q = 0; q < kTables; ++q)
         ok = ok && cudaStreamCreateWithFlags(&b->side[q], cudaStreamNonBlocking) == cudaSuccess &&
@@ -519,7 +516,7 @@ int lat_batch_advance(lat_batch* b, int32_t nsteps)
         for (size_t q = 0; q < b->jobs.size(); ++q) {
             if (plan[q].steps == 0) continue;
             const Geom& g = b->jobs[q].h->geom;
-            items += march_tiles(g) * ((g.hix - g.lox + c - 1) / c);
+            items += march_tiles(g, b->jobs[q].h->p.model == LAT_MODEL_MOORE) * ((g.hix - g.lox + c - 1) / c);
         }
         if (items >= 1100) chunk = c;
     }
@@ -552,8 +549,8 @@ int lat_batch_advance(lat_batch* b, int32_t nsteps)
         J.chunk = b->chunk > 0 ? std::min(x, b->chunk) : std::max(chunk, planes);
         J.psub = J.chunk % planes == 0 ? planes : 0;
         J.vec = tiled_vec_ok(h->geom, level_fields(h, h->n)) ? 1 : 0;
-        const bool pair = plan[q].table >= 2;
-        const dim3 tg = pair ? pair_grid(h->geom, J.chunk) : tiled_grid(h->geom, J.chunk);
+        const dim3 tg = plan[q].table == kMooreTiled ? tiled_grid(h->geom, J.chunk)
+                                                     : pair_shape_grid(h->geom, moore ? 32 : pair_tz2(h->geom), J.chunk);
         J.tiles_z = (int)tg.x;
         J.tiles_y = (int)tg.y;
         J.items = (int)(tg.x * tg.y * tg.z);
@@ -577,8 +574,8 @@ int lat_batch_advance(lat_batch* b, int32_t nsteps)
                 J = tmpl[q];
                 J.f = level_fields(h, n);
                 const StepCoef c64 = make_coef(h->p, n);
-                if (t >= 2) J.pc = pair_coef(c64);
-                else J.c = coef_as<float>(c64);
+                if (t == kMooreTiled) J.c = coef_as<float>(c64);
+                else J.pc = pair_coef(c64);
                 const bool diag = j.diag_every > 0 && n % j.diag_every == 0;
                 const bool next_diag = j.diag_every > 0 && (n + 1) % j.diag_every == 0;
                 J.d.store_div = next_diag && h->p.g != 0;  // keep div(theta) for the next step's Gauss term

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <initializer_list>
 #include <string>
 
 #include "../../include/lattice_gpu.h"
@@ -88,10 +89,13 @@ inline int flat_grid(unsigned n)
 }
 // (energy, |G|) pairs a handle's diagnostic steps may write
 int64_t moore_march_partials(const Geom& g);
+int64_t march_tiles(const Geom& g, bool moore);   // tiles of a plane of the x-marching FP32 step
 inline int64_t partial_pairs(const Geom& g)
 {
-    const int64_t tiles = tile_count(g), flat = flat_grid(flat_region(g).n), march = moore_march_partials(g);
-    return tiles > flat ? (tiles > march ? tiles : march) : (flat > march ? flat : march);
+    int64_t most = tile_count(g);
+    for (const int64_t n : {(int64_t)flat_grid(flat_region(g).n), moore_march_partials(g), march_tiles(g, false) * (g.hix - g.lox)})
+        most = n > most ? n : most;
+    return most;
 }
 
 // ---------------------------------------------------------------------------
@@ -189,15 +193,11 @@ cudaError_t launch_moore_march_fast(const Geom&, const Fields<double, 7>&, const
 // x-planes per CTA of the tiled FP32 step for a new handle (tuned value of the
 // shape if known in this process, else a heuristic); tune.cu
 int default_chunk(const lat_params& p);
-// tiles of a plane of the x-marching step
-int64_t march_tiles(const Geom& g);
 // x-planes per CTA of a served lattice's final diagnostics (its shape only)
 int batch_chunk(const Geom& g);
-// number of CTAs (and diagnostic partials) of the tiled FP32 step
-int tiled_blocks(const Geom&, int chunk);
 // x-marching FP32 steps, `chunk` x-planes per CTA.  variant 0: the pair step
-// (two z-sites per thread, pair_step.cuh) where the layout allows it, else the
-// tiled step (tiled_step.cuh); 2: the tiled step with one-element staging
+// (two z-sites per thread, pair_step.cuh; Moore lattices where pair_moore_ok,
+// else the tiled step); 2: the tiled step (tiled_step.cuh) with one-element staging
 // copies; 3: the tiled step with 16-byte staging where allowed.  *blocks
 // receives the CTAs (diagnostic partials) of the kernel launched.
 cudaError_t launch_ah_tiled_f32(const Geom&, const Fields<float, 5>&, const StepCoef&, const DiagOut&, bool diag,

@@ -1,5 +1,5 @@
-// Moore-model step kernels, float instantiation: the tiled FP32 step
-// (tiled_step.cuh, two scalars) and the one-pass kernel kept for cross-checks.
+// Moore-model step kernels, float instantiation: the FP32 pair step
+// (pair_step.cuh, the tiled step of tiled_step.cuh for checks, two scalars) and the one-pass kernel kept for cross-checks.
 #include "moore_step.cuh"
 #include "pair_step.cuh"
 #include "tiled_step.cuh"
@@ -12,21 +12,13 @@ cudaError_t launch_moore_step_f32(const Geom& g, const Fields<float, 7>& f, cons
     return launch_moore_step_t<float>(g, f, c, d, diag, st);
 }
 
-// variant 0: the pair step where the layout allows it, else the tiled step
-// (16-byte staging where allowed); 2: the tiled step staging one element per
-// copy; 3: the tiled step with 16-byte staging.  *blocks = the CTAs (and
+// variant 0: the pair step (pair_moore_ok), else the tiled step; 2: the tiled step staging one element per
+// copy; 3: the tiled step with 16-byte staging where allowed.  *blocks = the CTAs (and
 // diagnostic partials) of the kernel that ran.
 cudaError_t launch_moore_tiled_f32(const Geom& g, const Fields<float, 7>& f, const StepCoef& c, const DiagOut& d,
                                      bool diag, int chunk, cudaStream_t st, int variant, int* blocks)
 {
-    if (variant == 0) {
-        const cudaError_t e = launch_pair_t<2>(g, f, c, d, diag, chunk, st);
-        if (e != cudaErrorNotSupported) {
-            const dim3 t = pair_grid(g, chunk);
-            *blocks = (int)(t.x * t.y * t.z);
-            return e;
-        }
-    }
+    if (variant == 0 && pair_moore_ok(g, f)) return launch_pair_t<2>(g, f, c, d, diag, chunk, st, blocks);
     const dim3 t = tiled_grid(g, chunk);
     *blocks = (int)(t.x * t.y * t.z);
     return launch_tiled_t<float, 2>(g, f, c, d, diag, chunk, st, variant != 2);

@@ -13,7 +13,7 @@
 // friends): one instruction updates two sites.  A pair is also one 8-byte
 // shared-memory or global access, and its inner z-neighbours are in
 // registers.  The structure is otherwise the tiled step's:
-//   * a CTA (4 warps) owns a 64 (z) x 4 (y) tile and marches `chunk`
+//   * a CTA (4 warps) owns a 64 (z) x 4 (y) or 32 x 8 tile and marches `chunk`
 //     x-planes; four CTAs share an SM, so while one waits at a barrier the
 //     others issue (8-row tiles of 8 warps, two per SM, ran 6 % slower);
 //   * each plane's now level, tile plus one-site halo, is staged in shared
@@ -37,9 +37,11 @@
 //   * Moore with charges 1 and 2 (the benchmark's) runs a kernel instance with
 //     e^{i q theta} in closed form instead of the general power loop, the same
 //     operations (0.711 -> 0.767).
-// Used where the layout allows 16-byte chunks and aligned pairs: periodic z,
-// nz a multiple of 4, 16-byte aligned fields (every benchmark and serving
-// shape); x and y may be periodic or fixed.  Elsewhere the tiled step runs.
+// 16-byte chunks and 8-byte pairs need periodic z, nz a multiple of 4 and
+// 16-byte aligned fields (every benchmark and serving shape); odd extents and
+// fixed z walls take an instance that stages and accesses single elements
+// (Abelian-Higgs 201 x 199 x 203: 138 us a step, 146 on the one-site tiled step;
+// 96^3 on 32x8 tiles 16.5 us, 18.6 before; 32^3 4.3, 6.2 before).
 // HBM traffic is the algorithmic 3 accesses per value.  Energy and Gauss sums
 // are accumulated in FP64.
 #pragma once
@@ -52,13 +54,12 @@
 namespace lat {
 
 constexpr int PT_TZ = 32;              // threads along z (each two sites)
-constexpr int PT_Z = 2 * PT_TZ;        // tile width along z
-constexpr int PT_Y = 4;                // tile height along y (warps per CTA)
+constexpr int PT_Y = 4;                // warps per CTA (rows of a 32-pair tile)
 constexpr int PT_THREADS = PT_TZ * PT_Y;
-constexpr int PT_HY = PT_Y + 2;        // staged rows j0-1 .. j0+PT_Y
-constexpr int PT_PZ = 72;              // staged row pitch (floats): column c holds z = k0 - 4 + c
-constexpr int PT_C0 = 4;               // column of z = k0 (16-byte aligned; own pairs 8-byte aligned)
-constexpr int PT_NQ = PT_PZ / 4;       // 16-byte chunks per staged row
+// the 64x4 tile's shared memory, which every shape fits: staged rows j0-1 ..
+// j0+4 of 72 floats (column c0 + m holds z = k0 + m)
+constexpr int PT_HY = PT_Y + 2;
+constexpr int PT_PZ = 72;
 constexpr int PT_LY = PT_Y + 1;        // link rows j0-1 .. j0+PT_Y-1 (row ly holds j0 - 1 + ly)
 constexpr int PT_LP = 68;              // link row pitch (floats): column PT_LC0 + m holds z = k0 + m
 constexpr int PT_LC0 = 2;
@@ -146,21 +147,27 @@ __device__ __forceinline__ void charged2_fixed(float2 c1, float2 s1, float2& cq,
     }
 }
 
-// Whether the pair step runs: 16-byte staging and 8-byte aligned pairs, and
-// z-tiles at least 90 % full.  A 64-wide pair tile on nz = 32 leaves half its
-// threads idle, where the 32-wide tiled step fills its tiles (a 32^3 ensemble
-// ran 1.5x faster on the tiled step); nz = 64, 128, 192, 256, 512, 768 and
-// nz >= 576 qualify.
-template <int NC>
-inline bool pair_ok(const Geom& g, const Fields<float, NC>& f)
-{
-    const int tiles = (g.nz + PT_Z - 1) / PT_Z;
-    return tiled_vec_ok<float, NC>(g, f) && 10 * g.nz >= 9 * PT_Z * tiles;
-}
+// Tile shapes, 128 threads with compile-time strides: thread t owns pair
+// t % TZ2 of row t / TZ2.  VEC: 16-byte staging and 8-byte aligned pairs
+// (periodic z, nz a multiple of 4); else one element per copy and access (odd
+// extents, fixed z walls), where the last pair of a row may be a single site.
+// A half-warp reads 16 pairs of one row, so that neither 32 nor 16 pairs a row
+// have bank conflicts.  (Tiles fitted to the lattice at run time, 24x5 for 48
+// or 21x6 for 201, had them, and lost more than the idle lanes they saved: 277
+// us against 235 for a step of 12 + 4 lattices of 96^3.)
+template <int TZ2, bool VEC>
+struct PairShape {
+    static constexpr int tz2 = TZ2, ty = PT_THREADS / TZ2, pitch = 2 * TZ2 + (VEC ? 8 : 4), lpitch = 2 * TZ2 + 4,
+                         c0 = VEC ? 4 : 2;
+    static constexpr bool vec = VEC;
+    static_assert((ty + 2) * pitch <= PT_HY * PT_PZ && (ty + 1) * lpitch <= PT_LY * PT_LP, "the tile's shared memory");
+    static_assert(VEC ? (ty + 2) * (TZ2 / 2 + 2) <= PT_THREADS : ty + 2 <= 12, "the staging plan");
+};
 
-inline dim3 pair_grid(const Geom& g, int chunk)
+inline dim3 pair_shape_grid(const Geom& g, int tz2, int chunk)
 {
-    return dim3((unsigned)((g.nz + PT_Z - 1) / PT_Z), (unsigned)((g.hiy - g.loy + PT_Y - 1) / PT_Y),
+    const int ty = PT_THREADS / tz2;
+    return dim3((unsigned)((g.hiz - g.loz + 2 * tz2 - 1) / (2 * tz2)), (unsigned)((g.hiy - g.loy + ty - 1) / ty),
                 (unsigned)((g.hix - g.lox + chunk - 1) / chunk));
 }
 
@@ -212,25 +219,74 @@ inline PairCoef pair_coef(const StepCoef& c)
     return o;
 }
 
-// Issue the 16-byte copies of plane `pi` into stage b: thread p < PT_HY*PT_NQ
-// copies (row p / PT_NQ, chunk p % PT_NQ) of every component.  Chunk q of row
-// hy holds z = k0-4+4q .. k0-1+4q of row j0-1+hy; only the rows and chunks the
-// tile's in-range sites use are copied (rows hy <= wy+1, chunks q <= 1+wz/4),
-// whose indices wrap at most once.
-template <int NS>
-__device__ __forceinline__ void pair_stage(PairSmem<NS>& sm, int b, const Fields<float, 2 * NS + 3>& f, const Geom& g,
-                                           int pi, int off, int dst)
+// Staging of a plane.  16-byte copies: thread p < rows*chunks copies (row
+// p / chunks, chunk p % chunks) of every component; chunk q of row hy holds
+// z = k0-4+4q .. k0-1+4q of row j0-1+hy; only the rows and chunks the tile's
+// in-range sites use are copied (rows hy <= wy+1, chunks q <= 1+wz/4), whose
+// indices wrap at most once.  Element copies: warp w copies rows w, w+4, w+8,
+// its lanes columns lane, lane+32, lane+64 of z = k0-1 .. k0+wz.
+struct PairPlan {
+    int off, dst;          // 16-byte copies: source within a plane, destination within a component (or -1)
+    int row[3], col[3];    // element copies: sources of the warp's rows and the lane's columns (or -1)
+};
+
+template <int NS, class SH>
+__device__ __forceinline__ PairPlan pair_plan(const SH& sh, const Geom& g, int tid, int j0, int k0, int wy, int wz)
 {
-    if (dst >= 0) {
-        const int s = pi * (int)g.syz + off;   // below nx*ny*nz < 2^31
+    PairPlan pl;
+    pl.off = 0;
+    pl.dst = -1;
+    if constexpr (SH::vec) {
+        const int nq = sh.pitch / 4;
+        const int hq = tid / nq, q = tid - hq * nq;
+        if (hq < sh.ty + 2 && hq <= wy + 1 && q <= 1 + (wz >> 2)) {
+            pl.off = wrap_idx(j0 - 1 + hq, g.ny) * g.nz + wrap_idx(k0 - 4 + 4 * q, g.nz);
+            pl.dst = hq * sh.pitch + 4 * q;
+        }
+    }
+    if constexpr (!SH::vec) {
 #pragma unroll
-        for (int c = 0; c < 2 * NS + 3; ++c)
-            __pipeline_memcpy_async(&sm.st[b][c][0][0] + dst, f.now[c] + s, 16);
+        for (int r = 0; r < 3; ++r) {
+            const int hq = (tid >> 5) + 4 * r, q = (tid & 31) + 32 * r;
+            pl.row[r] = hq <= wy + 1 ? wrap_idx(j0 - 1 + hq, g.ny) * g.nz : -1;
+            pl.col[r] = q <= wz + 1 ? wrap_idx(k0 - 1 + q, g.nz) : -1;
+        }
+    }
+    return pl;
+}
+
+template <int NS, class SH>
+__device__ __forceinline__ void pair_stage(PairSmem<NS>& sm, const SH& sh, int b, const Fields<float, 2 * NS + 3>& f,
+                                           const Geom& g, int pi, const PairPlan& pl)
+{
+    const int base = pi * (int)g.syz;   // below nx*ny*nz < 2^31
+    if constexpr (SH::vec) {
+        if (pl.dst >= 0) {
+            const int s = base + pl.off;
+#pragma unroll
+            for (int c = 0; c < 2 * NS + 3; ++c)
+                __pipeline_memcpy_async(&sm.st[b][c][0][0] + pl.dst, f.now[c] + s, 16);
+        }
+    } else {
+        const int w = (int)(threadIdx.y * PT_TZ + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+#pragma unroll
+        for (int r = 0; r < 3; ++r) {
+            if (pl.row[r] < 0) continue;
+#pragma unroll
+            for (int q = 0; q < 3; ++q) {
+                if (pl.col[q] < 0) continue;
+                const int s = base + pl.row[r] + pl.col[q];
+                float* const dst = &sm.st[b][0][0][0] + (w + 4 * r) * sh.pitch + sh.c0 - 1 + lane + 32 * q;
+#pragma unroll
+                for (int c = 0; c < 2 * NS + 3; ++c)
+                    __pipeline_memcpy_async(dst + c * PT_HY * PT_PZ, f.now[c] + s, 4);
+            }
+        }
     }
     __pipeline_commit();
 }
 
-// One tile: z-pairs (bx*64.., by*4..) of the evolved region, x-planes
+// One tile: z-pairs (bx*2*tz2.., by*ty..) of the evolved region, x-planes
 // [bz*chunk, bz*chunk + chunk).  Called by every thread of the CTA.  With DIAG
 // the CTA's energy and |G| sums are written to part[0], part[1]; with psub > 0
 // the sums of every psub planes to part[0..1], part[pstride..], ...  PIPE: the
@@ -239,8 +295,8 @@ __device__ __forceinline__ void pair_stage(PairSmem<NS>& sm, int b, const Fields
 // without copies); Abelian-Higgs in its own kernel.  The Moore tile, at the
 // register limit of four CTAs per SM, and the batch kernel, which holds both
 // DIAG forms, keep the plain march.
-template <int NS, bool DIAG, bool PIPE = false, bool Q12 = false>
-__device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const Fields<float, 2 * NS + 3>& f,
+template <int NS, bool DIAG, bool PIPE, bool Q12, class SH>
+__device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const SH& sh, const Geom& g, const Fields<float, 2 * NS + 3>& f,
                                           const PairCoef& c, const Charges<float>& ch, const DiagOut& d, int bx,
                                           int by, int bz, int chunk, double* part, int psub = 0, int pstride = 0)
 {
@@ -256,33 +312,47 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
         }
     };
 
-    const int tz = threadIdx.x, ty = threadIdx.y;
-    const int tid = ty * PT_TZ + tz;
-    const int k0 = bx * PT_Z;
-    const int j0 = g.loy + by * PT_Y;
+    const int tid = threadIdx.y * PT_TZ + threadIdx.x;
+    constexpr int per = PT_TZ / SH::tz2;   // rows of a warp
+    const int ty = per == 1 ? threadIdx.y : threadIdx.y * per + threadIdx.x / SH::tz2;
+    const int tz = per == 1 ? threadIdx.x : threadIdx.x % SH::tz2;
+    const int k0 = SH::vec ? bx * 2 * sh.tz2 : g.loz + bx * 2 * sh.tz2;
+    const int j0 = g.loy + by * sh.ty;
     const int ib = g.lox + bz * chunk;
     const int ie = min(ib + chunk, g.hix);
-    const int wy = min(PT_Y, g.hiy - j0), wz = min(PT_Z, g.nz - k0);
+    const int wy = min(sh.ty, g.hiy - j0), wz = min(2 * sh.tz2, (SH::vec ? g.nz : g.hiz) - k0);
     const int k = k0 + 2 * tz, j = j0 + ty;
     const bool active = (2 * tz < wz) && (ty < wy);
     const int kk = active ? k : k0, jj = active ? j : j0;    // in-range copy for the prologue loads
     const int hy = ty + 1;                                    // own staged row
-    const int col = PT_C0 + 2 * tz;                           // own staged column (z = k)
+    const int col = sh.c0 + 2 * tz;                           // own staged column (z = k)
     const int ly = ty + 1, lcol = PT_LC0 + 2 * tz;            // own link position
-
-    // staging plan: (row, chunk) of this thread, or none
-    int soff = 0, sdst = -1;
-    {
-        const int hq = tid / PT_NQ, q = tid - hq * PT_NQ;
-        if (tid < PT_HY * PT_NQ && hq <= wy + 1 && q <= 1 + (wz >> 2)) {
-            soff = wrap_idx(j0 - 1 + hq, g.ny) * g.nz + wrap_idx(k0 - 4 + 4 * q, g.nz);
-            sdst = hq * PT_PZ + 4 * q;
+    // wide: pairs are 8-byte aligned and complete; else the second site of a
+    // row's last pair may lie outside the region
+    constexpr bool wide = SH::vec;
+    const bool second = wide || 2 * tz + 1 < wz;
+    auto ld = [&](const float* p) {
+        return wide ? *reinterpret_cast<const float2*>(p) : make_float2(p[0], second ? p[1] : 0.f);
+    };
+    auto store = [&](float* p, float2 v) {
+        if (wide) {
+            *reinterpret_cast<float2*>(p) = v;
+        } else {
+            p[0] = v.x;
+            if (second) p[1] = v.y;
         }
-    }
-    // halo tasks: the last warp the low row (ly = 0) as pairs, the first PT_Y lanes of the
-    // warp before it the low column (z = k0-1); threads 0 .. PT_HY*PT_NQ-1 issue the staging copies
-    const bool halo_row = ty == PT_Y - 1;
-    const bool halo_col = ty == PT_Y - 2 && tz < PT_Y;
+    };
+    const PairPlan plan = pair_plan<NS>(sh, g, tid, j0, k0, wy, wz);
+    auto stage = [&](int b, int pi) { pair_stage<NS>(sm, sh, b, f, g, wrap_idx(pi, g.nx), plan); };
+    // halo tasks: the low row (link row 0) as pairs by the last threads, the low
+    // column (z = k0-1) by those before them; threads from 0 on issue the 16-byte copies
+    const bool halo_row = ty == SH::ty - 1;
+    const bool halo_col = threadIdx.y == 2 && threadIdx.x < SH::ty;
+    const int hp = tz, hr = threadIdx.x + 1;
+    constexpr int CS = PT_HY * PT_PZ;   // floats per staged component
+    auto at = [&](const float* base, int comp, int row, int column) { return base + comp * CS + row * sh.pitch + column; };
+    constexpr int LS = PT_LY * PT_LP;   // floats per link array
+    auto lk = [&](int a, int row, int column) { return &sm.L[0][0][0] + a * LS + row * sh.lpitch + column; };
 
     const float2 inv_dx2 = p2(c.inv_dx2), inv_dy2 = p2(c.inv_dy2), inv_dz2 = p2(c.inv_dz2);
 
@@ -294,12 +364,12 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
         const long long sxp = ((long long)ib0 * g.ny + jj) * g.nz + kk;
         const long long syp = ((long long)im * g.ny + wrap_idx(jj + 1, g.ny)) * g.nz + kk;
         const long long szp = ((long long)im * g.ny + jj) * g.nz + wrap_idx(kk + 2, g.nz);
-        const float2 tx = *reinterpret_cast<const float2*>(f.now[TH] + s);
-        const float2 tyv = *reinterpret_cast<const float2*>(f.now[TH + 1] + s);
-        const float2 tzv = *reinterpret_cast<const float2*>(f.now[TH + 2] + s);
-        const float2 tyxp = *reinterpret_cast<const float2*>(f.now[TH + 1] + sxp);
-        const float2 tzxp = *reinterpret_cast<const float2*>(f.now[TH + 2] + sxp);
-        const float2 txyp = *reinterpret_cast<const float2*>(f.now[TH] + syp);
+        // the pair's second site is read at its wrapped position (it may be the
+        // first one's forward neighbour outside the region)
+        const int up = wide ? 1 : wrap_idx(kk + 1, g.nz) - kk;
+        auto ld2 = [&](const float* p) { return wide ? *reinterpret_cast<const float2*>(p) : make_float2(p[0], p[up]); };
+        const float2 tx = ld2(f.now[TH] + s), tyv = ld2(f.now[TH + 1] + s), tzv = ld2(f.now[TH + 2] + s);
+        const float2 tyxp = ld2(f.now[TH + 1] + sxp), tzxp = ld2(f.now[TH + 2] + sxp), txyp = ld2(f.now[TH] + syp);
         const float2 txzp = make_float2(tx.y, f.now[TH][szp]);
         float2 c1, s1;
         sincos2(tx, s1, c1);
@@ -309,12 +379,12 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
         sPxz_xm = sin2(sub2(sub2(add2(tx, tzxp), txzp), tzv));
         txm = tx;
 #pragma unroll
-        for (int cc = 0; cc < 2 * NS; ++cc) vm[cc] = *reinterpret_cast<const float2*>(f.now[cc] + s);
+        for (int cc = 0; cc < 2 * NS; ++cc) vm[cc] = ld2(f.now[cc] + s);
     }
     constexpr int ST = pt_stages<NS>();
     int cur = 0;
 #pragma unroll
-    for (int b = 0; b < ST - 1; ++b) pair_stage<NS>(sm, b, f, g, wrap_idx(ib + b, g.nx), soff, sdst);
+    for (int b = 0; b < ST - 1; ++b) stage(b, ib + b);
 
     double e_acc = 0.0, g_acc = 0.0;
     // the CTA's sums so far to `part`
@@ -324,9 +394,9 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
             e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
             g_acc += __shfl_down_sync(0xffffffffu, g_acc, o);
         }
-        if (tz == 0) {
-            sm.red[0][ty] = e_acc;
-            sm.red[1][ty] = g_acc;
+        if ((tid & 31) == 0) {
+            sm.red[0][tid >> 5] = e_acc;
+            sm.red[1][tid >> 5] = g_acc;
         }
         __syncthreads();
         if (tid == 0) {
@@ -348,7 +418,7 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
         const int s0 = (ib * g.ny + jj) * g.nz + kk;
 #pragma unroll
         for (int cc = 0; cc < 2 * NS + 3; ++cc)
-            qn[cc] = (active && ib < ie) ? *reinterpret_cast<const float2*>(f.past[cc] + s0) : p2(0.f);
+            qn[cc] = (active && ib < ie) ? ld(f.past[cc] + s0) : p2(0.f);
     }
     // own values of the current plane carried from the previous plane's x-forward reads
     float2 v[2 * NS], tyo, tzo;
@@ -366,12 +436,10 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
         __syncthreads();
         // plane i+ST-1 into the slot plane i-1 left; one group per plane, so
         // that the wait above always counts planes
-        if (i + ST - 2 < ie) pair_stage<NS>(sm, nn, f, g, wrap_idx(i + ST - 1, g.nx), soff, sdst);
+        if (i + ST - 2 < ie) stage(nn, i + ST - 1);
         else __pipeline_commit();
         const float* S = &sm.st[cur][0][0][0];
         const float* X = &sm.st[nxt][0][0][0];
-        constexpr int CS = PT_HY * PT_PZ;   // floats per staged component
-        auto at = [&](const float* base, int comp, int row, int column) { return base + comp * CS + row * PT_PZ + column; };
 
         // the own pair's level n-1: loaded now so that the link phase covers the
         // latency, or (PIPE) taken from the previous plane's load
@@ -383,11 +451,11 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
             if (active && i + 1 < ie) {
 #pragma unroll
                 for (int cc = 0; cc < 2 * NS + 3; ++cc)
-                    qn[cc] = *reinterpret_cast<const float2*>(f.past[cc] + (s + (int)g.syz));
+                    qn[cc] = ld(f.past[cc] + (s + (int)g.syz));
             }
         } else if (active) {
 #pragma unroll
-            for (int cc = 0; cc < 2 * NS + 3; ++cc) qv[cc] = *reinterpret_cast<const float2*>(f.past[cc] + s);
+            for (int cc = 0; cc < 2 * NS + 3; ++cc) qv[cc] = ld(f.past[cc] + s);
         } else {
 #pragma unroll
             for (int cc = 0; cc < 2 * NS + 3; ++cc) qv[cc] = p2(0.f);
@@ -431,50 +499,51 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
         }
 #pragma unroll
         for (int q = 0; q < NS; ++q) {
-            sts2(&sm.L[LI::cy(q)][ly][lcol], cy[q]);
-            sts2(&sm.L[LI::sy(q)][ly][lcol], sy[q]);
-            sts2(&sm.L[LI::cz(q)][ly][lcol], cz[q]);
-            sts2(&sm.L[LI::sz(q)][ly][lcol], sz[q]);
+            sts2(lk(LI::cy(q), ly, lcol), cy[q]);
+            sts2(lk(LI::sy(q), ly, lcol), sy[q]);
+            sts2(lk(LI::cz(q), ly, lcol), cz[q]);
+            sts2(lk(LI::sz(q), ly, lcol), sz[q]);
         }
-        sts2(&sm.L[LI::pxy][ly][lcol], sPxy);
-        sts2(&sm.L[LI::pxz][ly][lcol], sPxz);
-        sts2(&sm.L[LI::pyz][ly][lcol], sPyz);
+        sts2(lk(LI::pxy, ly, lcol), sPxy);
+        sts2(lk(LI::pxz, ly, lcol), sPxz);
+        sts2(lk(LI::pyz, ly, lcol), sPyz);
         if (halo_row) {
+            const int hcol = sh.c0 + 2 * hp, hl = PT_LC0 + 2 * hp;
             // row j0-1 (staged row 0), the pair at z = k: what row j0 reads as its y-backward data
-            const float2 hty = lds2(at(S, TH + 1, 0, col)), htx = lds2(at(S, TH, 0, col));
-            const float2 htz = lds2(at(S, TH + 2, 0, col));
-            const float2 htyxp = lds2(at(X, TH + 1, 0, col)), htxyp = lds2(at(S, TH, 1, col));
-            const float2 htzyp = lds2(at(S, TH + 2, 1, col));
-            const float2 htyzp = make_float2(hty.y, *at(S, TH + 1, 0, col + 2));
+            const float2 hty = lds2(at(S, TH + 1, 0, hcol)), htx = lds2(at(S, TH, 0, hcol));
+            const float2 htz = lds2(at(S, TH + 2, 0, hcol));
+            const float2 htyxp = lds2(at(X, TH + 1, 0, hcol)), htxyp = lds2(at(S, TH, 1, hcol));
+            const float2 htzyp = lds2(at(S, TH + 2, 1, hcol));
+            const float2 htyzp = make_float2(hty.y, *at(S, TH + 1, 0, hcol + 2));
             float2 c1, s1, hc, hs;
             sincos2(hty, s1, c1);
 #pragma unroll
             for (int q = 0; q < NS; ++q) {
                 chg(hty, c1, s1, q, hc, hs);
-                sts2(&sm.L[LI::cy(q)][0][lcol], hc);
-                sts2(&sm.L[LI::sy(q)][0][lcol], hs);
+                sts2(lk(LI::cy(q), 0, hl), hc);
+                sts2(lk(LI::sy(q), 0, hl), hs);
             }
-            sts2(&sm.L[LI::pxy][0][lcol], sin2(sub2(sub2(add2(htx, htyxp), htxyp), hty)));
-            sts2(&sm.L[LI::pyz][0][lcol], sin2(sub2(sub2(add2(hty, htzyp), htyzp), htz)));
+            sts2(lk(LI::pxy, 0, hl), sin2(sub2(sub2(add2(htx, htyxp), htxyp), hty)));
+            sts2(lk(LI::pyz, 0, hl), sin2(sub2(sub2(add2(hty, htzyp), htyzp), htz)));
         }
         if (halo_col) {
             // z = k0-1 of row j0+tz (staged column PT_C0-1): what z = k0 reads as its z-backward data
-            const int r = tz + 1;
-            const float htx = *at(S, TH, r, PT_C0 - 1), hty = *at(S, TH + 1, r, PT_C0 - 1);
-            const float htz = *at(S, TH + 2, r, PT_C0 - 1);
-            const float htzxp = *at(X, TH + 2, r, PT_C0 - 1), htxzp = *at(S, TH, r, PT_C0);
-            const float htzyp = *at(S, TH + 2, r + 1, PT_C0 - 1), htyzp = *at(S, TH + 1, r, PT_C0);
+            const int r = hr;
+            const float htx = *at(S, TH, r, sh.c0 - 1), hty = *at(S, TH + 1, r, sh.c0 - 1);
+            const float htz = *at(S, TH + 2, r, sh.c0 - 1);
+            const float htzxp = *at(X, TH + 2, r, sh.c0 - 1), htxzp = *at(S, TH, r, sh.c0);
+            const float htzyp = *at(S, TH + 2, r + 1, sh.c0 - 1), htyzp = *at(S, TH + 1, r, sh.c0);
             float s1, c1;
             Trig<float>::sincos(htz, &s1, &c1);
 #pragma unroll
             for (int q = 0; q < NS; ++q) {
                 float hc, hs;
                 charged<float>(htz, c1, s1, ch, q, hc, hs);
-                sm.L[LI::cz(q)][r][PT_LC0 - 1] = hc;
-                sm.L[LI::sz(q)][r][PT_LC0 - 1] = hs;
+                *lk(LI::cz(q), r, PT_LC0 - 1) = hc;
+                *lk(LI::sz(q), r, PT_LC0 - 1) = hs;
             }
-            sm.L[LI::pxz][r][PT_LC0 - 1] = Trig<float>::sin(htx + htzxp - htxzp - htz);
-            sm.L[LI::pyz][r][PT_LC0 - 1] = Trig<float>::sin(hty + htzyp - htyzp - htz);
+            *lk(LI::pxz, r, PT_LC0 - 1) = Trig<float>::sin(htx + htzxp - htxzp - htz);
+            *lk(LI::pyz, r, PT_LC0 - 1) = Trig<float>::sin(hty + htzyp - htyzp - htz);
         }
         __syncthreads();
 
@@ -487,9 +556,9 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
 #pragma unroll
         for (int cc = 0; cc < 2 * NS; ++cc) vxp[cc] = lds2(at(X, cc, hy, col));
         if (active) {
-            const float2 sPxy_ym = lds2(&sm.L[LI::pxy][ly - 1][lcol]), sPyz_ym = lds2(&sm.L[LI::pyz][ly - 1][lcol]);
-            const float2 sPxz_zm = make_float2(sm.L[LI::pxz][ly][lcol - 1], sPxz.x);
-            const float2 sPyz_zm = make_float2(sm.L[LI::pyz][ly][lcol - 1], sPyz.x);
+            const float2 sPxy_ym = lds2(lk(LI::pxy, ly - 1, lcol)), sPyz_ym = lds2(lk(LI::pyz, ly - 1, lcol));
+            const float2 sPxz_zm = make_float2(*lk(LI::pxz, ly, lcol - 1), sPxz.x);
+            const float2 sPyz_zm = make_float2(*lk(LI::pyz, ly, lcol - 1), sPyz.x);
 
             float2 mag[NS], npot[NS];
 #pragma unroll
@@ -515,19 +584,19 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
                 const float2 rezm = make_float2(*at(S, 2 * q, hy, col - 1), re.x);
                 const float2 imzm = make_float2(*at(S, 2 * q + 1, hy, col - 1), imv.x);
                 const float2 rexm = vm[2 * q], imxm = vm[2 * q + 1];
-                const float2 cym = lds2(&sm.L[LI::cy(q)][ly - 1][lcol]), sym = lds2(&sm.L[LI::sy(q)][ly - 1][lcol]);
+                const float2 cym = lds2(lk(LI::cy(q), ly - 1, lcol)), sym = lds2(lk(LI::sy(q), ly - 1, lcol));
                 // Moore reads its own y and z link data back from shared memory
                 // rather than holding it across the barrier (four CTAs per SM
                 // leave it 128 registers)
                 float2 cyq = cy[q], syq = sy[q], czq = cz[q], szq = sz[q];
                 if constexpr (NS == 2) {
-                    cyq = lds2(&sm.L[LI::cy(q)][ly][lcol]);
-                    syq = lds2(&sm.L[LI::sy(q)][ly][lcol]);
-                    czq = lds2(&sm.L[LI::cz(q)][ly][lcol]);
-                    szq = lds2(&sm.L[LI::sz(q)][ly][lcol]);
+                    cyq = lds2(lk(LI::cy(q), ly, lcol));
+                    syq = lds2(lk(LI::sy(q), ly, lcol));
+                    czq = lds2(lk(LI::cz(q), ly, lcol));
+                    szq = lds2(lk(LI::sz(q), ly, lcol));
                 }
-                const float2 czm = make_float2(sm.L[LI::cz(q)][ly][lcol - 1], czq.x);
-                const float2 szm = make_float2(sm.L[LI::sz(q)][ly][lcol - 1], szq.x);
+                const float2 czm = make_float2(*lk(LI::cz(q), ly, lcol - 1), czq.x);
+                const float2 szm = make_float2(*lk(LI::sz(q), ly, lcol - 1), szq.x);
                 const float2 m2re = mul2(p2(-2.f), re), m2im = mul2(p2(-2.f), imv);
                 // covariant Laplacian: c = +1 for the real part, -1 for the imaginary part
                 float2 lx = fma2(cx[q], rexp, fma2(sx[q], imxp, fma2(cxm[q], rexm, fma2(neg2(sxm[q]), imxm, m2re))));
@@ -601,7 +670,7 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
                     fc = fma2(onem2, p2(c.inv_gyz2), fma2(onem1, p2(c.inv_gxz2), mul2(onem0, p2(c.inv_gxy2))));
                 }
                 if (c.g != 0) {
-                    const float2 divPast = *reinterpret_cast<const float2*>(reinterpret_cast<const float*>(d.divbuf) + s);
+                    const float2 divPast = ld(reinterpret_cast<const float*>(d.divbuf) + s);
                     gauss = fma2(p2(-c.twog), gsum, mul2(mul2(sub2(divNow, divPast), p2(c.inv_dt)), p2(c.inv_g)));
                     if (d.energy_form != LAT_ENERGY_MPI) {
                         const float2 a0 = mul2(sub2(tx, qv[TH]), p2(c.inv_gdtdx));
@@ -630,18 +699,18 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
                     ed = fma2(mul2(p2(c.halfLambda12e), m1), m2, ed);
                 }
                 const float scale = d.energy_form == LAT_ENERGY_MPI ? c.dxdydz : c.dV;
-                e_acc += (double)(ed.x * scale) + (double)(ed.y * scale);
-                g_acc += (double)fabsf(gauss.x) + (double)fabsf(gauss.y);
+                e_acc += (double)(ed.x * scale) + (second ? (double)(ed.y * scale) : 0.0);
+                g_acc += (double)fabsf(gauss.x) + (second ? (double)fabsf(gauss.y) : 0.0);
             }
-            if (d.store_div) *reinterpret_cast<float2*>(reinterpret_cast<float*>(d.divbuf) + s) = divNow;
+            if (d.store_div) store(reinterpret_cast<float*>(d.divbuf) + s, divNow);
             if (d.write) {
                 const float2 dt2 = p2(c.dt2);
 #pragma unroll
                 for (int cc = 0; cc < 2 * NS; ++cc)
-                    *reinterpret_cast<float2*>(f.past[cc] + s) = fma2(dt2, acc[cc], add2(v[cc], sub2(v[cc], qv[cc])));
-                *reinterpret_cast<float2*>(f.past[TH] + s) = fma2(dt2, ttx, add2(tx, sub2(tx, qv[TH])));
-                *reinterpret_cast<float2*>(f.past[TH + 1] + s) = fma2(dt2, tty, add2(tyv, sub2(tyv, qv[TH + 1])));
-                *reinterpret_cast<float2*>(f.past[TH + 2] + s) = fma2(dt2, ttz, add2(tzv, sub2(tzv, qv[TH + 2])));
+                    store(f.past[cc] + s, fma2(dt2, acc[cc], add2(v[cc], sub2(v[cc], qv[cc]))));
+                store(f.past[TH] + s, fma2(dt2, ttx, add2(tx, sub2(tx, qv[TH]))));
+                store(f.past[TH + 1] + s, fma2(dt2, tty, add2(tyv, sub2(tyv, qv[TH + 1]))));
+                store(f.past[TH + 2] + s, fma2(dt2, ttz, add2(tzv, sub2(tzv, qv[TH + 2]))));
             }
         }
         // carry: x-backward data of the next plane, and its own values read here as x-forward neighbours
@@ -672,25 +741,44 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const Geom& g, const
     }
 }
 
-template <int NS, bool DIAG, bool Q12>
+template <int NS, bool DIAG, bool Q12, class SH>
 __global__ void __launch_bounds__(PT_THREADS, 4)
-pair_step_kernel(const Geom g, const Fields<float, 2 * NS + 3> f, const PairCoef c, const Charges<float> ch,
+pair_step_kernel(const Geom g, const SH sh, const Fields<float, 2 * NS + 3> f, const PairCoef c, const Charges<float> ch,
                  const DiagOut d, const int chunk)
 {
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PairSmem<NS>& sm = *reinterpret_cast<PairSmem<NS>*>(smem_raw);
     const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
-    pair_tile<NS, DIAG, NS == 1, Q12>(sm, g, f, c, ch, d, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, chunk,
-                        DIAG ? d.partials + 2 * blk : nullptr);
+    pair_tile<NS, DIAG, NS == 1, Q12>(sm, sh, g, f, c, ch, d, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, chunk,
+                                      DIAG ? d.partials + 2 * blk : nullptr);
 }
 
-// Launch the pair step if the layout allows it; returns cudaErrorNotSupported
-// (nothing launched) otherwise.
+// Whether a Moore lattice takes the pair step, on 64x4 tiles: 16-byte staging,
+// and z-tiles at least 90 % full; elsewhere the tiled step runs.  (The other
+// tiles are 10-25 % faster for Moore too, 96^3 21 us instead of 29, but round
+// differently from the tiled step, and at strong coupling, g >= 1.2 at spacing
+// 0.5 without friction, the two-scalar model grows a last-bit difference to
+// 1e-3 within 120 steps.)
+inline bool pair_moore_ok(const Geom& g, const Fields<float, 7>& f)
+{
+    const int tiles = (g.nz + 63) / 64;
+    return tiled_vec_ok<float, 7>(g, f) && 10 * g.nz >= 9 * 64 * tiles;
+}
+
+// Pairs per row of an Abelian-Higgs lattice's tile: 32 or 16, whichever leaves
+// fewer lanes idle; 32 for equal counts.
+inline int pair_tz2(const Geom& g)
+{
+    const int z = g.hiz - g.loz, y = g.hiy - g.loy;
+    const int64_t wide = (int64_t)((z + 63) / 64) * ((y + 3) / 4), narrow = (int64_t)((z + 31) / 32) * ((y + 7) / 8);
+    return wide <= narrow ? 32 : 16;
+}
+
+// Launch the pair step (Moore: where pair_moore_ok).  *blocks receives the CTAs (diagnostic partials).
 template <int NS>
 cudaError_t launch_pair_t(const Geom& g, const Fields<float, 2 * NS + 3>& f, const StepCoef& c64, const DiagOut& d,
-                          bool diag, int chunk, cudaStream_t st)
+                          bool diag, int chunk, cudaStream_t st, int* blocks)
 {
-    if (!pair_ok(g, f)) return cudaErrorNotSupported;
     Charges<float> ch;
     if (NS == 1) {
         ch.q[0] = 1;
@@ -706,20 +794,36 @@ cudaError_t launch_pair_t(const Geom& g, const Fields<float, 2 * NS + 3>& f, con
     ch.charge_current = d.charge_current;
     const PairCoef c = pair_coef(c64);
     const size_t smem = sizeof(PairSmem<NS>);
-    const dim3 grid = pair_grid(g, chunk);
     const dim3 block(PT_TZ, PT_Y);
     // Moore with charges 1 and 2 (the benchmark's) takes e^{i q theta} in closed form
     const bool q12 = NS == 2 && ch.qpow[0] == 1 && ch.qpow[1] == 2;
-    auto go = [&](auto kernel) {
+    auto go = [&](auto kernel, auto sh, dim3 grid) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kernel<<<grid, block, smem, st>>>(g, f, c, ch, d, chunk);
+        kernel<<<grid, block, smem, st>>>(g, sh, f, c, ch, d, chunk);
+        *blocks = (int)(grid.x * grid.y * grid.z);
     };
-    if (q12) {
-        if (diag) go(pair_step_kernel<NS, true, NS == 2>);
-        else go(pair_step_kernel<NS, false, NS == 2>);
+    auto pick = [&](auto sh, dim3 grid) {
+        using SH = decltype(sh);
+        if (q12) {
+            if (diag) go(pair_step_kernel<NS, true, NS == 2, SH>, sh, grid);
+            else go(pair_step_kernel<NS, false, NS == 2, SH>, sh, grid);
+        } else {
+            if (diag) go(pair_step_kernel<NS, true, false, SH>, sh, grid);
+            else go(pair_step_kernel<NS, false, false, SH>, sh, grid);
+        }
+    };
+    if constexpr (NS == 2) {
+        pick(PairShape<32, true>{}, pair_shape_grid(g, 32, chunk));
     } else {
-        if (diag) go(pair_step_kernel<NS, true, false>);
-        else go(pair_step_kernel<NS, false, false>);
+        const int tz2 = pair_tz2(g);
+        const dim3 grid = pair_shape_grid(g, tz2, chunk);
+        if (tiled_vec_ok(g, f)) {
+            if (tz2 == 32) pick(PairShape<32, true>{}, grid);
+            else pick(PairShape<16, true>{}, grid);
+        } else {
+            if (tz2 == 32) pick(PairShape<32, false>{}, grid);
+            else pick(PairShape<16, false>{}, grid);
+        }
     }
     return cudaGetLastError();
 }

@@ -44,23 +44,14 @@ namespace lat {
 
 // Time of an x-marching FP32 step, in arbitrary units, with `ctas` CTAs of
 // `chunk` planes each: a CTA's prologue costs about 1.7 planes; a plane takes
-// 1.05 while an SM has one or two CTAs and 0.575 for each of its CTAs above
-// (the SM's throughput).  Fitted to chunks of 1..128 on 32^3 .. 384^3, both
-// models; the chunk it picks is
-// within 5 % of the best one measured, where the rule before it (the largest
-// chunk with four CTAs per SM) lost 5 % at 384^3 (645 -> 614 us), 14 % at
-// 201x199x203 (169 -> 146) and 28 % at 40x36x33 (8.7 -> 6.3).
+// 0.4, and 0.41 for each of the SM's CTAs (latency and throughput).  Fitted to
+// chunks of 1..128 on 32^3 .. 384^3, both models; the chunk it picks is within
+// 5 % of the best one measured, where the rule before it (the largest chunk
+// with four CTAs per SM) lost 5 % at 384^3 (645 -> 614 us), 14 % at 201x199x203
+// (169 -> 146) and 28 % at 40x36x33 (8.7 -> 6.3).
 static double march_cost(int chunk, double ctas)
 {
-    const double per_sm = std::ceil(ctas / 152);
-    return (chunk + 1.7) * std::max(1.05, 0.575 * per_sm);
-}
-
-int64_t march_tiles(const Geom& g)
-{
-    const int64_t y = g.hiy - g.loy, z = g.hiz - g.loz;
-    const bool pair = z == g.nz && z % 4 == 0 && 10 * z >= 9 * 64 * ((z + 63) / 64);   // as pair_ok
-    return pair ? ((z + 63) / 64) * ((y + 3) / 4) : ((z + 31) / 32) * ((y + 7) / 8);
+    return (chunk + 1.7) * (0.4 + 0.41 * std::ceil(ctas / 152));
 }
 
 // Default chunk for a handle: the tuned value of its shape, else the cheapest
@@ -73,7 +64,7 @@ int default_chunk(const lat_params& p)
         if (it != g_tune.end()) return it->second.chunk;
     }
     const Geom g = make_geom(p);
-    const double tiles = (double)march_tiles(g);
+    const double tiles = (double)march_tiles(g, p.model == LAT_MODEL_MOORE);
     const int x = g.hix - g.lox;
     int best = 1;
     double cost = 1e300;
