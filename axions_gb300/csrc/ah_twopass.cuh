@@ -17,6 +17,8 @@
 // ulp per operation.
 #pragma once
 
+#include <type_traits>
+
 #include "site_common.cuh"
 
 namespace lat {
@@ -162,7 +164,18 @@ struct AhSite {
 
 // The update of one site (mpi_evolution.cpp:412-501) and its diagnostics: new
 // values to `next` (phi, then theta), div(theta) to divNow.
-template <bool STRICT, bool DIAG, bool RECIP>
+// cm*x + sm*y, out of line: where a compiler would predicate it, it costs the
+// FP64 pipe on every path
+static __device__ __noinline__ double mul_add_rare(double cm, double x, double sm, double y)
+{
+    return __dadd_rn(__dmul_rn(cm, x), __dmul_rn(sm, y));
+}
+
+// How the strict update takes its products: on the FP64 pipe, or by integer
+// instructions, with sines that may be zero or not (about 4 % slower if so)
+enum { FP_PRODUCTS, INT_PRODUCTS, INT_ZERO_SINES };
+
+template <bool STRICT, bool DIAG, bool RECIP, int INT>
 __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, const DiagOut& d, double (&next)[5],
                                         double& divNow, double& e_site, double& g_site)
 {
@@ -180,21 +193,73 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
 
     double tt0 = 0, tt1 = 0, curx, cury, curz;
     if constexpr (STRICT) {
-        // covariant Laplacian (mpi_evolution.cpp:418-428), c = +1 then c = -1
-        tt0 = lap_minus<RECIP>(minus_twice(cx * p0xp + sx * p1xp, p0) + cxm * p0xm - sxm_ * p1xm,
-                               minus_twice(cy * p0yp + sy * p1yp, p0) + cym * p0ym - sym * p1ym,
-                               minus_twice(cz * p0zp + sz * p1zp, p0) + czm * p0zm - szm_ * p1zm, pot * p0, c);
-        tt1 = lap_minus<RECIP>(minus_twice(cx * p1xp - sx * p0xp, p1) + cxm * p1xm + sxm_ * p0xm,
-                               minus_twice(cy * p1yp - sy * p0yp, p1) + cym * p1ym + sym * p0ym,
-                               minus_twice(cz * p1zp - sz * p0zp, p1) + czm * p1zm + szm_ * p0zm, pot * p1, c);
+        // INT: the products of the covariant Laplacian (mpi_evolution.cpp:418-428)
+        // and of the current go through the integer pipes, where every factor
+        // allows it: 42 of the update's 139 FP64 instructions.  With general
+        // spacings the quotients take the integer pipes already, and the
+        // current's outer products stay (128^3: 612 us a step, 635 without).
+        // The remaining products, moved as well, gave nothing.
+        const double val[20] = {p0,   p1,   p0xp, p1xp, p0yp, p1yp, p0zp, p1zp, p0xm, p1xm,
+                                p0ym, p1ym, p0zm, p1zm, cx,   cy,   cz,   cxm,  cym,  czm};
+        double br[6];
+        const double sines[6] = {sx, sy, sz, sxm_, sym, szm_};
+        unsigned range = INT != FP_PRODUCTS ? 0 : kProductSpan;
+        if constexpr (INT != FP_PRODUCTS) {
+#pragma unroll
+            for (int k = 0; k < 20; ++k) range = max(range, product_range(val[k]));
+#pragma unroll
+            for (int k = 0; k < 6; ++k)
+                range = max(range, INT == INT_ZERO_SINES ? product_range_or_zero(sines[k]) : product_range(sines[k]));
+        }
+        // times: a product; sine: one whose first factor is a sine
+        auto terms = [&](auto times, auto sine) {
+            // c = +1 then c = -1
+            tt0 = lap_minus<RECIP>(minus_twice(times(cx, p0xp) + sine(sx, p1xp), p0) + times(cxm, p0xm) - sine(sxm_, p1xm),
+                                   minus_twice(times(cy, p0yp) + sine(sy, p1yp), p0) + times(cym, p0ym) - sine(sym, p1ym),
+                                   minus_twice(times(cz, p0zp) + sine(sz, p1zp), p0) + times(czm, p0zm) - sine(szm_, p1zm),
+                                   pot * p0, c);
+            tt1 = lap_minus<RECIP>(minus_twice(times(cx, p1xp) - sine(sx, p0xp), p1) + times(cxm, p1xm) + sine(sxm_, p0xm),
+                                   minus_twice(times(cy, p1yp) - sine(sy, p0yp), p1) + times(cym, p1ym) + sine(sym, p0ym),
+                                   minus_twice(times(cz, p1zp) - sine(sz, p0zp), p1) + times(czm, p1zm) + sine(szm_, p0zm),
+                                   pot * p1, c);
+            // brackets of the gauge current (mpi_evolution.cpp:459-466)
+            br[0] = times(p1, p0xp) - times(p0, p1xp), br[1] = times(p0, p0xp) + times(p1, p1xp);
+            br[2] = times(p1, p0yp) - times(p0, p1yp), br[3] = times(p0, p0yp) + times(p1, p1yp);
+            br[4] = times(p1, p0zp) - times(p0, p1zp), br[5] = times(p0, p0zp) + times(p1, p1zp);
+        };
+        auto rounded = [](double x, double y) { return __dmul_rn(x, y); };
+        bool in = INT != FP_PRODUCTS && range < kProductSpan;
+        if (in) {
+            auto sine = [](double x, double y) {
+                if constexpr (INT == INT_ZERO_SINES) return mul_or_zero(x, y);
+                else return mul(factor(x), factor(y));
+            };
+            terms([](double x, double y) { return mul(factor(x), factor(y)); }, sine);
+            range = 0;
+#pragma unroll
+            for (int k = 0; k < 6; ++k) range = max(range, product_range(br[k]));
+            in = RECIP && range < kProductSpan;
+            if (in) {
+                curx = mul(factor(cx), factor(br[0])) + sine(sx, br[1]);
+                cury = mul(factor(cy), factor(br[2])) + sine(sy, br[3]);
+                curz = mul(factor(cz), factor(br[4])) + sine(sz, br[5]);
+            }
+        } else {
+            terms(rounded, rounded);
+        }
+        if (!in) {
+            auto current = [](double cm, double x, double sm, double y) {
+                if constexpr (INT != FP_PRODUCTS && RECIP) return mul_add_rare(cm, x, sm, y);
+                else return __dadd_rn(__dmul_rn(cm, x), __dmul_rn(sm, y));
+            };
+            curx = current(cx, br[0], sx, br[1]);
+            cury = current(cy, br[2], sy, br[3]);
+            curz = current(cz, br[4], sz, br[5]);
+        }
         if (nonzero(c.fric)) {
             tt0 = tt0 - c.fric * cdiv(p0 - q0, c.dt, c.inv_dt);
             tt1 = tt1 - c.fric * cdiv(p1 - q1, c.dt, c.inv_dt);
         }
-        // gauge current (mpi_evolution.cpp:459-466)
-        curx = cx * (p1 * p0xp - p0 * p1xp) + sx * (p0 * p0xp + p1 * p1xp);
-        cury = cy * (p1 * p0yp - p0 * p1yp) + sy * (p0 * p0yp + p1 * p1yp);
-        curz = cz * (p1 * p0zp - p0 * p1zp) + sz * (p0 * p0zp + p1 * p1zp);
     } else {
         // The same quantities with fewer FP64 instructions.  The forward
         // link-transported neighbour U_mu phi(x+mu), A = c phi0' + s phi1',
@@ -321,10 +386,22 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
     }
 }
 
-template <bool STRICT, bool DIAG, bool RECIP>
-__global__ void __launch_bounds__(BLOCK, 2) ah_update_kernel(const Geom g, const Flat r, const Fields<double, 5> f,
-                                                          const LinkSlotsC L, const StepCoef c,
-                                                          const DiagOut d)
+// Lattices whose LAT_F64 update takes its products by integer instructions: those
+// on which the FP64 pipe bounds it.  us per step with FP64 products and with
+// integer ones: 128^3 675 and 525 (diagnostic 1106 and 957; general spacings 665
+// and 563), 64^3 96 and 77, 32^3 20.7 and 18.6 (diagnostic 40.8 and 38.6).  On
+// smaller ones, with less than two warps for each scheduler, the longer chain of
+// instructions counts: 24^3 diagnostic 31.5 and 33.6, general spacings 18.6 and
+// 20.6.
+constexpr unsigned INT_PRODUCT_SITES = 32 * 32 * 32;
+
+// 128 registers: three blocks of 168 spill nothing and are no faster with plain
+// steps (128^3: 527 us against 525), slower with diagnostic ones (1009 against 957).
+constexpr int UPDATE_BLOCK = 128;   // flat_block's largest
+
+template <bool STRICT, bool DIAG, bool RECIP, int INT>
+__global__ void __launch_bounds__(UPDATE_BLOCK, 4)
+ah_update_kernel(const Geom g, const Flat r, const Fields<double, 5> f, const LinkSlotsC L, const StepCoef c, const DiagOut d)
 {
     const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
     double e_site = 0.0, g_site = 0.0;
@@ -364,7 +441,7 @@ __global__ void __launch_bounds__(BLOCK, 2) ah_update_kernel(const Geom g, const
             if (nonzero(c.g)) v.divPast = reinterpret_cast<const double*>(d.divbuf)[s];
         }
         double next[5], divNow;
-        ah_site<STRICT, DIAG, RECIP>(v, c, d, next, divNow, e_site, g_site);
+        ah_site<STRICT, DIAG, RECIP, INT>(v, c, d, next, divNow, e_site, g_site);
         if (d.store_div) reinterpret_cast<double*>(d.divbuf)[s] = divNow;
         if (d.write) {  // in-place update of the past slot
 #pragma unroll
@@ -394,13 +471,21 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
     if (e != cudaSuccess) return e;
     const Flat r = flat_region(g);
     const int grid = flat_grid(r.n), block = flat_block(r.n);
-    if (diag) {
-        if (recip) ah_update_kernel<STRICT, true, true><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
-        else ah_update_kernel<STRICT, true, false><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
-    } else {
-        if (recip) ah_update_kernel<STRICT, false, true><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
-        else ah_update_kernel<STRICT, false, false><<<grid, block, 0, st>>>(g, r, f, Lr, c, d);
+    auto go = [&](auto kernel) { kernel<<<grid, block, 0, st>>>(g, r, f, Lr, c, d); };
+    auto pick = [&](auto form) {
+        constexpr int INT = decltype(form)::value;
+        if (diag) recip ? go(ah_update_kernel<STRICT, true, true, INT>) : go(ah_update_kernel<STRICT, true, false, INT>);
+        else recip ? go(ah_update_kernel<STRICT, false, true, INT>) : go(ah_update_kernel<STRICT, false, false, INT>);
+    };
+    if constexpr (STRICT) {
+        if (r.n >= INT_PRODUCT_SITES) {
+            // the link phases vanish for good on fixed walls, and without coupling
+            if (r.n != ra.n || c.g == 0) pick(std::integral_constant<int, INT_ZERO_SINES>{});
+            else pick(std::integral_constant<int, INT_PRODUCTS>{});
+            return cudaGetLastError();
+        }
     }
+    pick(std::integral_constant<int, FP_PRODUCTS>{});
     return cudaGetLastError();
 }
 

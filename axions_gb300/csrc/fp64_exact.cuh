@@ -60,4 +60,62 @@ __device__ __forceinline__ double cdiv(double a, double b, double y)
     return __longlong_as_double((long long)(sign | (((u64)(ea - eb + 1022u - (unsigned)below) << 52) + q)));
 }
 
+// The IEEE product a * b by integer instructions, for steps that the FP64 pipe
+// bounds: the 53-bit mantissas' exact 106-bit product, rounded to nearest even.
+// A product costs the integer pipes about as long as the FP64 pipe (some 30
+// instructions), but the two run side by side.  Operands that enter several
+// products are unpacked once.  Both factors have to be in product_range,
+// [2^-510, 2^512): no zeros, subnormals, Inf or NaN, and no product that leaves
+// the normal range.
+struct Factor {
+    unsigned long long m;   // the mantissa, its leading one at bit 63
+    unsigned hi;            // the high word: sign and exponent
+};
+
+__device__ __forceinline__ Factor factor(double a)
+{
+    const unsigned long long b = (unsigned long long)__double_as_longlong(a);
+    return Factor{(b << 11) | 0x8000000000000000ull, (unsigned)(b >> 32)};
+}
+
+// 0 .. kProductSpan-1 exactly for a double in product_range; the maximum over
+// several values tells whether all are
+constexpr unsigned kProductSpan = 1022u << 20;   // biased exponents 513 .. 1534
+__device__ __forceinline__ unsigned product_range(double a)
+{
+    return ((unsigned)((unsigned long long)__double_as_longlong(a) >> 32) & 0x7fffffffu) - (513u << 20);
+}
+
+__device__ __forceinline__ double mul(const Factor& a, const Factor& b)
+{
+    typedef unsigned long long u64;
+    const unsigned ah = (unsigned)(a.m >> 32), al = (unsigned)a.m, bh = (unsigned)(b.m >> 32), bl = (unsigned)b.m;
+    const u64 t0 = (u64)al * bl, t1 = (u64)ah * bl + (t0 >> 32), t2 = (u64)al * bh + (unsigned)t1;
+    u64 h = (u64)ah * bh + (t1 >> 32) + (t2 >> 32);   // in [2^62, 2^64); below it (t2, t0) low words
+    // The product's lowest 22 bits are zero, so the top bit of the low half and
+    // whether anything is left of it are in t2's low word and t0's.
+    const int below = (int)(h >> 63) ^ 1;             // the product is under 2: one bit more
+    const unsigned l2 = (unsigned)t2;
+    h = (h << below) | (below ? l2 >> 31 : 0u);
+    const unsigned rest = ((unsigned)h & 0x7ffu) | (((l2 << below) | (unsigned)t0) != 0 ? 1u : 0u);
+    u64 n = h >> 11;
+    // the bits below the last one: above half, or half and the last one odd
+    n += (rest + ((unsigned)n & 1u)) > 0x400u ? 1 : 0;
+    const unsigned e = ((a.hi & 0x7ff00000u) + (b.hi & 0x7ff00000u)) - ((1023u + (unsigned)below) << 20);
+    return __longlong_as_double((long long)(n + ((u64)(e + ((a.hi ^ b.hi) & 0x80000000u)) << 32)));
+}
+
+// The same where a may also be zero (the sine of a vanishing angle)
+__device__ __forceinline__ unsigned product_range_or_zero(double a)
+{
+    return (__double_as_longlong(a) << 1) == 0 ? 0 : product_range(a);
+}
+__device__ __forceinline__ double mul_or_zero(double a, double b)
+{
+    const unsigned long long sign =
+        (unsigned long long)(__double_as_longlong(a) ^ __double_as_longlong(b)) & 0x8000000000000000ull;
+    const double r = mul(factor(a), factor(b));
+    return (__double_as_longlong(a) << 1) == 0 ? __longlong_as_double((long long)sign) : r;
+}
+
 }  // namespace lat

@@ -72,13 +72,13 @@ inline Flat flat_region(const Geom& g)
     return r;
 }
 
-// Threads per block of the flat kernels: 256, and fewer where 256 would leave
+// Threads per block of the flat kernels: 128, and fewer where 128 would leave
 // fewer than four blocks for each of the 152 SMs (a warp keeps a quarter of an
 // SM's FP64 pipe busy by itself, so a small lattice is as fast as its warps are
 // spread: caller-owned 24^3 steps took 25.6 us with 256-thread blocks).
 inline int flat_block(unsigned n)
 {
-    int b = 256;
+    int b = 128;
     while (b > 32 && (n + b - 1) / b < 4 * 152) b /= 2;
     return b;
 }
