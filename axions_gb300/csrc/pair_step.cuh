@@ -746,6 +746,7 @@ __global__ void __launch_bounds__(PT_THREADS, 4)
 pair_step_kernel(const Geom g, const SH sh, const Fields<float, 2 * NS + 3> f, const PairCoef c, const Charges<float> ch,
                  const DiagOut d, const int chunk)
 {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     PairSmem<NS>& sm = *reinterpret_cast<PairSmem<NS>*>(smem_raw);
     const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
@@ -797,9 +798,10 @@ cudaError_t launch_pair_t(const Geom& g, const Fields<float, 2 * NS + 3>& f, con
     const dim3 block(PT_TZ, PT_Y);
     // Moore with charges 1 and 2 (the benchmark's) takes e^{i q theta} in closed form
     const bool q12 = NS == 2 && ch.qpow[0] == 1 && ch.qpow[1] == 2;
+    cudaError_t err = cudaSuccess;
     auto go = [&](auto kernel, auto sh, dim3 grid) {
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-        kernel<<<grid, block, smem, st>>>(g, sh, f, c, ch, d, chunk);
+        err = launch_chained(kernel, grid, block, smem, st, g, sh, f, c, ch, d, chunk);
         *blocks = (int)(grid.x * grid.y * grid.z);
     };
     auto pick = [&](auto sh, dim3 grid) {
@@ -825,7 +827,7 @@ cudaError_t launch_pair_t(const Geom& g, const Fields<float, 2 * NS + 3>& f, con
             else pick(PairShape<16, false>{}, grid);
         }
     }
-    return cudaGetLastError();
+    return err;
 }
 
 }  // namespace lat

@@ -513,6 +513,7 @@ __global__ void __launch_bounds__(TT_THREADS, NS == 1 ? 4 : 3)
 tiled_step_kernel(const Geom g, const Fields<T, 2 * NS + 3> f, const StepCoefT<T> c, const Charges<T> ch,
                   const DiagOut d, const int chunk, const int vec)
 {
+    chain_wait();
     extern __shared__ __align__(16) unsigned char smem_raw[];
     TiledSmem<T, NS>& sm = *reinterpret_cast<TiledSmem<T, NS>*>(smem_raw);
     const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
@@ -557,9 +558,8 @@ cudaError_t launch_tiled_t(const Geom& g, const Fields<T, 2 * NS + 3>& f, const 
     const dim3 grid = tiled_grid(g, chunk);
     const dim3 block(TT_Z, TT_Y);
     const int vec = allow_vec && tiled_vec_ok(g, f) ? 1 : 0;
-    if (diag) tiled_step_kernel<T, NS, true><<<grid, block, smem, st>>>(g, f, c, ch, d, chunk, vec);
-    else tiled_step_kernel<T, NS, false><<<grid, block, smem, st>>>(g, f, c, ch, d, chunk, vec);
-    return cudaGetLastError();
+    return launch_chained(diag ? tiled_step_kernel<T, NS, true> : tiled_step_kernel<T, NS, false>, grid, block, smem, st, g, f,
+                          c, ch, d, chunk, vec);
 }
 
 }  // namespace lat
