@@ -73,14 +73,16 @@ inline Flat flat_region(const Geom& g)
     return r;
 }
 
-// A kernel of a chain of steps starts while its predecessor in the stream drains:
-// launch_chained lets its blocks be placed from when all the predecessor's have
-// been, chain_wait, the kernel's first statement, holds them until the
-// predecessor is complete and its writes are visible.  It takes the launch and
-// the block set-up, 1.5 to 3 us, off each step: 200 FP32 steps of 40 x 36 x 33
-// 1.57 to 1.27 ms, a caller's four steps of 24^3 70 to 55 us, 200 Moore FP32
-// steps of 192^3 34.0 to 32.9 ms.  A kernel launched this way
-// reaches chain_wait before any access to global memory.
+// A kernel of a chain of steps starts as its predecessor in the stream ends:
+// launch_chained lets its blocks be placed once all the predecessor's have
+// exited, without waiting for the grid's completion and the next launch;
+// chain_wait, the kernel's first statement, holds them until the predecessor is
+// complete and its writes are visible.  us per step, plain launches and these:
+// FP32 32^3 4.3 and 2.6, 64^3 9.0 and 6.9, 256^3 191.9 and 189.1; FP64 24^3 16.4
+// and 11.6, 48^3 39.0 and 34.7.  (Blocks placed earlier, while the predecessor
+// runs, crowd the SMs with the most free room, several kernels deep: FP64 32^3
+// 27.4, FP32 64^3 9.7.)  A kernel launched this way reaches chain_wait before any
+// access to global memory.
 template <class... P, class... A>
 cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st, A&&... args)
 {
@@ -99,7 +101,6 @@ cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t s
 }
 __device__ __forceinline__ void chain_wait()
 {
-    asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
     asm volatile("griddepcontrol.wait;" ::: "memory");
 }
 
