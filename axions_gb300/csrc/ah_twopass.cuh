@@ -19,6 +19,7 @@
 
 #include <type_traits>
 
+#include "fixed_point.cuh"
 #include "site_common.cuh"
 
 namespace lat {
@@ -100,7 +101,8 @@ __device__ __forceinline__ double twice_minus(double x, double y) { return __fma
 // t - 2*x
 __device__ __forceinline__ double minus_twice(double t, double x) { return __fma_rn(-2.0, x, t); }
 
-template <bool STRICT, bool DIAG>
+// FIX: the cosines and sines of the links as fixed-point data (fixed_point.cuh)
+template <bool STRICT, bool DIAG, bool FIX>
 __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Flat r, const double* __restrict__ TX,
                                                          const double* __restrict__ TY,
                                                          const double* __restrict__ TZ, const LinkSlots L)
@@ -115,16 +117,17 @@ __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Fla
     const double tyxp = TY[s + n.xp], tzxp = TZ[s + n.xp];
     const double txyp = TX[s + n.yp], tzyp = TZ[s + n.yp];
     const double txzp = TX[s + n.zp], tyzp = TY[s + n.zp];
+    auto link = [](double v) { return FIX ? __longlong_as_double(fix::link_of(v)) : v; };
     double sv, cv;
     dsincos(tx, &sv, &cv);
-    L.p[L_CX][s] = cv;
-    L.p[L_SX][s] = sv;
+    L.p[L_CX][s] = link(cv);
+    L.p[L_SX][s] = link(sv);
     dsincos(ty, &sv, &cv);
-    L.p[L_CY][s] = cv;
-    L.p[L_SY][s] = sv;
+    L.p[L_CY][s] = link(cv);
+    L.p[L_SY][s] = link(sv);
     dsincos(tz, &sv, &cv);
-    L.p[L_CZ][s] = cv;
-    L.p[L_SZ][s] = sv;
+    L.p[L_CZ][s] = link(cv);
+    L.p[L_SZ][s] = link(sv);
     // plaquette angles, summed in the reference's order (mpi_evolution.cpp:471-487)
     const double Pxy = tx + tyxp - txyp - ty;
     const double Pxz = tx + tzxp - txzp - tz;
@@ -173,8 +176,10 @@ static __device__ __noinline__ double mul_add_rare(double cm, double x, double s
 }
 
 // How the strict update takes its products: on the FP64 pipe, or by integer
-// instructions, with sines that may be zero or not (about 4 % slower if so)
-enum { FP_PRODUCTS, INT_PRODUCTS, INT_ZERO_SINES };
+// instructions, with sines that may be zero or not (about 4 % slower if so).
+// FIXED_POINT: the fused update of equal spacings, its Laplacian and current by
+// fixed_point.cuh from link data in that form.
+enum { FP_PRODUCTS, INT_PRODUCTS, INT_ZERO_SINES, FIXED_POINT };
 
 template <bool STRICT, bool DIAG, bool RECIP, int INT>
 __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, const DiagOut& d, double (&next)[5],
@@ -267,24 +272,45 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
         // B = c phi1' - s phi0', enters both the Laplacian and the current:
         // j_mu = c (phi1 phi0' - phi0 phi1') + s (phi0 phi0' + phi1 phi1')
         //      = phi1 A - phi0 B.
-        const double Ax = fma(sx, p1xp, cx * p0xp), Bx = fma(-sx, p0xp, cx * p1xp);
-        const double Ay = fma(sy, p1yp, cy * p0yp), By = fma(-sy, p0yp, cy * p1yp);
-        const double Az = fma(sz, p1zp, cz * p0zp), Bz = fma(-sz, p0zp, cz * p1zp);
-        const double x0 = fma(-sxm_, p1xm, fma(cxm, p0xm, Ax)), x1 = fma(sxm_, p0xm, fma(cxm, p1xm, Bx));
-        const double y0 = fma(-sym, p1ym, fma(cym, p0ym, Ay)), y1 = fma(sym, p0ym, fma(cym, p1ym, By));
-        const double z0 = fma(-szm_, p1zm, fma(czm, p0zm, Az)), z1 = fma(szm_, p0zm, fma(czm, p1zm, Bz));
-        curx = fma(p1, Ax, -p0 * Bx);
-        cury = fma(p1, Ay, -p0 * By);
-        curz = fma(p1, Az, -p0 * Bz);
-        if (nonzero(c.iso)) {
+        // FIXED_POINT: the sums less six times the scalar come from integers.
+        double x0, x1, y0 = 0, y1 = 0, z0 = 0, z1 = 0;
+        bool done = false;
+        if constexpr (INT == FIXED_POINT) {
+            auto q = [](double v) { return (int64_t)__double_as_longlong(v); };
+            const int64_t cs[3] = {q(cx), q(cy), q(cz)}, sn[3] = {q(sx), q(sy), q(sz)};
+            const int64_t csm[3] = {q(cxm), q(cym), q(czm)}, snm[3] = {q(sxm_), q(sym), q(szm_)};
+            double u[2], j[3];
+            done = fix::scalar_terms({p0, p1}, {{p0xp, p1xp}, {p0yp, p1yp}, {p0zp, p1zp}},
+                                     {{p0xm, p1xm}, {p0ym, p1ym}, {p0zm, p1zm}}, cs, sn, csm, snm, u, j);
+            x0 = u[0], x1 = u[1], curx = j[0], cury = j[1], curz = j[2];
+        }
+        if (!done) {
+            auto link = [](double v) { return INT == FIXED_POINT ? fix::link_value(__double_as_longlong(v)) : v; };
+            auto direction = [&](double cp, double sp, double cm, double sm, double ap, double bp, double am, double bm,
+                                 double& a, double& b, double& cur) {
+                const double A = fma(sp, bp, cp * ap), B = fma(-sp, ap, cp * bp);
+                a = fma(-sm, bm, fma(cm, am, A)), b = fma(sm, am, fma(cm, bm, B));
+                cur = fma(p1, A, -p0 * B);
+            };
+            direction(link(cx), link(sx), link(cxm), link(sxm_), p0xp, p1xp, p0xm, p1xm, x0, x1, curx);
+            direction(link(cy), link(sy), link(cym), link(sym), p0yp, p1yp, p0ym, p1ym, y0, y1, cury);
+            direction(link(cz), link(sz), link(czm), link(szm_), p0zp, p1zp, p0zm, p1zm, z0, z1, curz);
+            if constexpr (INT == FIXED_POINT) {
+                x0 = fma(-6.0, p0, x0 + y0 + z0);
+                x1 = fma(-6.0, p1, x1 + y1 + z1);
+            }
+        }
+        if (INT == FIXED_POINT || nonzero(c.iso)) {
             // Equal spacings: every term of an update carries its factor dt^2
             // times a constant from the host and is added to the difference
             // of the two levels, which is small and exact, before that is
-            // added to the level: 71 FP64 instructions a site (74 with the
+            // added to the level: 71 FP64 instructions a site, 33 with FIXED_POINT (74 with the
             // acceleration formed first) and one rounding of the level's size
             // instead of two.
             const double ps = c.kPot * (phiMagSqr - c.etaSq);
-            const double u0 = fma(-ps, p0, fma(-6.0, p0, x0 + y0 + z0)), u1 = fma(-ps, p1, fma(-6.0, p1, x1 + y1 + z1));
+            const double s0 = INT == FIXED_POINT ? x0 : fma(-6.0, p0, x0 + y0 + z0);
+            const double s1 = INT == FIXED_POINT ? x1 : fma(-6.0, p1, x1 + y1 + z1);
+            const double u0 = fma(-ps, p0, s0), u1 = fma(-ps, p1, s1);
             double d0 = p0 - q0, d1 = p1 - q1, dx = tx - qx, dy = ty - qy, dz = tz - qz;
             if (nonzero(c.fric)) {
                 d0 = fma(-c.kFric, d0, d0);
@@ -307,7 +333,7 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
         }
     }
 
-    if (STRICT || !nonzero(c.iso)) {
+    if (STRICT || (INT != FIXED_POINT && !nonzero(c.iso))) {
         if constexpr (!STRICT) {
             if (nonzero(c.fric)) {
                 tt0 = fma(-c.fric_dt, p0 - q0, tt0);
@@ -387,14 +413,17 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
     }
 }
 
-// Lattices whose LAT_F64 update takes its products by integer instructions: those
-// on which the FP64 pipe bounds it.  us per step with FP64 products and with
+// Lattices whose update moves FP64 work to integer instructions: those on which
+// the FP64 pipe bounds it.  LAT_F64, us per step with FP64 products and with
 // integer ones: 128^3 675 and 525 (diagnostic 1106 and 957; general spacings 665
 // and 563), 64^3 96 and 77, 32^3 20.7 and 18.6 (diagnostic 40.8 and 38.6).  On
 // smaller ones, with less than two warps for each scheduler, the longer chain of
 // instructions counts: 24^3 diagnostic 31.5 and 33.6, general spacings 18.6 and
 // 20.6.
-constexpr unsigned INT_PRODUCT_SITES = 32 * 32 * 32;
+// The fused form (equal spacings, plain steps), FP64 and fixed_point.cuh: 256^3
+// 3120 and 2129, 128^3 400 and 276, 64^3 54.5 and 40.6, 40^3 18.5 and 16.5, 32^3
+// 11.5 and 11.3, 24^3 9.0 and 9.7.
+constexpr unsigned INT_SITES = 32 * 32 * 32;
 
 // 128 registers: three blocks of 168 spill nothing and are no faster with plain
 // steps (128^3: 527 us against 525), slower with diagnostic ones (1009 against 957).
@@ -467,10 +496,12 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
     all.hiz = g.nz;
     const Flat ra = flat_region(all);
     const int la = flat_grid(ra.n), lb = flat_block(ra.n);
-    cudaError_t e = launch_chained(diag ? ah_links_kernel<STRICT, true> : ah_links_kernel<STRICT, false>, la, lb, 0, st, all,
-                                   ra, f.now[2], f.now[3], f.now[4], Lw);
-    if (e != cudaSuccess) return e;
     const Flat r = flat_region(g);
+    const bool fixed = !STRICT && !diag && c.iso != 0 && r.n >= INT_SITES;
+    cudaError_t e = launch_chained(fixed ? ah_links_kernel<STRICT, false, !STRICT>
+                                         : (diag ? ah_links_kernel<STRICT, true, false> : ah_links_kernel<STRICT, false, false>),
+                                   la, lb, 0, st, all, ra, f.now[2], f.now[3], f.now[4], Lw);
+    if (e != cudaSuccess) return e;
     const int grid = flat_grid(r.n), block = flat_block(r.n);
     auto go = [&](auto kernel) { e = launch_chained(kernel, grid, block, 0, st, g, r, f, Lr, c, d); };
     auto pick = [&](auto form) {
@@ -479,10 +510,16 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
         else recip ? go(ah_update_kernel<STRICT, false, true, INT>) : go(ah_update_kernel<STRICT, false, false, INT>);
     };
     if constexpr (STRICT) {
-        if (r.n >= INT_PRODUCT_SITES) {
+        if (r.n >= INT_SITES) {
             // the link phases vanish for good on fixed walls, and without coupling
             if (r.n != ra.n || c.g == 0) pick(std::integral_constant<int, INT_ZERO_SINES>{});
             else pick(std::integral_constant<int, INT_PRODUCTS>{});
+            return e;
+        }
+    }
+    if constexpr (!STRICT) {
+        if (fixed) {
+            go(recip ? ah_update_kernel<false, false, true, FIXED_POINT> : ah_update_kernel<false, false, false, FIXED_POINT>);
             return e;
         }
     }
