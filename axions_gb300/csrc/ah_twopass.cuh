@@ -198,6 +198,7 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
     const double pot = c.halfLambda * (phiMagSqr - c.etaSq);
 
     double tt0 = 0, tt1 = 0, curx, cury, curz;
+    double gr[3][2];   // FIXED_POINT diagnostics: phi less its transported backward neighbours
     if constexpr (STRICT) {
         // INT: the products of the covariant Laplacian (mpi_evolution.cpp:418-428)
         // and of the current go through the integer pipes, where every factor
@@ -280,21 +281,25 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
             const int64_t cs[3] = {q(cx), q(cy), q(cz)}, sn[3] = {q(sx), q(sy), q(sz)};
             const int64_t csm[3] = {q(cxm), q(cym), q(czm)}, snm[3] = {q(sxm_), q(sym), q(szm_)};
             double u[2], j[3];
-            done = fix::scalar_terms({p0, p1}, {{p0xp, p1xp}, {p0yp, p1yp}, {p0zp, p1zp}},
-                                     {{p0xm, p1xm}, {p0ym, p1ym}, {p0zm, p1zm}}, cs, sn, csm, snm, u, j);
+            done = fix::scalar_terms<DIAG>({p0, p1}, {{p0xp, p1xp}, {p0yp, p1yp}, {p0zp, p1zp}},
+                                     {{p0xm, p1xm}, {p0ym, p1ym}, {p0zm, p1zm}}, cs, sn, csm, snm, u, j, gr);
             x0 = u[0], x1 = u[1], curx = j[0], cury = j[1], curz = j[2];
         }
         if (!done) {
             auto link = [](double v) { return INT == FIXED_POINT ? fix::link_value(__double_as_longlong(v)) : v; };
             auto direction = [&](double cp, double sp, double cm, double sm, double ap, double bp, double am, double bm,
-                                 double& a, double& b, double& cur) {
+                                 double& a, double& b, double& cur, double (&g)[2]) {
                 const double A = fma(sp, bp, cp * ap), B = fma(-sp, ap, cp * bp);
                 a = fma(-sm, bm, fma(cm, am, A)), b = fma(sm, am, fma(cm, bm, B));
                 cur = fma(p1, A, -p0 * B);
+                if constexpr (INT == FIXED_POINT && DIAG) {
+                    g[0] = p0 - cm * am + sm * bm;
+                    g[1] = p1 - cm * bm - sm * am;
+                }
             };
-            direction(link(cx), link(sx), link(cxm), link(sxm_), p0xp, p1xp, p0xm, p1xm, x0, x1, curx);
-            direction(link(cy), link(sy), link(cym), link(sym), p0yp, p1yp, p0ym, p1ym, y0, y1, cury);
-            direction(link(cz), link(sz), link(czm), link(szm_), p0zp, p1zp, p0zm, p1zm, z0, z1, curz);
+            direction(link(cx), link(sx), link(cxm), link(sxm_), p0xp, p1xp, p0xm, p1xm, x0, x1, curx, gr[0]);
+            direction(link(cy), link(sy), link(cym), link(sym), p0yp, p1yp, p0ym, p1ym, y0, y1, cury, gr[1]);
+            direction(link(cz), link(sz), link(czm), link(szm_), p0zp, p1zp, p0zm, p1zm, z0, z1, curz, gr[2]);
             if constexpr (INT == FIXED_POINT) {
                 x0 = fma(-6.0, p0, x0 + y0 + z0);
                 x1 = fma(-6.0, p1, x1 + y1 + z1);
@@ -376,12 +381,17 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
         const double cPxy = v.cPxy, cPxz = v.cPxz, cPyz = v.cPyz;
         const double pt0 = cdiv(p0 - q0, c.dt, c.inv_dt);
         const double pt1 = cdiv(p1 - q1, c.dt, c.inv_dt);
-        const double px0 = sdiv<RECIP>(p0 - cxm * p0xm + sxm_ * p1xm, c.dx, c.inv_dx);
-        const double px1 = sdiv<RECIP>(p1 - cxm * p1xm - sxm_ * p0xm, c.dx, c.inv_dx);
-        const double py0 = sdiv<RECIP>(p0 - cym * p0ym + sym * p1ym, c.dy, c.inv_dy);
-        const double py1 = sdiv<RECIP>(p1 - cym * p1ym - sym * p0ym, c.dy, c.inv_dy);
-        const double pz0 = sdiv<RECIP>(p0 - czm * p0zm + szm_ * p1zm, c.dz, c.inv_dz);
-        const double pz1 = sdiv<RECIP>(p1 - czm * p1zm - szm_ * p0zm, c.dz, c.inv_dz);
+        if constexpr (INT != FIXED_POINT) {
+            gr[0][0] = p0 - cxm * p0xm + sxm_ * p1xm;
+            gr[0][1] = p1 - cxm * p1xm - sxm_ * p0xm;
+            gr[1][0] = p0 - cym * p0ym + sym * p1ym;
+            gr[1][1] = p1 - cym * p1ym - sym * p0ym;
+            gr[2][0] = p0 - czm * p0zm + szm_ * p1zm;
+            gr[2][1] = p1 - czm * p1zm - szm_ * p0zm;
+        }
+        const double px0 = sdiv<RECIP>(gr[0][0], c.dx, c.inv_dx), px1 = sdiv<RECIP>(gr[0][1], c.dx, c.inv_dx);
+        const double py0 = sdiv<RECIP>(gr[1][0], c.dy, c.inv_dy), py1 = sdiv<RECIP>(gr[1][1], c.dy, c.inv_dy);
+        const double pz0 = sdiv<RECIP>(gr[2][0], c.dz, c.inv_dz), pz1 = sdiv<RECIP>(gr[2][1], c.dz, c.inv_dz);
         double tdc = 0, fc = 0, gauss = 0;
         if (d.energy_form == LAT_ENERGY_MPI) {
             const double a0 = cdiv(tx - qx, c.dt, c.inv_dt), a1 = cdiv(ty - qy, c.dt, c.inv_dt),
@@ -420,9 +430,9 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
 // smaller ones, with less than two warps for each scheduler, the longer chain of
 // instructions counts: 24^3 diagnostic 31.5 and 33.6, general spacings 18.6 and
 // 20.6.
-// The fused form (equal spacings, plain steps), FP64 and fixed_point.cuh: 256^3
-// 3120 and 2129, 128^3 400 and 276, 64^3 54.5 and 40.6, 40^3 18.5 and 16.5, 32^3
-// 11.5 and 11.3, 24^3 9.0 and 9.7.
+// The fused form (equal spacings), FP64 and fixed_point.cuh: 256^3 3120 and 2129
+// (diagnostic 5549 and 4387), 128^3 400 and 276, 64^3 54.5 and 40.6, 40^3 18.5
+// and 16.5, 32^3 11.5 and 11.3, 24^3 9.0 and 9.7.
 constexpr unsigned INT_SITES = 32 * 32 * 32;
 
 // 128 registers: three blocks of 168 spill nothing and are no faster with plain
@@ -497,10 +507,12 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
     const Flat ra = flat_region(all);
     const int la = flat_grid(ra.n), lb = flat_block(ra.n);
     const Flat r = flat_region(g);
-    const bool fixed = !STRICT && !diag && c.iso != 0 && r.n >= INT_SITES;
-    cudaError_t e = launch_chained(fixed ? ah_links_kernel<STRICT, false, !STRICT>
-                                         : (diag ? ah_links_kernel<STRICT, true, false> : ah_links_kernel<STRICT, false, false>),
-                                   la, lb, 0, st, all, ra, f.now[2], f.now[3], f.now[4], Lw);
+    const bool fixed = !STRICT && c.iso != 0 && r.n >= INT_SITES;
+    auto links = [&](auto kernel) {
+        return launch_chained(kernel, la, lb, 0, st, all, ra, f.now[2], f.now[3], f.now[4], Lw);
+    };
+    cudaError_t e = fixed ? links(diag ? ah_links_kernel<STRICT, true, !STRICT> : ah_links_kernel<STRICT, false, !STRICT>)
+                          : links(diag ? ah_links_kernel<STRICT, true, false> : ah_links_kernel<STRICT, false, false>);
     if (e != cudaSuccess) return e;
     const int grid = flat_grid(r.n), block = flat_block(r.n);
     auto go = [&](auto kernel) { e = launch_chained(kernel, grid, block, 0, st, g, r, f, Lr, c, d); };
@@ -519,7 +531,7 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
     }
     if constexpr (!STRICT) {
         if (fixed) {
-            go(recip ? ah_update_kernel<false, false, true, FIXED_POINT> : ah_update_kernel<false, false, false, FIXED_POINT>);
+            pick(std::integral_constant<int, FIXED_POINT>{});
             return e;
         }
     }

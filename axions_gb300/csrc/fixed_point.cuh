@@ -108,10 +108,13 @@ constexpr unsigned kTopLow = 560, kTopHigh = 1500;
 // u[comp]: the sum over the directions of the transported neighbours minus six
 // times the site's scalar; cur[mu] = phi1 A_mu - phi0 B_mu, (A_mu, B_mu) the
 // transported forward neighbour.  p: the site's scalar, fwd and bwd its
-// neighbours', cs, sn, csm, snm the link data.  false: out of range.
+// neighbours', cs, sn, csm, snm the link data.  GRAD: grad[mu], the scalar less
+// its transported backward neighbour.  false: out of range.
+template <bool GRAD = false>
 __host__ __device__ inline bool scalar_terms(const double (&p)[2], const double (&fwd)[3][2], const double (&bwd)[3][2],
                                              const int64_t (&cs)[3], const int64_t (&sn)[3], const int64_t (&csm)[3],
-                                             const int64_t (&snm)[3], double (&u)[2], double (&cur)[3])
+                                             const int64_t (&snm)[3], double (&u)[2], double (&cur)[3],
+                                             double (*grad)[2] = nullptr)
 {
     unsigned top = 0;
     int low = 0;
@@ -143,8 +146,13 @@ __host__ __device__ inline bool scalar_terms(const double (&p)[2], const double 
         const int64_t a0 = fixed(bits_of(fwd[a][0]), top, 3), a1 = fixed(bits_of(fwd[a][1]), top, 3);
         const int64_t b0 = fixed(bits_of(bwd[a][0]), top, 3), b1 = fixed(bits_of(bwd[a][1]), top, 3);
         const int64_t A = hi(a0, cs[a]) + hi(a1, sn[a]), B = hi(a1, cs[a]) - hi(a0, sn[a]);
-        x0 += A + (hi(b0, csm[a]) - hi(b1, snm[a]));
-        x1 += B + (hi(b1, csm[a]) + hi(b0, snm[a]));
+        const int64_t t0 = hi(b0, csm[a]) - hi(b1, snm[a]), t1 = hi(b1, csm[a]) + hi(b0, snm[a]);
+        x0 += A + t0;
+        x1 += B + t1;
+        if constexpr (GRAD) {
+            grad[a][0] = to_double((f0 >> 2) - t0, (int)top - 1081);
+            grad[a][1] = to_double((f1 >> 2) - t1, (int)top - 1081);
+        }
         cur[a] = to_double(hi(f1, A * 4) - hi(f0, B * 4), 2 * (int)top - 2102);
     }
     u[0] = to_double(x0, (int)top - 1081);

@@ -59,3 +59,18 @@ def test_values_out_of_range(value, component):
     want, _ = _run(lattice, _params(sides, 0, 0.5, 0, 1), ic, steps=3)
     got, _ = _run(lattice, _params(sides, 0, 0.5, F64_FAST), ic, steps=3)
     assert np.array_equal(np.isfinite(got), np.isfinite(want))
+
+
+@pytest.mark.parametrize("sides,bc", [((31, 32, 33), 0), ((32, 32, 32), 0), ((41, 37, 33), 1)])
+def test_fields_do_not_depend_on_the_diagnostics(sides, bc):
+    from axions_gb300 import lattice
+    from axions_gb300.params import F64_FAST
+    p = _params(sides, bc, 0.5, F64_FAST)
+    ic = np.array(lattice.random_phase_ic(p, 5))
+    res = []
+    for every in (0, 1, 3):
+        with lattice.Lattice(p) as lat:
+            lat.set_state(ic, ic, 0)
+            lat.advance(7, diag_every=every)
+            res.append(lat.get_slots())
+    assert np.array_equal(res[0], res[1]) and np.array_equal(res[0], res[2])
