@@ -101,8 +101,7 @@ __device__ __forceinline__ double twice_minus(double x, double y) { return __fma
 // t - 2*x
 __device__ __forceinline__ double minus_twice(double t, double x) { return __fma_rn(-2.0, x, t); }
 
-// FIX: the cosines and sines of the links as fixed-point data (fixed_point.cuh)
-template <bool STRICT, bool DIAG, bool FIX>
+template <bool STRICT, bool DIAG>
 __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Flat r, const double* __restrict__ TX,
                                                          const double* __restrict__ TY,
                                                          const double* __restrict__ TZ, const LinkSlots L)
@@ -117,17 +116,16 @@ __global__ void __launch_bounds__(BLOCK) ah_links_kernel(const Geom g, const Fla
     const double tyxp = TY[s + n.xp], tzxp = TZ[s + n.xp];
     const double txyp = TX[s + n.yp], tzyp = TZ[s + n.yp];
     const double txzp = TX[s + n.zp], tyzp = TY[s + n.zp];
-    auto link = [](double v) { return FIX ? __longlong_as_double(fix::link_of(v)) : v; };
     double sv, cv;
     dsincos(tx, &sv, &cv);
-    L.p[L_CX][s] = link(cv);
-    L.p[L_SX][s] = link(sv);
+    L.p[L_CX][s] = cv;
+    L.p[L_SX][s] = sv;
     dsincos(ty, &sv, &cv);
-    L.p[L_CY][s] = link(cv);
-    L.p[L_SY][s] = link(sv);
+    L.p[L_CY][s] = cv;
+    L.p[L_SY][s] = sv;
     dsincos(tz, &sv, &cv);
-    L.p[L_CZ][s] = link(cv);
-    L.p[L_SZ][s] = link(sv);
+    L.p[L_CZ][s] = cv;
+    L.p[L_SZ][s] = sv;
     // plaquette angles, summed in the reference's order (mpi_evolution.cpp:471-487)
     const double Pxy = tx + tyxp - txyp - ty;
     const double Pxz = tx + tzxp - txzp - tz;
@@ -178,7 +176,7 @@ static __device__ __noinline__ double mul_add_rare(double cm, double x, double s
 // How the strict update takes its products: on the FP64 pipe, or by integer
 // instructions, with sines that may be zero or not (about 4 % slower if so).
 // FIXED_POINT: the fused update of equal spacings, its Laplacian and current by
-// fixed_point.cuh from link data in that form.
+// fixed_point.cuh.
 enum { FP_PRODUCTS, INT_PRODUCTS, INT_ZERO_SINES, FIXED_POINT };
 
 template <bool STRICT, bool DIAG, bool RECIP, int INT>
@@ -277,16 +275,16 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
         double x0, x1, y0 = 0, y1 = 0, z0 = 0, z1 = 0;
         bool done = false;
         if constexpr (INT == FIXED_POINT) {
-            auto q = [](double v) { return (int64_t)__double_as_longlong(v); };
-            const int64_t cs[3] = {q(cx), q(cy), q(cz)}, sn[3] = {q(sx), q(sy), q(sz)};
-            const int64_t csm[3] = {q(cxm), q(cym), q(czm)}, snm[3] = {q(sxm_), q(sym), q(szm_)};
+            using fix::link_of;
+            const int64_t cs[3] = {link_of(cx), link_of(cy), link_of(cz)}, sn[3] = {link_of(sx), link_of(sy), link_of(sz)};
+            const int64_t csm[3] = {link_of(cxm), link_of(cym), link_of(czm)};
+            const int64_t snm[3] = {link_of(sxm_), link_of(sym), link_of(szm_)};
             double u[2], j[3];
             done = fix::scalar_terms<DIAG>({p0, p1}, {{p0xp, p1xp}, {p0yp, p1yp}, {p0zp, p1zp}},
                                      {{p0xm, p1xm}, {p0ym, p1ym}, {p0zm, p1zm}}, cs, sn, csm, snm, u, j, gr);
             x0 = u[0], x1 = u[1], curx = j[0], cury = j[1], curz = j[2];
         }
         if (!done) {
-            auto link = [](double v) { return INT == FIXED_POINT ? fix::link_value(__double_as_longlong(v)) : v; };
             auto direction = [&](double cp, double sp, double cm, double sm, double ap, double bp, double am, double bm,
                                  double& a, double& b, double& cur, double (&g)[2]) {
                 const double A = fma(sp, bp, cp * ap), B = fma(-sp, ap, cp * bp);
@@ -297,9 +295,9 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
                     g[1] = p1 - cm * bm - sm * am;
                 }
             };
-            direction(link(cx), link(sx), link(cxm), link(sxm_), p0xp, p1xp, p0xm, p1xm, x0, x1, curx, gr[0]);
-            direction(link(cy), link(sy), link(cym), link(sym), p0yp, p1yp, p0ym, p1ym, y0, y1, cury, gr[1]);
-            direction(link(cz), link(sz), link(czm), link(szm_), p0zp, p1zp, p0zm, p1zm, z0, z1, curz, gr[2]);
+            direction(cx, sx, cxm, sxm_, p0xp, p1xp, p0xm, p1xm, x0, x1, curx, gr[0]);
+            direction(cy, sy, cym, sym, p0yp, p1yp, p0ym, p1ym, y0, y1, cury, gr[1]);
+            direction(cz, sz, czm, szm_, p0zp, p1zp, p0zm, p1zm, z0, z1, curz, gr[2]);
             if constexpr (INT == FIXED_POINT) {
                 x0 = fma(-6.0, p0, x0 + y0 + z0);
                 x1 = fma(-6.0, p1, x1 + y1 + z1);
@@ -430,9 +428,9 @@ __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, cons
 // smaller ones, with less than two warps for each scheduler, the longer chain of
 // instructions counts: 24^3 diagnostic 31.5 and 33.6, general spacings 18.6 and
 // 20.6.
-// The fused form (equal spacings), FP64 and fixed_point.cuh: 256^3 3120 and 2129
-// (diagnostic 5549 and 4387), 128^3 400 and 276, 64^3 54.5 and 40.6, 40^3 18.5
-// and 16.5, 32^3 11.5 and 11.3, 24^3 9.0 and 9.7.
+// The fused form (equal spacings), FP64 and fixed_point.cuh: 256^3 3091 and 2085
+// (diagnostic 5534 and 4349), 128^3 393 and 269, 64^3 54.6 and 40.2, 40^3 17.9
+// and 15.2, 32^3 10.8 and 10.4, 24^3 8.2 and 9.0.
 constexpr unsigned INT_SITES = 32 * 32 * 32;
 
 // 128 registers: three blocks of 168 spill nothing and are no faster with plain
@@ -508,11 +506,8 @@ cudaError_t launch_ah_twopass(const Geom& g, const Fields<double, 5>& f, double*
     const int la = flat_grid(ra.n), lb = flat_block(ra.n);
     const Flat r = flat_region(g);
     const bool fixed = !STRICT && c.iso != 0 && r.n >= INT_SITES;
-    auto links = [&](auto kernel) {
-        return launch_chained(kernel, la, lb, 0, st, all, ra, f.now[2], f.now[3], f.now[4], Lw);
-    };
-    cudaError_t e = fixed ? links(diag ? ah_links_kernel<STRICT, true, !STRICT> : ah_links_kernel<STRICT, false, !STRICT>)
-                          : links(diag ? ah_links_kernel<STRICT, true, false> : ah_links_kernel<STRICT, false, false>);
+    cudaError_t e = launch_chained(diag ? ah_links_kernel<STRICT, true> : ah_links_kernel<STRICT, false>, la, lb, 0, st, all, ra,
+                                   f.now[2], f.now[3], f.now[4], Lw);
     if (e != cudaSuccess) return e;
     const int grid = flat_grid(r.n), block = flat_block(r.n);
     auto go = [&](auto kernel) { e = launch_chained(kernel, grid, block, 0, st, g, r, f, Lr, c, d); };

@@ -1,13 +1,21 @@
 // The covariant Laplacian and the gauge current of the fused FP64 Abelian-Higgs
-// update in 64-bit fixed point.
+// update by 64-bit integer instructions.
 //
 // They take 38 of the 71 FP64 instructions of a site, on a pipe that issues 2 an
-// SM and cycle and bounds the update.  As integers, a product is a 64 x 64-bit
-// multiplication's high word (about 9 instructions on pipes 32 times as wide)
-// and a sum one addition.  The 14 scalar values that enter share the exponent of
-// the largest (block floating point): units of 2^-60 of it, products truncated
-// to 2^-58 of it, where FP64 rounds every product and sum to 2^-53 of its size.
-// Link cosines and sines are multiples of 2^-62, exact for 1 and 0.
+// SM and cycle and bounds the update.  As integers, a product of two mantissas is
+// three 32 x 32-bit multiplications and a sum one addition after a shift, on pipes
+// 32 times as wide.
+//
+// Every value keeps its own exponent, and every sum is aligned on the largest of
+// its own terms, as a floating-point addition is: a product is truncated to 2^-59
+// of itself, the sum of two of them to 2^-58 of the larger one, each of a Laplacian's
+// seven terms to 2^-57 of the largest, where FP64 rounds each operation to 2^-53 of
+// its result.  So a component, a neighbour, a site's scalar (at a string's core) or
+// a sine that is small beside the others keeps the accuracy that FP64 gives it.
+// (One exponent for all the values of a site, in units of 2^-60 of the largest,
+// lost it: 2e-12 of the current where the scalar is 2^-20 of its neighbours.  It
+// was no faster: 256^3 2113 us a plain step against 2085, 4427 and 4349 with
+// diagnostics.)
 //
 // Only integer operations: the host evaluates the same (for checks).
 #pragma once
@@ -41,7 +49,7 @@ __host__ __device__ inline double of_bits(uint64_t b)
     return x;
 #endif
 }
-// x >> n, 0 for n >= 64
+// x >> n; 0, or the sign, for n >= 64
 __host__ __device__ inline uint64_t shr(uint64_t x, unsigned n)
 {
 #ifdef __CUDA_ARCH__
@@ -52,12 +60,14 @@ __host__ __device__ inline uint64_t shr(uint64_t x, unsigned n)
     return n > 63 ? 0 : x >> n;
 #endif
 }
-__host__ __device__ inline int64_t hi(int64_t a, int64_t b)
+__host__ __device__ inline int64_t sar(int64_t x, unsigned n)
 {
 #ifdef __CUDA_ARCH__
-    return __mul64hi(a, b);
+    int64_t r;
+    asm("shr.s64 %0, %1, %2;" : "=l"(r) : "l"(x), "r"(n));
+    return r;
 #else
-    return (int64_t)(((__int128)a * b) >> 64);
+    return x >> (n > 63 ? 63 : n);
 #endif
 }
 __host__ __device__ inline unsigned lead(uint64_t x)
@@ -68,16 +78,53 @@ __host__ __device__ inline unsigned lead(uint64_t x)
     return (unsigned)__builtin_clzll(x);
 #endif
 }
+__host__ __device__ inline unsigned larger(unsigned a, unsigned b) { return a > b ? a : b; }
 
-__host__ __device__ inline unsigned exponent(uint64_t b) { return (unsigned)(b >> 52) & 0x7ffu; }
+// A link datum: the bits of its cosine or sine.
+__host__ __device__ inline int64_t link_of(double v) { return (int64_t)bits_of(v); }
+__host__ __device__ inline double link_value(int64_t q) { return of_bits((uint64_t)q); }
 
-// The double with bits b, toward zero, in units of 2^(top - 1023 - 63 + drop),
-// top no less than its exponent.  Zeros and subnormals give 0 (top > 64).
-__host__ __device__ inline int64_t fixed(uint64_t b, unsigned top, unsigned drop)
+// A double as m * 2^(e - 1023 - 62), its sign in bit 31 of s: m in [2^62, 2^63),
+// 0 for zero.  Subnormals, infinities and NaN are the caller's to leave out.
+struct Num {
+    uint64_t m;
+    unsigned e, s;
+};
+__host__ __device__ inline Num num(uint64_t b)
 {
-    const uint64_t t = shr((b << 11) | 0x8000000000000000ull, top - exponent(b) + drop);
-    const int64_t s = (int64_t)b >> 63;
-    return ((int64_t)t ^ s) - s;
+    const unsigned h = (unsigned)(b >> 32);
+    const uint64_t lead_bit = (uint64_t)((h & 0x7fffffffu) != 0 ? 0x40000000u : 0u) << 32;
+    return Num{((b << 10) & 0x3fffffffffffffffull) | lead_bit, (h >> 20) & 0x7ffu, h};
+}
+
+// The high word of a * b, both below 2^63; at most 1 too small without EXACT
+// (the low words' product left out).
+template <bool EXACT = false>
+__host__ __device__ inline uint64_t high(uint64_t a, uint64_t b)
+{
+    const uint32_t ah = (uint32_t)(a >> 32), al = (uint32_t)a, bh = (uint32_t)(b >> 32), bl = (uint32_t)b;
+    uint64_t mid = (uint64_t)ah * bl + (uint64_t)al * bh;   // each below 2^63 - 2^32
+    if constexpr (EXACT) mid += ((uint64_t)al * bl) >> 32;
+    return (uint64_t)ah * bh + (mid >> 32);
+}
+
+// v * 2^(e - 2*1023 - 60)
+struct Sum {
+    int64_t v;
+    unsigned e;
+};
+// t with the sign of bit 31 of s
+__host__ __device__ inline int64_t with_sign(uint64_t t, unsigned s)
+{
+    const int64_t n = (int64_t)((int32_t)s >> 31);
+    return ((int64_t)t ^ n) - n;
+}
+// a*b + c*d, flip1, flip2 = ~0: that product with the other sign.  |v| < 2^63, as
+// each product is below 2^62
+__host__ __device__ inline Sum dot(const Num& a, const Num& b, unsigned flip1, const Num& c, const Num& d, unsigned flip2)
+{
+    const unsigned e1 = a.e + b.e, e2 = c.e + d.e, e = larger(e1, e2);
+    return Sum{with_sign(shr(high(a.m, b.m), e - e1), a.s ^ b.s ^ flip1) + with_sign(shr(high(c.m, d.m), e - e2), c.s ^ d.s ^ flip2), e};
 }
 
 // x * 2^k to nearest even; the result has to be normal
@@ -93,17 +140,12 @@ __host__ __device__ inline double to_double(int64_t x, int k)
     return of_bits(x == 0 ? 0 : (sign | m));
 }
 
-// a cosine or sine as a link datum: multiples of 2^-62, kNoLink for NaN
-constexpr int64_t kNoLink = INT64_MIN;
-__host__ __device__ inline int64_t link_of(double v)
-{
-    const uint64_t b = bits_of(v);
-    return exponent(b) > 1023 ? kNoLink : fixed(b, 1023, 1);
-}
-__host__ __device__ inline double link_value(int64_t q) { return q == kNoLink ? of_bits(0x7ff8000000000000ull) : to_double(q, -62); }
-
-// Exponents of the largest scalar for which every result is normal
-constexpr unsigned kTopLow = 560, kTopHigh = 1500;
+// Exponents for which no result leaves the normal range: of the largest scalar; of
+// any scalar or sine that is not zero (twice kLow is 60 bits above the least normal
+// result); of a current that is not zero (three times biased).  (A product with a zero
+// counts by its exponent too, which is under those of the others unless their sum is
+// below 2^-950 of a neighbour.)
+constexpr unsigned kTopLow = 560, kTopHigh = 1500, kLow = 548, kCurLow = 3 * 1023 - 940;
 
 // u[comp]: the sum over the directions of the transported neighbours minus six
 // times the site's scalar; cur[mu] = phi1 A_mu - phi0 B_mu, (A_mu, B_mu) the
@@ -116,48 +158,79 @@ __host__ __device__ inline bool scalar_terms(const double (&p)[2], const double 
                                              const int64_t (&snm)[3], double (&u)[2], double (&cur)[3],
                                              double (*grad)[2] = nullptr)
 {
-    unsigned top = 0;
-    int low = 0;
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-        const unsigned h = (unsigned)(bits_of(p[k]) >> 32) & 0x7fffffffu;
-        top = top > h ? top : h;
-    }
+    // top: of the scalars; low: of what is not zero (x - 1 wraps to the largest
+    // for zero); one: of the cosines, NaN and Inf above all others
+    unsigned top = 0, low = ~0u, one = 0;
+    auto magnitude = [](uint64_t b) { return (unsigned)(b >> 32) & 0x7fffffffu; };
+    auto scalar = [&](double v) {
+        const unsigned x = magnitude(bits_of(v));
+        top = larger(top, x);
+        low = x - 1 < low ? x - 1 : low;
+    };
+    auto link = [&](int64_t c, int64_t s) {
+        const unsigned x = magnitude((uint64_t)s) - 1;
+        one = larger(one, magnitude((uint64_t)c));
+        low = x < low ? x : low;
+    };
+    scalar(p[0]), scalar(p[1]);
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-#pragma unroll
-        for (int k = 0; k < 2; ++k) {
-            const unsigned f = (unsigned)(bits_of(fwd[a][k]) >> 32) & 0x7fffffffu;
-            const unsigned b = (unsigned)(bits_of(bwd[a][k]) >> 32) & 0x7fffffffu;
-            top = top > f ? top : f;
-            top = top > b ? top : b;
-        }
-        const int c0 = (int)(cs[a] >> 32), c1 = (int)(csm[a] >> 32);
-        low = low < c0 ? low : c0;
-        low = low < c1 ? low : c1;
+        scalar(fwd[a][0]), scalar(fwd[a][1]), scalar(bwd[a][0]), scalar(bwd[a][1]);
+        link(cs[a], sn[a]), link(csm[a], snm[a]);
     }
-    top >>= 20;
-    if (top - kTopLow >= kTopHigh - kTopLow || low < -(1 << 30)) return false;
+    if ((top >> 20) - kTopLow >= kTopHigh - kTopLow || low < (kLow << 20) - 1 || one >= 1024u << 20) return false;
 
-    const int64_t f0 = fixed(bits_of(p[0]), top, 3), f1 = fixed(bits_of(p[1]), top, 3);   // below 2^61
-    int64_t x0 = -((3 * f0) >> 1), x1 = -((3 * f1) >> 1);   // as the products: a quarter of the unit's count
+    const Num p0 = num(bits_of(p[0])), p1 = num(bits_of(p[1]));
+    // the site's scalar as a Sum: a cosine of 1 has exponent 1023, bit 62
+    const Sum s0{with_sign(p0.m >> 2, p0.s), p0.e + 1023}, s1{with_sign(p1.m >> 2, p1.s), p1.e + 1023};
+    Sum A[3], B[3], T0[3], T1[3];   // transported neighbours: forward, and the backward ones negated
+    unsigned e0 = s0.e, e1 = s1.e;
+    bool small = false;
 #pragma unroll
     for (int a = 0; a < 3; ++a) {
-        const int64_t a0 = fixed(bits_of(fwd[a][0]), top, 3), a1 = fixed(bits_of(fwd[a][1]), top, 3);
-        const int64_t b0 = fixed(bits_of(bwd[a][0]), top, 3), b1 = fixed(bits_of(bwd[a][1]), top, 3);
-        const int64_t A = hi(a0, cs[a]) + hi(a1, sn[a]), B = hi(a1, cs[a]) - hi(a0, sn[a]);
-        const int64_t t0 = hi(b0, csm[a]) - hi(b1, snm[a]), t1 = hi(b1, csm[a]) + hi(b0, snm[a]);
-        x0 += A + t0;
-        x1 += B + t1;
+        const Num a0 = num(bits_of(fwd[a][0])), a1 = num(bits_of(fwd[a][1]));
+        const Num c = num((uint64_t)cs[a]), s = num((uint64_t)sn[a]);
+        A[a] = dot(a0, c, 0, a1, s, 0);
+        B[a] = dot(a1, c, 0, a0, s, ~0u);
+        const Num b0 = num(bits_of(bwd[a][0])), b1 = num(bits_of(bwd[a][1]));
+        const Num cm = num((uint64_t)csm[a]), sm = num((uint64_t)snm[a]);
+        T0[a] = dot(b1, sm, 0, b0, cm, ~0u);
+        T1[a] = dot(b1, cm, ~0u, b0, sm, ~0u);
+        e0 = larger(e0, larger(A[a].e, T0[a].e));
+        e1 = larger(e1, larger(B[a].e, T1[a].e));
+
+        const unsigned j1 = p1.e + A[a].e, j0 = p0.e + B[a].e, j = larger(j1, j0);
+        // exact before the truncation: a uniform scalar's two products cancel
+        auto times = [](const Num& x, const Sum& y, unsigned n) {
+            const unsigned ys = (unsigned)((uint64_t)y.v >> 32);
+            return with_sign(shr(high<true>((uint64_t)with_sign((uint64_t)y.v, ys), x.m), n), x.s ^ ys);
+        };
+        const int64_t q = times(p1, A[a], j - j1) - times(p0, B[a], j - j0);
+        small |= q != 0 && j < kCurLow;
+        cur[a] = to_double(q, (int)j - 3 * 1023 - 58);
         if constexpr (GRAD) {
-            grad[a][0] = to_double((f0 >> 2) - t0, (int)top - 1081);
-            grad[a][1] = to_double((f1 >> 2) - t1, (int)top - 1081);
+            auto less = [&](const Sum& x, const Sum& t) {
+                const unsigned e = larger(x.e, t.e);
+                // |t.v| is up to 2^63; x.v has eight zero bits, and one bit stands for those that a longer shift leaves out
+                const unsigned n = e - x.e + 1;
+                const int64_t d = (sar(x.v, n) | (n > 8 ? 1 : 0)) + sar(t.v, e - t.e + 1);
+                return to_double(d, (int)e - 2 * 1023 - 59);
+            };
+            grad[a][0] = less(s0, T0[a]);
+            grad[a][1] = less(s1, T1[a]);
         }
-        cur[a] = to_double(hi(f1, A * 4) - hi(f0, B * 4), 2 * (int)top - 2102);
     }
-    u[0] = to_double(x0, (int)top - 1081);
-    u[1] = to_double(x1, (int)top - 1081);
-    return true;
+    // In eighths, which sum up to less than (6 * 2^63 + 6 * 2^61) / 8; the backward
+    // terms subtracted, so that the truncations' means cancel.
+    int64_t x0 = -sar(3 * s0.v, e0 - s0.e + 2), x1 = -sar(3 * s1.v, e1 - s1.e + 2);
+#pragma unroll
+    for (int a = 0; a < 3; ++a) {
+        x0 += sar(A[a].v, e0 - A[a].e + 3) - sar(T0[a].v, e0 - T0[a].e + 3);
+        x1 += sar(B[a].v, e1 - B[a].e + 3) - sar(T1[a].v, e1 - T1[a].e + 3);
+    }
+    u[0] = to_double(x0, (int)e0 - 2 * 1023 - 57);
+    u[1] = to_double(x1, (int)e1 - 2 * 1023 - 57);
+    return !small;
 }
 
 }  // namespace fix
