@@ -282,7 +282,7 @@ int lat_create(const lat_params* p, lat_handle** out)
     };
     h->recip = pow2(p->dx) && pow2(p->dy) && pow2(p->dz);
     h->geom = make_geom(*p);
-    h->chunk = default_chunk(*p);
+    set_chunk(h, default_chunk(*p));
     cudaGetDevice(&h->device);
     auto fail = [&](int code) {
         lat_destroy(h);
@@ -555,7 +555,7 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
                 f.past[c] = (float*)h->slot(c, tPast);
             }
             if (p.kernel_variant != 1)
-                LAT_CKL(launch_ah_tiled_f32(h->geom, f, cf, d, diag, h->chunk, h->stream, p.kernel_variant, &used));
+                LAT_CKL(launch_ah_tiled_f32(h->geom, f, cf, d, diag, h->launch_chunk, h->stream, p.kernel_variant, &used));
             else LAT_CKL(launch_ah_step_f32(h->geom, f, cf, d, diag, h->stream));
         }
     } else {
@@ -581,7 +581,7 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
                 f.past[c] = (float*)h->slot(c, tPast);
             }
             if (p.kernel_variant != 1) {
-                LAT_CKL(launch_moore_tiled_f32(h->geom, f, cf, d, diag, h->chunk, h->stream, p.kernel_variant, &used));
+                LAT_CKL(launch_moore_tiled_f32(h->geom, f, cf, d, diag, h->launch_chunk, h->stream, p.kernel_variant, &used));
             } else {
                 LAT_CKL(launch_moore_step_f32(h->geom, f, cf, d, diag, h->stream));
                 used = tile_count(h->geom);

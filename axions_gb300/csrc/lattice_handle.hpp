@@ -25,6 +25,7 @@ struct lat_handle {
     size_t links_bytes = 0;
     bool recip = false;        // every spacing is a power of two: exact reciprocals
     int chunk = 32;            // x-planes per CTA of the tiled FP32 kernel
+    int launch_chunk = 32;     // those its steps are launched with (set_chunk)
     double* partials = nullptr;
     int nblocks = 0;           // capacity of `partials` in (energy, |G|) pairs
     double* diag_dev = nullptr;
@@ -55,3 +56,7 @@ struct lat_handle {
 
     char* slot(int comp, int t) const { return (char*)fields + ((size_t)comp * 2 + (size_t)t) * (size_t)N * elem; }
 };
+
+namespace lat {
+void set_chunk(lat_handle* h, int chunk);   // tune.cu
+}

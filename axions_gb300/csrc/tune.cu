@@ -1,7 +1,8 @@
 // Autotuning of the tiled FP32 step: the number of x-planes each CTA marches
 // through ("chunk").  Short chunks give small lattices enough CTAs to fill the
 // 152 SMs; long chunks spend less on each CTA's prologue (one extra plane of
-// link data and the pipeline fill).  lat_autotune() times every candidate on a
+// link data and the pipeline fill).  lat_autotune() times candidates, every default
+// among them, on a
 // scratch lattice of the caller's shape (device-generated IC, the caller's
 // state is not touched), applies the fastest to the handle and remembers it
 // per shape; new handles of a tuned shape start with the remembered value and
@@ -13,6 +14,7 @@
 #include <fstream>
 #include <map>
 #include <mutex>
+#include <set>
 #include <sstream>
 #include <string>
 #include <tuple>
@@ -36,7 +38,9 @@ std::map<Key, Entry> g_tune;
 
 Key key_of(const lat_params& p) { return Key(p.model, p.precision, p.bc, p.nx, p.ny, p.nz); }
 
-const int kCandidates[] = {4, 8, 16, 32, 64, 128};
+// Timed by lat_autotune: the long ones, then the others default_chunk may pick.
+const int kLong[] = {4, 8, 16, 32, 64, 128};
+const int kOthers[] = {1, 2, 6, 12, 24};
 
 }  // namespace
 
@@ -54,8 +58,28 @@ static double march_cost(int chunk, double ctas)
     return (chunk + 1.7) * (0.4 + 0.41 * std::ceil(ctas / 152));
 }
 
-// Default chunk for a handle: the tuned value of its shape, else the cheapest
-// by march_cost.
+static double march_ctas(const lat_params& p, int chunk)
+{
+    const Geom g = make_geom(p);
+    return (double)march_tiles(g, p.model == LAT_MODEL_MOORE) * ((g.hix - g.lox - 1) / chunk + 1);
+}
+
+// The cheapest chunk by march_cost.
+static int model_chunk(const lat_params& p)
+{
+    int best = 1;
+    double cost = 1e300;
+    for (int c : {1, 2, 4, 6, 8, 12, 16, 24, 32}) {
+        const double t = march_cost(c, march_ctas(p, c));
+        if (t < cost) {
+            cost = t;
+            best = c;
+        }
+    }
+    return best;
+}
+
+// Default chunk for a handle: the tuned value of its shape, else the model's.
 int default_chunk(const lat_params& p)
 {
     {
@@ -63,19 +87,22 @@ int default_chunk(const lat_params& p)
         auto it = g_tune.find(key_of(p));
         if (it != g_tune.end()) return it->second.chunk;
     }
-    const Geom g = make_geom(p);
-    const double tiles = (double)march_tiles(g, p.model == LAT_MODEL_MOORE);
-    const int x = g.hix - g.lox;
-    int best = 1;
-    double cost = 1e300;
-    for (int c : {1, 2, 4, 6, 8, 12, 16, 24, 32}) {
-        const double t = march_cost(c, tiles * ((x + c - 1) / c));
-        if (t < cost) {
-            cost = t;
-            best = c;
-        }
-    }
-    return best;
+    return model_chunk(p);
+}
+
+// Sets a handle's chunk and the one its steps are launched with: the same, except
+// that one longer than the model's choice gives way to it where it leaves SMs
+// without a CTA or is more than 10 % dearer by the model, twice what that is off by.
+// Files tuned to longer chunks and chunks set for another shape leave a small
+// lattice with too few CTAs otherwise: 32^3 with 4 planes takes 5.3 us a step, with 1
+// 2.5; 64x48x40 6.5 with 4 and 5.1 with 2; 40x36x33 6.4 with 4 and 4.0 with 1.
+void set_chunk(lat_handle* h, int chunk)
+{
+    const int model = model_chunk(h->p);
+    const double ctas = march_ctas(h->p, chunk), best = march_ctas(h->p, model);
+    h->chunk = chunk;
+    h->launch_chunk =
+        chunk > model && (ctas < 152 || march_cost(chunk, ctas) > 1.1 * march_cost(model, best)) ? model : chunk;
 }
 
 }  // namespace lat
@@ -103,7 +130,7 @@ int lat_set_tuning(lat_handle* h, const lat_tuning* t)
         set_error("lat_set_tuning: bad argument");
         return LAT_ERR_INVALID;
     }
-    h->chunk = t->chunk;
+    set_chunk(h, t->chunk);
     return LAT_OK;
 }
 
@@ -135,27 +162,38 @@ int lat_autotune(lat_handle* h, int32_t trial_steps, lat_tuning* out)
     const Geom& g = h->geom;
     double best_ms = 1e300;
     int best = h->chunk, tried = 0;
-    for (int c : kCandidates) {
-        if (c > 2 * (g.hix - g.lox) && c != kCandidates[0]) continue;  // beyond the lattice: same as a shorter one
-        t->chunk = c;
-        if ((rc = lat_step(t, 1))) break;  // warm-up
-        cudaEventRecord(e0, t->stream);
-        if ((rc = lat_step(t, trial_steps))) break;
-        cudaEventRecord(e1, t->stream);
-        cudaEventSynchronize(e1);
-        float ms = 0;
-        cudaEventElapsedTime(&ms, e0, e1);
+    std::set<int> launched;   // the chunks timed, as launched
+    auto time = [&](int c) {   // the fastest of three runs
+        launched.insert(t->launch_chunk);
         ++tried;
-        if (ms / trial_steps < best_ms) {
-            best_ms = ms / trial_steps;
-            best = c;
+        for (int run = 0; run < 3; ++run) {
+            if ((rc = lat_step(t, 1))) return;  // warm-up
+            cudaEventRecord(e0, t->stream);
+            if ((rc = lat_step(t, trial_steps))) return;
+            cudaEventRecord(e1, t->stream);
+            cudaEventSynchronize(e1);
+            float ms = 0;
+            cudaEventElapsedTime(&ms, e0, e1);
+            if (ms / trial_steps < best_ms) {
+                best_ms = ms / trial_steps;
+                best = c;
+            }
         }
+    };
+    for (int c : kLong) {
+        if (rc || (c > 2 * (g.hix - g.lox) && c != kLong[0])) continue;  // beyond the lattice: same as a shorter one
+        set_chunk(t, c);
+        time(c);
+    }
+    for (int c : kOthers) {
+        set_chunk(t, c);
+        if (!rc && !launched.count(t->launch_chunk)) time(c);
     }
     cudaEventDestroy(e0);
     cudaEventDestroy(e1);
     lat_destroy(t);
     if (rc) return rc;
-    h->chunk = best;
+    set_chunk(h, best);
     {
         std::lock_guard<std::mutex> lock(g_tune_mu);
         g_tune[key_of(h->p)] = {best, best_ms};

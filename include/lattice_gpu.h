@@ -427,10 +427,11 @@ int lat_philox4x32_10(const uint32_t counter[4], const uint32_t key[2], uint32_t
 int lat_dtrig_eval(const double* x, int64_t n, double* out);
 
 /* ---- tuning of the tiled FP32 step ------------------------------------------------
- * chunk = x-planes each CTA of the tiled FP32 step marches through.  New
- * handles start with the value tuned for their shape in this process (or
- * loaded from a cache file), else with a heuristic.  lat_autotune times the
- * candidates on a scratch lattice of the same shape (the handle's state is
+ * chunk = x-planes each CTA of the tiled FP32 step marches through (fewer where
+ * so many would leave the GPU with too few CTAs).  New handles start with the
+ * value tuned for their shape in this process (or loaded from a cache file),
+ * else with a heuristic.  lat_autotune times candidates, the heuristic's choice
+ * among them, on a scratch lattice of the same shape (the handle's state is
  * untouched), applies the fastest and remembers it.  No counterpart in the
  * reference. */
 typedef struct lat_tuning {
