@@ -548,7 +548,7 @@ int lat_batch_advance(lat_batch* b, int32_t nsteps)
         J.d.write = 1;
         const int x = h->geom.hix - h->geom.lox;
         const int planes = partial_planes(h->N);
-        J.chunk = b->chunk > 0 ? std::min(x, b->chunk) : std::max(chunk, planes);
+        J.chunk = b->chunk > 0 ? b->chunk : std::max(chunk, planes);   // may exceed x: one item, the same partials
         J.psub = J.chunk % planes == 0 ? planes : 0;
         J.vec = tiled_vec_ok(h->geom, level_fields(h, h->n)) ? 1 : 0;
         const dim3 tg = plan[q].table == kMooreTiled ? tiled_grid(h->geom, J.chunk)

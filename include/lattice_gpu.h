@@ -466,7 +466,7 @@ int lat_batch_destroy(lat_batch* b);                               /* handles ar
 int lat_batch_add(lat_batch* b, lat_handle* h, int32_t diag_every, int64_t stop_step);
 int lat_batch_remove(lat_batch* b, lat_handle* h);
 int lat_batch_size(const lat_batch* b);
-/* x-planes per work item for every lattice of the batch (clamped to its x
+/* x-planes per work item for every lattice of the batch (at most its x
    extent); 0 restores the default, which depends on how much work the running
    lattices are together.  The fields do not depend on it; the diagnostics'
    partial sums do for explicit values that are no multiple of 8, never for
