@@ -557,6 +557,10 @@ int lat_batch_advance(lat_batch* b, int32_t nsteps)
         J.tiles_y = (int)tg.y;
         J.items = (int)(tg.x * tg.y * tg.z);
         J.partials = J.tiles_z * J.tiles_y * (J.psub > 0 ? (x + J.psub - 1) / J.psub : (int)tg.z);
+        if (J.partials > h->nblocks) {
+            set_error("lat_batch_advance: more diagnostic partials than a lattice has room for");
+            return LAT_ERR_STATE;
+        }
     }
     for (int s = 0; s < K; ++s) {
         BatchJob* const jobs = b->jobs_of(b->tab_host, s);

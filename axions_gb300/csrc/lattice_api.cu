@@ -554,9 +554,12 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
                 f.now[c] = (const float*)h->slot(c, tNow);
                 f.past[c] = (float*)h->slot(c, tPast);
             }
-            if (p.kernel_variant != 1)
+            if (p.kernel_variant != 1) {
+                used = h->nblocks;
                 LAT_CKL(launch_ah_tiled_f32(h->geom, f, cf, d, diag, h->launch_chunk, h->stream, p.kernel_variant, &used));
-            else LAT_CKL(launch_ah_step_f32(h->geom, f, cf, d, diag, h->stream));
+            } else {
+                LAT_CKL(launch_ah_step_f32(h->geom, f, cf, d, diag, h->stream));
+            }
         }
     } else {
         if (h->elem == 8) {
@@ -581,6 +584,7 @@ static int do_step(lat_handle* h, bool diag, bool store_div, double* diag_dst, b
                 f.past[c] = (float*)h->slot(c, tPast);
             }
             if (p.kernel_variant != 1) {
+                used = h->nblocks;
                 LAT_CKL(launch_moore_tiled_f32(h->geom, f, cf, d, diag, h->launch_chunk, h->stream, p.kernel_variant, &used));
             } else {
                 LAT_CKL(launch_moore_step_f32(h->geom, f, cf, d, diag, h->stream));

@@ -122,10 +122,11 @@ inline int flat_grid(unsigned n)
 // (energy, |G|) pairs a handle's diagnostic steps may write
 int64_t moore_march_partials(const Geom& g);
 int64_t march_tiles(const Geom& g, bool moore);   // tiles of a plane of the x-marching FP32 step
+int64_t march_tiles_most(const Geom& g);          // the same for the tile shape with the most of them
 inline int64_t partial_pairs(const Geom& g)
 {
     int64_t most = tile_count(g);
-    for (const int64_t n : {(int64_t)flat_grid(flat_region(g).n), moore_march_partials(g), march_tiles(g, false) * (g.hix - g.lox)})
+    for (const int64_t n : {(int64_t)flat_grid(flat_region(g).n), moore_march_partials(g), march_tiles_most(g) * (g.hix - g.lox)})
         most = n > most ? n : most;
     return most;
 }
@@ -230,8 +231,9 @@ int batch_chunk(const Geom& g);
 // x-marching FP32 steps, `chunk` x-planes per CTA.  variant 0: the pair step
 // (two z-sites per thread, pair_step.cuh; Moore lattices where pair_moore_ok,
 // else the tiled step); 2: the tiled step (tiled_step.cuh) with one-element staging
-// copies; 3: the tiled step with 16-byte staging where allowed.  *blocks
-// receives the CTAs (diagnostic partials) of the kernel launched.
+// copies; 3: the tiled step with 16-byte staging where allowed.  *blocks: the
+// diagnostic partials there is room for (a diagnostic step that needs more is not
+// launched); receives the CTAs (diagnostic partials) of the kernel launched.
 cudaError_t launch_ah_tiled_f32(const Geom&, const Fields<float, 5>&, const StepCoef&, const DiagOut&, bool diag,
                                 int chunk, cudaStream_t, int variant, int* blocks);
 cudaError_t launch_moore_tiled_f32(const Geom&, const Fields<float, 7>&, const StepCoef&, const DiagOut&, bool diag,

@@ -760,11 +760,12 @@ pair_step_kernel(const Geom g, const SH sh, const Fields<float, 2 * NS + 3> f, c
 // differently from the tiled step, and at strong coupling, g >= 1.2 at spacing
 // 0.5 without friction, the two-scalar model grows a last-bit difference to
 // 1e-3 within 120 steps.)
-inline bool pair_moore_ok(const Geom& g, const Fields<float, 7>& f)
+inline bool pair_moore_fits(const Geom& g)
 {
     const int tiles = (g.nz + 63) / 64;
-    return tiled_vec_ok<float, 7>(g, f) && 10 * g.nz >= 9 * 64 * tiles;
+    return tiled_vec_fits(g) && 10 * g.nz >= 9 * 64 * tiles;
 }
+inline bool pair_moore_ok(const Geom& g, const Fields<float, 7>& f) { return pair_moore_fits(g) && tiled_vec_ok<float, 7>(g, f); }
 
 // Pairs per row of an Abelian-Higgs lattice's tile: 32 or 16, whichever leaves
 // fewer lanes idle; 32 for equal counts.
@@ -775,7 +776,8 @@ inline int pair_tz2(const Geom& g)
     return wide <= narrow ? 32 : 16;
 }
 
-// Launch the pair step (Moore: where pair_moore_ok).  *blocks receives the CTAs (diagnostic partials).
+// Launch the pair step (Moore: where pair_moore_ok).  *blocks: room for diagnostic
+// partials in, the CTAs (diagnostic partials) out.
 template <int NS>
 cudaError_t launch_pair_t(const Geom& g, const Fields<float, 2 * NS + 3>& f, const StepCoef& c64, const DiagOut& d,
                           bool diag, int chunk, cudaStream_t st, int* blocks)
@@ -800,9 +802,14 @@ cudaError_t launch_pair_t(const Geom& g, const Fields<float, 2 * NS + 3>& f, con
     const bool q12 = NS == 2 && ch.qpow[0] == 1 && ch.qpow[1] == 2;
     cudaError_t err = cudaSuccess;
     auto go = [&](auto kernel, auto sh, dim3 grid) {
+        const int ctas = (int)(grid.x * grid.y * grid.z);
+        if (diag && ctas > *blocks) {
+            err = cudaErrorInvalidConfiguration;
+            return;
+        }
+        *blocks = ctas;
         cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
         err = launch_chained(kernel, grid, block, smem, st, g, sh, f, c, ch, d, chunk);
-        *blocks = (int)(grid.x * grid.y * grid.z);
     };
     auto pick = [&](auto sh, dim3 grid) {
         using SH = decltype(sh);

@@ -172,10 +172,11 @@ __device__ __forceinline__ void stage_plane_vec(TiledSmem<T, NS>& sm, int b, con
 // Whether the tiled step may stage by 16-byte copies: FP32 fields, periodic z
 // with nz a multiple of 4 (rows and chunk starts on 16-byte boundaries) and
 // every field pointer 16-byte aligned.
+inline bool tiled_vec_fits(const Geom& g) { return g.loz == 0 && g.hiz == g.nz && (g.nz & 3) == 0; }
 template <class T, int NC>
 inline bool tiled_vec_ok(const Geom& g, const Fields<T, NC>& f)
 {
-    if (sizeof(T) != 4 || g.loz != 0 || g.hiz != g.nz || (g.nz & 3) != 0) return false;
+    if (sizeof(T) != 4 || !tiled_vec_fits(g)) return false;
     for (int c = 0; c < NC; ++c)
         if ((reinterpret_cast<uintptr_t>(f.now[c]) & 15) != 0) return false;
     return true;
