@@ -8,6 +8,7 @@
 #include <string>
 #include <vector>
 
+#include "alloc_retry.hpp"
 #include "lattice_handle.hpp"
 #include "lattice_internal.cuh"
 
@@ -785,6 +786,16 @@ static DetectStash detect_stash(lat_handle* h, int nb, int64_t want)
     return DetectStash{h->det_stash, cap};
 }
 
+// The stash given back, for an allocation that failed; false if there was none.
+static bool drop_stash(lat_handle* h)
+{
+    cudaGetLastError();
+    const bool held = h->det_stash != nullptr;
+    dev_free(h, &h->det_stash, h->det_stash_bytes);   // waits for what reads it
+    h->det_stash_bytes = 0;
+    return held;
+}
+
 // count the crossings of `field` on the current level (block totals scanned in
 // place); `want` of them are to be written afterwards, *sh tells detect_write
 // where they are kept
@@ -814,14 +825,20 @@ static int detect_count(lat_handle* h, int32_t field, int64_t want, int64_t* tot
     return LAT_OK;
 }
 
-// write the first nw of the `total` crossings (after detect_count) into h->det_xyz
-static int detect_write(lat_handle* h, int32_t field, int64_t total, int64_t nw, const DetectStash& sh)
+// write the first nw of the `total` crossings (after detect_count) into h->det_xyz;
+// where the list does not fit beside the stash, it takes the stash's place and the
+// crossings are found again
+static int detect_write(lat_handle* h, int32_t field, int64_t total, int64_t nw, DetectStash sh)
 {
     if (nw <= 0) return LAT_OK;
     if (nw > h->det_cap) {
         dev_free(h, (void**)&h->det_xyz, sizeof(double) * 3 * (size_t)h->det_cap);
         h->det_cap = 0;
-        int rc = dev_alloc(h, (void**)&h->det_xyz, sizeof(double) * 3 * (size_t)nw);
+        int rc = alloc_or_release([&] { return dev_alloc(h, (void**)&h->det_xyz, sizeof(double) * 3 * (size_t)nw); },
+                                  [&] {
+                                      sh = DetectStash{};
+                                      return drop_stash(h);
+                                  });
         if (rc) return rc;
         h->det_cap = nw;
     }
@@ -880,9 +897,17 @@ int lat_string_length(lat_handle* h, int32_t field, int32_t split, int32_t metho
     if (total == 0) return LAT_OK;
     if ((rc = detect_write(h, field, total, total, sh))) return rc;
     if (method == LAT_CHAIN_AUTO) method = periodic ? LAT_CHAIN_HASH : LAT_CHAIN_EXHAUSTIVE;
-    const ChainGeom g = make_chain_geom(h->p, total);
+    ChainGeom g = make_chain_geom(h->p, total);
     double out[2];
-    rc = chain_length_run(g, h->det_xyz, total, split, method, h->chain, &h->bytes, h->stream, out, &h->launches);
+    rc = alloc_or_release(
+        [&] { return chain_length_run(g, h->det_xyz, total, split, method, h->chain, &h->bytes, h->stream, out, &h->launches); },
+        [&] { return drop_stash(h); },
+        [&] {
+            cudaGetLastError();
+            chain_buffers_release(h->chain, &h->bytes);
+            g = make_chain_geom(h->p, total, 2);
+            return true;
+        });
     if (rc) return rc;
     *L0 = out[0];
     *L1 = out[1];

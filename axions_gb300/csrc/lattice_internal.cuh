@@ -308,7 +308,8 @@ struct ChainGeom {
     signed char off[27][3];
 };
 
-ChainGeom make_chain_geom(const lat_params& p, int64_t M);
+// cells: hash cells per crossing where the cutoff allows as many (up to 2^22 cells)
+ChainGeom make_chain_geom(const lat_params& p, int64_t M, int cells = 64);
 // points lie in the box the hash covers (finite, within [lo, lo+L] per axis)
 bool chain_points_in_box(const ChainGeom& g, const double* xyz_host, int64_t M);
 // device buffers of the chaining, kept between calls (grown as needed)

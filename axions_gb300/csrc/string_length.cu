@@ -42,6 +42,7 @@
 #include <climits>
 #include <cmath>
 
+#include "alloc_retry.hpp"
 #include "lattice_internal.cuh"
 
 namespace lat {
@@ -950,7 +951,7 @@ int coop_grid(int64_t M, int* grid)
 // ---------------------------------------------------------------------------
 // host side
 // ---------------------------------------------------------------------------
-ChainGeom make_chain_geom(const lat_params& p, int64_t M)
+ChainGeom make_chain_geom(const lat_params& p, int64_t M, int cells)
 {
     ChainGeom g{};
     const int64_t n[3] = {p.nx, p.ny, p.nz};
@@ -974,12 +975,12 @@ ChainGeom make_chain_geom(const lat_params& p, int64_t M)
         nb[a] = (long long)q;
     }
     // Cells as small as the cutoff allows, as long as their tables (12 B a cell)
-    // stay small: 64 cells per crossing up to 2^22 cells (50 MB), else two per
-    // crossing.  Strings leave most cells empty, so two per crossing are cells
+    // stay small: 64 cells per crossing (`cells`) up to 2^22 cells (50 MB), else two
+    // per crossing, which is also what is left where 50 MB are not to be had.  Strings leave most cells empty, so two per crossing are cells
     // several cutoffs wide, full of crossings out of reach (0.73 ms instead of
     // a fraction of that for the link count of 6.7x10^4 crossings at 256^3).
     const long long m1 = std::max<int64_t>(M, 1);
-    const long long cap = std::max<long long>(64, std::max<long long>(2 * m1, std::min<long long>(64 * m1, 1 << 22)));
+    const long long cap = std::max<long long>(64, std::max<long long>(2 * m1, std::min<long long>(cells * m1, 1 << 22)));
     while (nb[0] * nb[1] * nb[2] > cap) {
         int a = 0;
         if (nb[1] > nb[a]) a = 1;
@@ -1155,7 +1156,7 @@ extern "C" int lat_string_length_points(const lat_params* p, const double* xyz, 
     }
     *L0 = *L1 = 0.0;
     if (M == 0) return LAT_OK;
-    const ChainGeom g = make_chain_geom(*p, M);
+    ChainGeom g = make_chain_geom(*p, M);
     const bool hashable = g.periodic[0] && g.periodic[1] && g.periodic[2] && chain_points_in_box(g, xyz, M);
     if (method == LAT_CHAIN_HASH && !hashable) {
         set_error("lat_string_length_points: the hash needs a periodic lattice and points inside the box");
@@ -1175,7 +1176,13 @@ extern "C" int lat_string_length_points(const lat_params* p, const double* xyz, 
         set_error(std::string("lat_string_length_points: ") + cudaGetErrorString(e));
         rc = e == cudaErrorMemoryAllocation ? LAT_ERR_NOMEM : LAT_ERR_CUDA;
     } else {
-        rc = chain_length_run(g, d_xyz, M, split, method, buf, nullptr, st, out, nullptr);
+        rc = alloc_or_release([&] { return chain_length_run(g, d_xyz, M, split, method, buf, nullptr, st, out, nullptr); },
+                              [&] {
+                                  cudaGetLastError();
+                                  chain_buffers_release(buf, nullptr);
+                                  g = make_chain_geom(*p, M, 2);
+                                  return true;
+                              });
     }
     if (st) cudaStreamSynchronize(st);
     chain_buffers_release(buf, nullptr);
