@@ -20,10 +20,16 @@ namespace lat {
 namespace {
 
 constexpr int DB = 256;           // threads per detection block
-constexpr int DR = 4;             // sites per thread
-constexpr int DSITES = DB * DR;   // sites per detection block
+constexpr int DR_MOST = 4;        // sites per thread: 4, or 1 (detect_rounds)
 constexpr int DWARPS = DB / 32;
-constexpr int DCHUNKS = 3 * DR;   // most chunks of DB candidate faces in a block
+constexpr int DCHUNKS = 3 * DR_MOST;   // most chunks of DB candidate faces in a block
+
+// Sites per thread: four, so that the faces left by the FP32 test fill the lanes
+// of the FP64 root search, unless that leaves fewer than two blocks for each SM.
+// us for counting FP64 levels, noise and 60 steps later, with one and with four:
+// 16^3 41, 29 and 78, 33; 32^3 41, 30 and 78, 34; 48^3 66, 29 and 77, 32; 64^3 115, 41
+// and 116, 42; 80^3 177, 54 and 201, 43; 128^3 606, 127 and 601, 102.
+inline int detect_rounds(int64_t sites) { return sites < 2 * 152 * DB * DR_MOST ? 1 : DR_MOST; }
 
 // Offsets to the forward neighbours of site s, and whether it is examined.
 struct Site {
@@ -59,17 +65,18 @@ inline double* stash_xyz(const DetectStash& sh, int nb)
 
 enum DetectMode { DETECT_COUNT, DETECT_STASH, DETECT_WRITE };
 
-// Sites [blockIdx.x*DSITES, +DSITES): candidate faces are listed in the
+// Sites [blockIdx.x*DB*DR, +DB*DR): candidate faces are listed in the
 // reference's order (sites in linear order; z-, y-, x-directed face), then
 // evaluated DB at a time.  COUNT: the block's number of crossings to totals;
 // STASH: the same, and the crossings to the stash (`used` counts them, beyond
 // `cap` they are not stored); WRITE: the crossings to xyz at totals (scanned).
-template <class T, int MODE>
+template <class T, int MODE, int DR>
 __global__ void __launch_bounds__(DB) detect_kernel(const DetectArgs a, const T* __restrict__ re,
                                                     const T* __restrict__ im, const float eref, long long* totals,
                                                     double* __restrict__ xyz, long long cap, unsigned* used,
                                                     StashChunk* __restrict__ chunks)
 {
+    constexpr int DSITES = DB * DR;
     __shared__ unsigned short list[3 * DSITES];   // site within the block * 4 + face
     __shared__ int wsum[DR * DWARPS];             // candidates of warp w, round r at [r*DWARPS + w]
     __shared__ int csum[DWARPS];                  // crossings of a warp in the current chunk
@@ -97,16 +104,17 @@ __global__ void __launch_bounds__(DB) detect_kernel(const DetectArgs a, const T*
         if (lane == 0) wsum[r * DWARPS + wid] = n;
     }
     __syncthreads();
-    static_assert(DR * DWARPS == 32, "one warp scans the warps' candidate counts");
+    constexpr int NSUM = DR * DWARPS;
+    static_assert(NSUM <= 32, "one warp scans the warps' candidate counts");
     if (wid == 0) {
-        const int own = wsum[lane];
+        const int own = lane < NSUM ? wsum[lane] : 0;
         int incl = own;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
             const int t = __shfl_up_sync(0xffffffffu, incl, o);
             if (lane >= o) incl += t;
         }
-        wsum[lane] = incl - own;
+        if (lane < NSUM) wsum[lane] = incl - own;
         if (lane == 31) s_base = (unsigned)incl;
     }
     __syncthreads();
@@ -354,27 +362,39 @@ inline float reference_error(const DetectArgs& a)
     return (float)(e < 1 ? e : 1);
 }
 
-template <class T>
-cudaError_t detect_launch(const DetectArgs& a, const T* re, const T* im, long long* bt, int nb, const DetectStash& sh,
-                          double* xyz, long long cap, cudaStream_t st)
+template <class T, int DR>
+cudaError_t detect_launch_t(const DetectArgs& a, const T* re, const T* im, long long* bt, int nb, const DetectStash& sh,
+                            double* xyz, long long cap, cudaStream_t st)
 {
     const float e = reference_error(a);
     if (xyz) {
-        detect_kernel<T, DETECT_WRITE><<<nb, DB, 0, st>>>(a, re, im, e, bt, xyz, cap, nullptr, nullptr);
+        detect_kernel<T, DETECT_WRITE, DR><<<nb, DB, 0, st>>>(a, re, im, e, bt, xyz, cap, nullptr, nullptr);
     } else if (sh.cap > 0) {
         const cudaError_t m = cudaMemsetAsync(sh.buf, 0, 16, st);
         if (m != cudaSuccess) return m;
-        detect_kernel<T, DETECT_STASH><<<nb, DB, 0, st>>>(a, re, im, e, bt, stash_xyz(sh, nb), sh.cap,
-                                                          (unsigned*)sh.buf, stash_chunks(sh));
+        detect_kernel<T, DETECT_STASH, DR><<<nb, DB, 0, st>>>(a, re, im, e, bt, stash_xyz(sh, nb), sh.cap,
+                                                              (unsigned*)sh.buf, stash_chunks(sh));
     } else {
-        detect_kernel<T, DETECT_COUNT><<<nb, DB, 0, st>>>(a, re, im, e, bt, nullptr, 0, nullptr, nullptr);
+        detect_kernel<T, DETECT_COUNT, DR><<<nb, DB, 0, st>>>(a, re, im, e, bt, nullptr, 0, nullptr, nullptr);
     }
     return cudaGetLastError();
 }
 
+template <class T>
+cudaError_t detect_launch(const DetectArgs& a, const T* re, const T* im, long long* bt, int nb, const DetectStash& sh,
+                          double* xyz, long long cap, cudaStream_t st)
+{
+    return detect_rounds((int64_t)a.nx * a.syz) == 1 ? detect_launch_t<T, 1>(a, re, im, bt, nb, sh, xyz, cap, st)
+                                                     : detect_launch_t<T, DR_MOST>(a, re, im, bt, nb, sh, xyz, cap, st);
+}
+
 }  // namespace
 
-int detect_blocks(int64_t sites) { return (int)((sites + DSITES - 1) / DSITES); }
+int detect_blocks(int64_t sites)
+{
+    const int64_t per = (int64_t)DB * detect_rounds(sites);
+    return (int)((sites + per - 1) / per);
+}
 
 size_t detect_stash_bytes(int nb, int64_t cap)
 {
