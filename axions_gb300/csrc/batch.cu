@@ -80,51 +80,39 @@ using TileSmem = std::conditional_t<is_tiled<SH>, TiledSmem<float, NS>, PairSmem
 
 template <int NS, class SH, bool DIAG, bool Q12>
 __device__ __forceinline__ void run_item(unsigned char* smem_raw, const BatchJob& J, const Fields<float, 5>& f5,
-                                         int bx, int by, int bz)
+                                         int bx, int by, int bz, const TileSums& sums)
 {
-    // partials by planes first, so that their order does not depend on the chunk
-    const int per = J.psub > 0 ? J.chunk / J.psub : 1;
-    const int stride = 2 * J.tiles_y * J.tiles_z;
-    double* part = DIAG ? J.d.partials + 2 * ((bz * per * J.tiles_y + by) * J.tiles_z + bx) : nullptr;
     TileSmem<NS, SH>& sm = *reinterpret_cast<TileSmem<NS, SH>*>(smem_raw);
     if constexpr (is_tiled<SH>)
-        tiled_tile<float, 2, DIAG>(sm, J.g, J.f, J.c, J.ch, J.d, bx, by, bz, J.chunk, part, J.vec != 0, J.psub, stride);
+        tiled_tile<float, 2, DIAG>(sm, J.g, J.f, J.c, J.ch, J.d, bx, by, bz, J.chunk, sums, J.vec != 0);
     else if constexpr (NS == 1)
-        pair_tile<1, DIAG, false, false>(sm, SH{}, J.g, f5, J.pc, J.ch, J.d, bx, by, bz, J.chunk, part, J.psub, stride);
+        pair_tile<1, DIAG, false, false>(sm, SH{}, J.g, f5, J.pc, J.ch, J.d, bx, by, bz, J.chunk, sums);
     else
-        pair_tile<2, DIAG, false, Q12>(sm, SH{}, J.g, J.f, J.pc, J.ch, J.d, bx, by, bz, J.chunk, part, J.psub, stride);
+        pair_tile<2, DIAG, false, Q12>(sm, SH{}, J.g, J.f, J.pc, J.ch, J.d, bx, by, bz, J.chunk, sums);
 }
 
 // Sum of a job's n diagnostic partials by the CTA that finished its last item:
 // every thread a fixed strided subset with Neumaier compensation, then a fixed
-// tree.  red: 2 * threads doubles of shared memory.
+// tree.  red: two doubles of shared memory for each warp.
 template <int THREADS>
 __device__ __forceinline__ void sum_partials(const double* partials, int n, double* out, double* red, int tid)
 {
     double e = 0, ce = 0, g = 0, cg = 0;
+    auto add = [](double& s, double& c, double x) {
+        // |s| >= |x|, by integer instructions
+        const bool larger = (unsigned long long)__double_as_longlong(s) << 1 >= (unsigned long long)__double_as_longlong(x) << 1;
+        const double t = s + x, a = larger ? s : x, b = larger ? x : s;
+        c += (a - t) + b;
+        s = t;
+    };
     for (int b = tid; b < n; b += THREADS) {
-        const double x = __ldcg(partials + 2 * b), y = __ldcg(partials + 2 * b + 1);  // other CTAs wrote them
-        double t = e + x;
-        ce += (fabs(e) >= fabs(x)) ? (e - t) + x : (x - t) + e;
-        e = t;
-        t = g + y;
-        cg += (fabs(g) >= fabs(y)) ? (g - t) + y : (y - t) + g;
-        g = t;
+        const double2 v = __ldcg(reinterpret_cast<const double2*>(partials) + b);   // other CTAs wrote them
+        add(e, ce, v.x);
+        add(g, cg, v.y);
     }
-    red[tid] = e + ce;
-    red[THREADS + tid] = g + cg;
+    warp_sum2(e + ce, g + cg, red[tid >> 5], red[THREADS / 32 + (tid >> 5)], tid & 31);
     __syncthreads();
-    for (int w = THREADS / 2; w > 0; w >>= 1) {
-        if (tid < w) {
-            red[tid] += red[tid + w];
-            red[THREADS + tid] += red[THREADS + tid + w];
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        out[0] = red[0];
-        out[1] = red[THREADS];
-    }
+    store_sum2<THREADS / 32>(red, red + THREADS / 32, out, tid);
 }
 
 // Persistent step kernel for the lattices with NS scalars whose tile is SH: CTAs
@@ -179,7 +167,10 @@ batch_step_kernel(const BatchHead* __restrict__ tab, BatchJob* __restrict__ jobs
         const int by = r % sj.tiles_y;
         const int bz = r / sj.tiles_y;
         if (sj.diag) {
-            run_item<NS, SH, true, Q12>(smem_raw, sj, sf5, bx, by, bz);
+            const int per = sj.psub > 0 ? sj.chunk / sj.psub : 1;
+            const TileSums s_sums{sj.d.partials + 2 * ((bz * per * sj.tiles_y + by) * sj.tiles_z + bx), sj.psub,
+                                  2 * sj.tiles_y * sj.tiles_z};
+            run_item<NS, SH, true, Q12>(smem_raw, sj, sf5, bx, by, bz, s_sums);
             if (tid == 0) {   // the thread that wrote the item's partials
                 __threadfence();
                 s_last = atomicAdd(&jobs[s_job].done, 1) == sj.items - 1;
@@ -190,7 +181,7 @@ batch_step_kernel(const BatchHead* __restrict__ tab, BatchJob* __restrict__ jobs
                 sum_partials<THREADS>(sj.d.partials, sj.partials, sj.diag_out, reinterpret_cast<double*>(smem_raw), tid);
             }
         } else {
-            run_item<NS, SH, false, Q12>(smem_raw, sj, sf5, bx, by, bz);
+            run_item<NS, SH, false, Q12>(smem_raw, sj, sf5, bx, by, bz, TileSums{nullptr, 0, 0});
         }
         __syncthreads();  // sj and the tile's shared memory are reused by the next item
     }

@@ -73,6 +73,7 @@ struct PairSmem {
     float st[pt_stages<NS>()][2 * NS + 3][PT_HY][PT_PZ];  // components in field order: scalars, then theta_x,y,z
     float L[4 * NS + 3][PT_LY][PT_LP];              // link data (LinkIdx<NS> order)
     double red[2][PT_Y];
+    double acc[2][PT_THREADS];                      // diagnostic steps: the threads' sums so far
 };
 
 // ---- paired FP32 arithmetic (two sites per instruction) --------------------
@@ -288,8 +289,7 @@ __device__ __forceinline__ void pair_stage(PairSmem<NS>& sm, const SH& sh, int b
 
 // One tile: z-pairs (bx*2*tz2.., by*ty..) of the evolved region, x-planes
 // [bz*chunk, bz*chunk + chunk).  Called by every thread of the CTA.  With DIAG
-// the CTA's energy and |G| sums are written to part[0], part[1]; with psub > 0
-// the sums of every psub planes to part[0..1], part[pstride..], ...  PIPE: the
+// the CTA's energy and |G| sums go where `sums` says.  PIPE: the
 // level n-1 of the own pair is loaded one plane ahead, and the plain step's
 // x-march is unrolled by two (the carried values then change registers
 // without copies); Abelian-Higgs in its own kernel.  The Moore tile, at the
@@ -298,7 +298,7 @@ __device__ __forceinline__ void pair_stage(PairSmem<NS>& sm, const SH& sh, int b
 template <int NS, bool DIAG, bool PIPE, bool Q12, class SH>
 __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const SH& sh, const Geom& g, const Fields<float, 2 * NS + 3>& f,
                                           const PairCoef& c, const Charges<float>& ch, const DiagOut& d, int bx,
-                                          int by, int bz, int chunk, double* part, int psub = 0, int pstride = 0)
+                                          int by, int bz, int chunk, const TileSums& sums)
 {
     using LI = LinkIdx<NS>;
     constexpr int TH = 2 * NS;  // first theta component
@@ -386,31 +386,15 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const SH& sh, const 
 #pragma unroll
     for (int b = 0; b < ST - 1; ++b) stage(b, ib + b);
 
-    double e_acc = 0.0, g_acc = 0.0;
-    // the CTA's sums so far to `part`
-    auto store_sums = [&]() {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
-            g_acc += __shfl_down_sync(0xffffffffu, g_acc, o);
-        }
-        if ((tid & 31) == 0) {
-            sm.red[0][tid >> 5] = e_acc;
-            sm.red[1][tid >> 5] = g_acc;
-        }
+    // the threads' sums are in shared memory: the plane loop has no registers to spare
+    if constexpr (DIAG) sm.acc[0][tid] = sm.acc[1][tid] = 0.0;
+    // the CTA's sums so far, planes up to i, to their place
+    auto store_sums = [&](int i) {
+        warp_sum2(sm.acc[0][tid], sm.acc[1][tid], sm.red[0][tid >> 5], sm.red[1][tid >> 5], tid & 31);
+        sm.acc[0][tid] = sm.acc[1][tid] = 0.0;
         __syncthreads();
-        if (tid == 0) {
-            double a = 0, b = 0;
-            for (int w = 0; w < PT_Y; ++w) {
-                a += sm.red[0][w];
-                b += sm.red[1][w];
-            }
-            part[0] = a;
-            part[1] = b;
-        }
+        store_sum2<PT_Y>(sm.red[0], sm.red[1], sums.place(i - ib), tid);
         __syncthreads();  // sm.red is reused
-        part += pstride;
-        e_acc = g_acc = 0.0;
     };
     // level n-1 of the own pair for the next plane (PIPE)
     float2 qn[2 * NS + 3];
@@ -699,8 +683,8 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const SH& sh, const 
                     ed = fma2(mul2(p2(c.halfLambda12e), m1), m2, ed);
                 }
                 const float scale = d.energy_form == LAT_ENERGY_MPI ? c.dxdydz : c.dV;
-                e_acc += (double)(ed.x * scale) + (second ? (double)(ed.y * scale) : 0.0);
-                g_acc += (double)fabsf(gauss.x) + (second ? (double)fabsf(gauss.y) : 0.0);
+                sm.acc[0][tid] += widen(ed.x * scale) + (second ? widen(ed.y * scale) : 0.0);
+                sm.acc[1][tid] += widen(fabsf(gauss.x)) + (second ? widen(fabsf(gauss.y)) : 0.0);
             }
             if (d.store_div) store(reinterpret_cast<float*>(d.divbuf) + s, divNow);
             if (d.write) {
@@ -732,13 +716,10 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const SH& sh, const 
         carried = true;
         cur = nxt;
         if constexpr (DIAG) {
-            if (psub > 0 && ((i + 1 - ib) % psub == 0 || i + 1 == ie)) store_sums();
+            if (sums.ends(i + 1 - ib) || i + 1 == ie) store_sums(i);
         }
     }
     __pipeline_wait_prior(0);  // nothing is in flight here; kept for an empty x-range
-    if constexpr (DIAG) {
-        if (psub == 0) store_sums();
-    }
 }
 
 template <int NS, bool DIAG, bool Q12, class SH>
@@ -751,7 +732,7 @@ pair_step_kernel(const Geom g, const SH sh, const Fields<float, 2 * NS + 3> f, c
     PairSmem<NS>& sm = *reinterpret_cast<PairSmem<NS>*>(smem_raw);
     const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     pair_tile<NS, DIAG, NS == 1, Q12>(sm, sh, g, f, c, ch, d, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, chunk,
-                                      DIAG ? d.partials + 2 * blk : nullptr);
+                                      TileSums{d.partials + 2 * blk, 0, 0});
 }
 
 // Whether a Moore lattice takes the pair step, on 64x4 tiles: 16-byte staging,

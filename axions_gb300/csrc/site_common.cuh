@@ -4,6 +4,7 @@
 #include "dtrig.cuh"
 #include "fp64_exact.cuh"
 #include "lattice_internal.cuh"
+#include "widen.cuh"
 
 namespace lat {
 
@@ -90,6 +91,38 @@ __device__ __forceinline__ Nbr flat_nbr(const Geom& g, const Flat& r, unsigned q
     const unsigned plane = (__umulhi(row, r.dy.mul) + row) >> r.dy.shift;
     return make_nbr(g, g.lox + (int)plane, g.loy + (int)(row - plane * (unsigned)r.hy),
                     g.loz + (int)(q - row * (unsigned)r.hz));
+}
+
+// The sums of a and b over a warp, by the tree of shfl_down additions, stored by
+// the lanes that have them.  After the first exchange lanes 0..15 go on with a and
+// lanes 16..31 with b: five FP64 additions instead of ten, the same ones.
+__device__ __forceinline__ void warp_sum2(double a, double b, double& sa, double& sb, int lane)
+{
+    const bool low = lane < 16;
+    double s = low ? a : b;
+    s += __shfl_xor_sync(0xffffffffu, low ? b : a, 16);
+#pragma unroll
+    for (int o = 8; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+    if (lane == 0) sa = s;
+    if (lane == 16) sb = s;
+}
+
+// part[0], part[1] = the sums of W values of ra and of rb in order, by thread 0;
+// called by the first warp at least
+template <int W>
+__device__ __forceinline__ void store_sum2(const double* ra, const double* rb, double* part, int tid)
+{
+    if (tid < 32) {
+        const double* const r = tid == 1 ? rb : ra;   // lane 1 adds rb's
+        double s = r[0];
+#pragma unroll
+        for (int w = 1; w < W; ++w) s += r[w];
+        const double b = __shfl_sync(0xffffffffu, s, 1);
+        if (tid == 0) {
+            part[0] = s;
+            part[1] = b;
+        }
+    }
 }
 
 // Sum two doubles over a one-dimensional block (a power of two of threads, at

@@ -182,17 +182,25 @@ inline bool tiled_vec_ok(const Geom& g, const Fields<T, NC>& f)
     return true;
 }
 
+// Where the diagnostic sums of a tile's march go: those of every `planes` planes (a
+// power of two) to part[0..1], part[stride..], ...; with 0 planes those of all to
+// part[0..1].
+struct TileSums {
+    double* part;
+    int planes, stride;
+    __device__ __forceinline__ bool ends(int done) const { return planes > 0 && (done & (planes - 1)) == 0; }
+    __device__ __forceinline__ double* place(int plane) const { return planes > 0 ? part + plane / planes * stride : part; }
+};
+
 // One tile: columns (bx*TZ.., by*TY..) of the evolved region, x-planes
 // [bz*chunk, bz*chunk + chunk).  Called by every thread of the CTA.  With DIAG
-// the CTA's energy and |G| sums are written to part[0], part[1]; with psub > 0
-// the sums of every psub planes to part[0..1], part[pstride..], ...  `vec`
+// the CTA's energy and |G| sums go where `sums` says.  `vec`
 // selects the 16-byte staging (only where tiled_vec_ok holds); both stagings
 // fill the same shared-memory positions, so the results are bitwise equal.
 template <class T, int NS, bool DIAG>
 __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, const Fields<T, 2 * NS + 3>& f,
                                            const StepCoefT<T>& c, const Charges<T>& ch, const DiagOut& d, int bx,
-                                           int by, int bz, int chunk, double* part, bool vec, int psub = 0,
-                                           int pstride = 0)
+                                           int by, int bz, int chunk, const TileSums& sums, bool vec)
 {
     using TR = Trig<T>;
     using LI = LinkIdx<NS>;
@@ -247,29 +255,12 @@ __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, 
     stage(1, wrap_idx(ib + 1, g.nx));
 
     double e_acc = 0.0, g_acc = 0.0;
-    // the CTA's sums so far to `part`
-    auto store_sums = [&]() {
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) {
-            e_acc += __shfl_down_sync(0xffffffffu, e_acc, o);
-            g_acc += __shfl_down_sync(0xffffffffu, g_acc, o);
-        }
-        if (tz == 0) {
-            sm.red[0][ty] = e_acc;
-            sm.red[1][ty] = g_acc;
-        }
+    // the CTA's sums so far, planes up to i, to their place
+    auto store_sums = [&](int i) {
+        warp_sum2(e_acc, g_acc, sm.red[0][ty], sm.red[1][ty], tz);
         __syncthreads();
-        if (tid == 0) {
-            double a = 0, b = 0;
-            for (int w = 0; w < TT_Y; ++w) {
-                a += sm.red[0][w];
-                b += sm.red[1][w];
-            }
-            part[0] = a;
-            part[1] = b;
-        }
+        store_sum2<TT_Y>(sm.red[0], sm.red[1], sums.place(i - ib), tid);
         __syncthreads();  // sm.red is reused
-        part += pstride;
         e_acc = g_acc = 0.0;
     };
 
@@ -475,8 +466,8 @@ __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, 
                     const T m2 = mag[1] - c.eta2Sq;
                     ed += c.quarterLambda2 * (m2 * m2) + c.halfLambda12e * m1 * m2;
                 }
-                e_acc += (double)(d.energy_form == LAT_ENERGY_MPI ? ed * c.dx * c.dy * c.dz : c.dV * ed);
-                g_acc += (double)fabs(gauss);
+                e_acc += widen(d.energy_form == LAT_ENERGY_MPI ? ed * c.dx * c.dy * c.dz : c.dV * ed);
+                g_acc += widen(fabs(gauss));
             }
             if (d.store_div) reinterpret_cast<T*>(d.divbuf)[s] = divNow;
             if (d.write) {
@@ -500,13 +491,10 @@ __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, 
         for (int cc = 0; cc < 2 * NS; ++cc) vm[cc] = v[cc];
         cur = nxt;
         if constexpr (DIAG) {
-            if (psub > 0 && ((i + 1 - ib) % psub == 0 || i + 1 == ie)) store_sums();
+            if (sums.ends(i + 1 - ib) || i + 1 == ie) store_sums(i);
         }
     }
     __pipeline_wait_prior(0);  // nothing is in flight here; kept for an empty x-range
-    if constexpr (DIAG) {
-        if (psub == 0) store_sums();
-    }
 }
 
 template <class T, int NS, bool DIAG>
@@ -519,7 +507,7 @@ tiled_step_kernel(const Geom g, const Fields<T, 2 * NS + 3> f, const StepCoefT<T
     TiledSmem<T, NS>& sm = *reinterpret_cast<TiledSmem<T, NS>*>(smem_raw);
     const int blk = blockIdx.x + gridDim.x * (blockIdx.y + gridDim.y * blockIdx.z);
     tiled_tile<T, NS, DIAG>(sm, g, f, c, ch, d, (int)blockIdx.x, (int)blockIdx.y, (int)blockIdx.z, chunk,
-                            DIAG ? d.partials + 2 * blk : nullptr, vec != 0);
+                            TileSums{d.partials + 2 * blk, 0, 0}, vec != 0);
 }
 
 inline dim3 tiled_grid(const Geom& g, int chunk)
