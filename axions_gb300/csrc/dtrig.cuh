@@ -18,9 +18,11 @@
 //       relative accuracy;
 //   the 64-bit result is rounded to the double.
 //
-// Against 60-digit values the error was at most 1.35 ulps (mean 0.29) over
-// 150,000 samples of |x| < 6e4, the zeros and quarter turns among them: the
-// rounding of r and the final one.  CUDA documents 2 ulps for its double sin.
+// At most 1.65 ulps: the rounding of r is half a unit of r, a whole one of a result
+// just below a power of two, pi/2's 2^-92.8 up to 0.09 and the integers 0.06 of one,
+// and the final rounding is half of one.  Over 750,000 samples at multiples of pi/2
+// and of pi/4 and powers of two from them 1.49 was found, over random ones 1.35
+// (mean 0.29).  CUDA documents 2 ulps for its double sin.
 // Measured on GB300, SM cycles for a warp's evaluation: sine 65, sincos 95.
 // The table-driven form before it, all on the FP64 pipe (13 and 15
 // instructions, at most 2.45 ulps), took 234 and 266.
@@ -46,7 +48,7 @@ namespace dtrig {
 constexpr int kHiLarge = 0x40f00000;  // high word of 2^16
 constexpr int kHiTiny = 0x3e400000;   // high word of 2^-27
 
-// pi/2 = P1 + P2 within 2^-93: 36 bits, then the nearest double of the rest
+// pi/2 = P1 + P2 within 2^-92.8: 36 bits, then the nearest double of the rest
 constexpr double kP1 = 0x1.921fb54440000p+0;
 constexpr double kP2 = 0x1.68c234c4c6629p-39;
 

@@ -9,7 +9,7 @@
 namespace lat {
 
 // Transcendentals by precision.  The FP64 path uses the fixed-point sine and
-// cosine of dtrig.cuh (at most 1.35 ulps, two FP64 instructions each); the
+// cosine of dtrig.cuh (at most 1.65 ulps, two FP64 instructions each); the
 // FP32 path the reduced hardware approximations below.
 template <class T>
 struct Trig;

@@ -419,7 +419,7 @@ int lat_simple_sine_ic_device(lat_handle* h, const lat_string_profile* prof, dou
 int lat_philox4x32_10(const uint32_t counter[4], const uint32_t key[2], uint32_t out[4]);
 
 /* The FP64 step's sine and cosine (fixed-point polynomials after a reduction to
- * |r| <= pi/4, within 1.35 ulps) evaluated on the current device at n host arguments x, for
+ * |r| <= pi/4, within 1.65 ulps) evaluated on the current device at n host arguments x, for
  * checks: out (5*n doubles, host) receives sin(x) from the sine alone, then
  * sin(x) and cos(x) from the joint sincos, then CUDA's sin(x) and cos(x).
  * No counterpart in the reference, whose step calls libm's sin and cos
