@@ -164,8 +164,6 @@ struct AhSite {
     double cPxy, cPxz, cPyz, divPast;   // diagnostic steps
 };
 
-// The update of one site (mpi_evolution.cpp:412-501) and its diagnostics: new
-// values to `next` (phi, then theta), div(theta) to divNow.
 // cm*x + sm*y, out of line: where a compiler would predicate it, it costs the
 // FP64 pipe on every path
 static __device__ __noinline__ double mul_add_rare(double cm, double x, double sm, double y)
@@ -179,6 +177,8 @@ static __device__ __noinline__ double mul_add_rare(double cm, double x, double s
 // fixed_point.cuh.
 enum { FP_PRODUCTS, INT_PRODUCTS, INT_ZERO_SINES, FIXED_POINT };
 
+// The update of one site (mpi_evolution.cpp:412-501) and its diagnostics: new
+// values to `next` (phi, then theta), div(theta) to divNow.
 template <bool STRICT, bool DIAG, bool RECIP, int INT>
 __device__ __forceinline__ void ah_site(const AhSite& v, const StepCoef& c, const DiagOut& d, double (&next)[5],
                                         double& divNow, double& e_site, double& g_site)

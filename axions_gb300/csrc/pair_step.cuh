@@ -40,7 +40,7 @@
 // 16-byte chunks and 8-byte pairs need periodic z, nz a multiple of 4 and
 // 16-byte aligned fields (every benchmark and serving shape); odd extents and
 // fixed z walls take an instance that stages and accesses single elements
-// (Abelian-Higgs 201 x 199 x 203: 138 us a step, 146 on the one-site tiled step;
+// (Abelian-Higgs 201 x 199 x 203: 136 us a step, 146 on the one-site tiled step;
 // 96^3 on 32x8 tiles 16.5 us, 18.6 before; 32^3 4.3, 6.2 before).
 // HBM traffic is the algorithmic 3 accesses per value.  Energy and Gauss sums
 // are accumulated in FP64.
@@ -511,7 +511,7 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const SH& sh, const 
             sts2(lk(LI::pyz, 0, hl), sin2(sub2(sub2(add2(hty, htzyp), htyzp), htz)));
         }
         if (halo_col) {
-            // z = k0-1 of row j0+tz (staged column PT_C0-1): what z = k0 reads as its z-backward data
+            // z = k0-1 of row j0+tz (staged column c0-1): what z = k0 reads as its z-backward data
             const int r = hr;
             const float htx = *at(S, TH, r, sh.c0 - 1), hty = *at(S, TH + 1, r, sh.c0 - 1);
             const float htz = *at(S, TH + 2, r, sh.c0 - 1);

@@ -45,7 +45,7 @@ struct Trig<float> {
 };
 
 // a / b.  FP64: the IEEE quotient (the reference's rounding) by cdiv from the
-// host reciprocal inv_b = RN(1/b), five FP64 instructions; FP32 multiplies by
+// host reciprocal inv_b = RN(1/b), by integer instructions; FP32 multiplies by
 // the reciprocal.
 template <class T>
 __device__ __forceinline__ T qdiv(T a, T b, T inv_b)

@@ -56,9 +56,10 @@ extern "C" {
 /* precision of the stored fields and of the step arithmetic */
 #define LAT_F64 0            /* the reference's arithmetic                          */
 #define LAT_F32 1            /* FP32 fields and step; energy/Gauss sums stay FP64   */
-#define LAT_F64_FAST 2       /* FP64 fields; fused multiply-adds and a corrected
-                                reciprocal for /dt (each operation within an ulp of
-                                LAT_F64's); not bit-identical to the reference's order */
+#define LAT_F64_FAST 2       /* FP64 fields; fused multiply-adds, constant factors taken
+                                together, one sine for a plaquette's two orientations
+                                (each operation rounded no more than LAT_F64's); not
+                                bit-identical to the reference's order */
 
 /* boundary handling: `bc` for the x and y axes (the reference's xyBC), `bc_z`
  * for z (zBC; 0 = the same as bc) */
@@ -453,11 +454,11 @@ int64_t lat_footprint_bytes(const lat_params* p);
  * The reference runs one lattice per program invocation; an ensemble of
  * independent lattices (different seeds, couplings, sizes, models) is a loop of
  * runs.  A batch advances all its lattices together: each step is one
- * persistent kernel over the tiles of every lattice, and nsteps of them are one
- * CUDA graph.  Lattices are ordinary FP32 handles (LAT_F32): state transfer,
- * detection and winding keep working on each handle between batch calls.  A
- * lattice's results are bitwise the same alone, in any mix and through
- * lat_step/lat_advance on its own handle. */
+ * persistent kernel per model and tile shape over the tiles of its lattices, and
+ * nsteps of them are one CUDA graph.  Lattices are ordinary FP32 handles
+ * (LAT_F32): state transfer, detection and winding keep working on each handle
+ * between batch calls.  A lattice's results are bitwise the same alone and in any
+ * mix; lat_step/lat_advance on its own handle give them to FP32 rounding. */
 typedef struct lat_batch lat_batch;
 int lat_batch_create(int32_t max_jobs, lat_batch** out);          /* max_jobs <= 256 */
 int lat_batch_destroy(lat_batch* b);                               /* handles are not freed */
