@@ -211,8 +211,9 @@ __global__ void __launch_bounds__(BLOCK) divergence_kernel(const Geom g, const T
     if (k >= g.hiz || j >= g.hiy) return;
     const Nbr n = make_nbr(g, i, j, k);
     const int s = n.s;
-    out[s] = qdiv<T>(TX[s] - TX[s + n.xm], c.dx2, c.inv_dx2) + qdiv<T>(TY[s] - TY[s + n.ym], c.dy2, c.inv_dy2)
-           + qdiv<T>(TZ[s] - TZ[s + n.zm], c.dz2, c.inv_dz2);
+    const T x = TX[s] - TX[s + n.xm], y = TY[s] - TY[s + n.ym], z = TZ[s] - TZ[s + n.zm];
+    if constexpr (sizeof(T) == 4) out[s] = div_sum(x, y, z, c.inv_dx2, c.inv_dy2, c.inv_dz2);
+    else out[s] = qdiv<T>(x, c.dx2, c.inv_dx2) + qdiv<T>(y, c.dy2, c.inv_dy2) + qdiv<T>(z, c.dz2, c.inv_dz2);
 }
 
 template <class T>

@@ -642,7 +642,7 @@ __device__ __forceinline__ void pair_tile(PairSmem<NS>& sm, const SH& sh, const 
             if (DIAG || d.store_div) {
                 const float2 tym = lds2(at(S, TH + 1, hy - 1, col));
                 const float2 tzm = make_float2(*at(S, TH + 2, hy, col - 1), tzv.x);
-                divNow = fma2(sub2(tzv, tzm), inv_dz2, fma2(sub2(tyv, tym), inv_dy2, mul2(sub2(tx, txm), inv_dx2)));
+                divNow = fma2(sub2(tzv, tzm), inv_dz2, fma2(sub2(tx, txm), inv_dx2, mul2(sub2(tyv, tym), inv_dy2)));   // as div_sum
             }
             if constexpr (DIAG) {
                 float2 tdc = p2(0.f), fc = p2(0.f), gauss = p2(0.f);

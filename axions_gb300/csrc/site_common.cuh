@@ -54,6 +54,14 @@ __device__ __forceinline__ T qdiv(T a, T b, T inv_b)
     else return a * inv_b;
 }
 
+// x/dx2 + y/dy2 + z/dz2 of the FP32 kernels, rounded alike in all of them: a Gauss
+// sum takes the difference of two levels' divergences, which different kernels may
+// have formed, and a static one has to cancel.
+__device__ __forceinline__ float div_sum(float x, float y, float z, float ix, float iy, float iz)
+{
+    return __fmaf_rn(z, iz, __fmaf_rn(x, ix, __fmul_rn(y, iy)));
+}
+
 // Leapfrog update X^{n+1} from X^n, X^{n-1} and the acceleration.
 // FP64 keeps the reference's expression 2*X - Xp + dt^2*a
 // (mpi_evolution.cpp:432).  FP32 uses X + (X - Xp) + dt^2*a: the difference

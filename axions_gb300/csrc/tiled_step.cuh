@@ -436,7 +436,7 @@ __device__ __forceinline__ void tiled_tile(TiledSmem<T, NS>& sm, const Geom& g, 
             T divNow = 0;
             if (DIAG || d.store_div) {
                 const T tym = sm.th[cur][1][hy - 1][hz + TT_C0], tzm = sm.th[cur][2][hy][hz - 1 + TT_C0];
-                divNow = (tx - txm_prev) * c.inv_dx2 + (tyv - tym) * c.inv_dy2 + (tzv - tzm) * c.inv_dz2;
+                divNow = div_sum(tx - txm_prev, tyv - tym, tzv - tzm, c.inv_dx2, c.inv_dy2, c.inv_dz2);
             }
             if constexpr (DIAG) {
                 T tdc = 0, fc = 0, gauss = 0;
